@@ -11,6 +11,7 @@
 // (src/alofa/kernels/cpu/scalar.mojo:93-470, paged.mojo:208-336,
 // segments.mojo:48-130) with fp32 instead of f64 accumulators.
 #include "common.cuh"
+#include <type_traits>
 
 // ---------------------------------------------------------------------------
 // Embedding: out[t, :] = table[ids[t], :] widened to fp32.
@@ -51,9 +52,10 @@ ALOFA_API int alofa_embed_gather(void* out, const void* table, const int* ids, c
 // shift, the variance being the mean of the squared deviations.
 // ---------------------------------------------------------------------------
 template <typename TO>
-__global__ void rmsnorm_kernel(TO* __restrict__ out, const float* __restrict__ x, const float* __restrict__ w,
+__global__ void rmsnorm_kernel(TO* __restrict__ out, const float* x, const float* __restrict__ w,
                                const float* __restrict__ shift, const int* __restrict__ rows, int hidden, float eps) {
   __shared__ float scratch[32];
+  pdl_begin();
   const int r = blockIdx.x;
   const float* xr = x + (size_t)(rows ? rows[r] : r) * hidden;
   float mean = 0.f;
@@ -72,13 +74,61 @@ __global__ void rmsnorm_kernel(TO* __restrict__ out, const float* __restrict__ x
   else for (int c = threadIdx.x; c < hidden; c += blockDim.x) out[(size_t)r * hidden + c] = from_f<TO>(xr[c] * scale * w[c]);
 }
 
+// Rows of up to 4,096 numbers in whole groups of four: every load of the row is in flight at once and the row stays in
+// registers, and the kernel before it may still run (one row of 896 in a decode step: 4.6 -> 1.5 us of the step's time).
+template <typename TO>
+__global__ void __launch_bounds__(256) rmsnorm_vector_kernel(TO* __restrict__ out, const float* x, const float* __restrict__ w,
+                                                             const float* __restrict__ shift, const int* __restrict__ rows, int hidden, float eps) {
+  __shared__ float scratch[32];
+  const int n4 = hidden >> 2;
+  float4 v[4], g[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {  // the norm's weight is a constant of the model: read ahead of the wait
+    const int c = threadIdx.x + i * 256;
+    g[i] = c < n4 ? reinterpret_cast<const float4*>(w)[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  pdl_begin();
+  const int r = blockIdx.x;
+  const float4* xr = reinterpret_cast<const float4*>(x + (size_t)(rows ? rows[r] : r) * hidden);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int c = threadIdx.x + i * 256;
+    v[i] = c < n4 ? xr[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  float mean = 0.f;
+  if (shift) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) mean += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+    mean = block_sum(mean, scratch) / (float)hidden;
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (threadIdx.x + i * 256 >= n4) continue;
+    const float a = v[i].x - mean, b = v[i].y - mean, c = v[i].z - mean, d = v[i].w - mean;
+    ss = fmaf(a, a, ss), ss = fmaf(b, b, ss), ss = fmaf(c, c, ss), ss = fmaf(d, d, ss);
+  }
+  ss = block_sum(ss, scratch);
+  const float scale = 1.0f / sqrtf(ss / (float)hidden + eps);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int c = threadIdx.x + i * 256;
+    if (c >= n4) continue;
+    float y[4] = {(v[i].x - mean) * scale * g[i].x, (v[i].y - mean) * scale * g[i].y, (v[i].z - mean) * scale * g[i].z, (v[i].w - mean) * scale * g[i].w};
+    TO* o = out + (size_t)r * hidden + 4 * c;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] = from_f<TO>(shift ? y[j] + shift[4 * c + j] : y[j]);
+  }
+}
+
 ALOFA_API int alofa_rmsnorm(void* out, const void* x, const void* w, const float* shift, const int* rows, int n_rows, int hidden, float eps,
                             int out_bf16, cudaStream_t stream) {
   if (n_rows <= 0) return ALOFA_OK;
+  const bool vector = hidden % 4 == 0 && hidden <= 4096 && ((uintptr_t)x | (uintptr_t)w) % 16 == 0;
   if (out_bf16)
-    rmsnorm_kernel<bf16><<<n_rows, 256, 0, stream>>>((bf16*)out, (const float*)x, (const float*)w, shift, rows, hidden, eps);
+    launch_dep(vector ? rmsnorm_vector_kernel<bf16> : rmsnorm_kernel<bf16>, n_rows, 256, 0, stream, (bf16*)out, (const float*)x, (const float*)w, shift, rows, hidden, eps);
   else
-    rmsnorm_kernel<float><<<n_rows, 256, 0, stream>>>((float*)out, (const float*)x, (const float*)w, shift, rows, hidden, eps);
+    launch_dep(vector ? rmsnorm_vector_kernel<float> : rmsnorm_kernel<float>, n_rows, 256, 0, stream, (float*)out, (const float*)x, (const float*)w, shift, rows, hidden, eps);
   return launch_status();
 }
 
@@ -171,6 +221,107 @@ __global__ void __launch_bounds__(256) gemm_generic_kernel(TO* __restrict__ out,
   }
 }
 
+// The same for 32-bit operands whose depth is a multiple of four: the product of the whole 32-bit path.  A warp owns MT
+// rows of x and NT columns of the output; lane l sums the depths 4 l .. 4 l + 3 of every run of 128 in ascending order, and
+// the 32 lanes' sums are added pairwise, 16, 8, 4, 2, 1 lanes apart.  That order depends on the depth alone, so a row's
+// result is the same in every tile shape below, whatever rows share the launch.  A decode step is bound by the weights'
+// bytes: one row takes one column a warp, with up to 16 loads of 16 bytes a lane in flight and the first of them ahead of
+// the dependency wait, where the 64 x 64 tiles above kept 14 of 148 SMs busy (one row, output and down projection of 896
+// columns: 318 -> 3.7 us on average; gate and up 244 -> 6.5 us, 5.4 TB/s).  Many rows are bound by the reads of x and w
+// through L1: 8 x 4 sums a lane from 12 such reads (40 rows, gate and up: 57 us).
+template <int V>
+__device__ __forceinline__ float reduce_across_lanes(float (&v)[V], int lane) {  // value i ends in the lanes i * (32 / V) ..
+  int o = 16;
+#pragma unroll
+  for (int half = V / 2; half >= 1; half >>= 1, o >>= 1) {
+    const bool upper = lane & o;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const float mine = upper ? v[half + i] : v[i], sent = upper ? v[i] : v[half + i];
+      v[i] = mine + __shfl_xor_sync(0xffffffffu, sent, o);
+    }
+  }
+  float s = v[0];
+#pragma unroll
+  for (int left = 32 / V / 2; left >= 1; left >>= 1) s += __shfl_xor_sync(0xffffffffu, s, left);
+  return s;
+}
+
+template <int MT, int NT, int EPI>
+__global__ void __launch_bounds__(256) gemm_f32_kernel(float* out, const float* x, const float* __restrict__ w, const float* __restrict__ bias, int M, int N, int K, int act,
+                                                       float gate_alpha, float gate_limit) {
+  constexpr int NW = EPI == EPI_GATED ? 2 : 1, R = NT * NW, V = MT * R;
+  constexpr int U = V == 1 ? 16 : R >= 8 ? 1 : 8 / R;  // runs of 128 whose weights are asked for together
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n0 = (blockIdx.x * 8 + warp) * NT, m0 = blockIdx.y * MT;
+  const int k4 = K >> 2;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4* wr[R];  // columns past the last read the last one's weights, and are not stored
+#pragma unroll
+  for (int r = 0; r < R; ++r) wr[r] = reinterpret_cast<const float4*>(w + ((size_t)(r % NW) * N + min(n0 + r / NW, N - 1)) * K);
+  float4 wv[U][R];
+  auto load_weights = [&](int c) {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int r = 0; r < R; ++r) wv[u][r] = c + u * 32 < k4 ? __ldg(wr[r] + c + u * 32) : zero;
+  };
+  load_weights(lane);
+  pdl_begin();
+  const float4* xr[MT];
+#pragma unroll
+  for (int m = 0; m < MT; ++m) xr[m] = reinterpret_cast<const float4*>(x + (size_t)min(m0 + m, M - 1) * K);
+  float acc[V];
+#pragma unroll
+  for (int v = 0; v < V; ++v) acc[v] = 0.f;
+  for (int c = lane; c < k4; c += 32 * U) {  // a lane past the end has left the loop: its sums stand
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float4 xv[MT];
+#pragma unroll
+      for (int m = 0; m < MT; ++m) xv[m] = c + u * 32 < k4 ? xr[m][c + u * 32] : zero;
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          float& a = acc[m * R + r];
+          a = fmaf(xv[m].x, wv[u][r].x, a), a = fmaf(xv[m].y, wv[u][r].y, a);
+          a = fmaf(xv[m].z, wv[u][r].z, a), a = fmaf(xv[m].w, wv[u][r].w, a);
+        }
+    }
+    load_weights(c + 32 * U);
+  }
+  float v = reduce_across_lanes<V>(acc, lane);
+  const int i = lane / (32 / V);  // the value this lane holds: row i / R, column (i % R) / NW, its gate or up sum
+  const int m = m0 + i / R, n = n0 + (i % R) / NW;
+  if (EPI == EPI_GATED) {
+    float u = __shfl_xor_sync(0xffffffffu, v, 32 / V);  // the up sum beside the gate's
+    if (i % NW || m >= M || n >= N || lane % (32 / V)) return;
+    if (bias) v += bias[n], u += bias[N + n];
+    out[(size_t)m * N + n] = gate_times(v, u, gate_alpha, gate_limit);
+    return;
+  }
+  if (m >= M || n >= N || lane % (32 / V)) return;
+  if (bias) v += bias[n];
+  float* o = out + (size_t)m * N + n;
+  *o = EPI == EPI_RESIDUAL ? *o + v : activate(v, act);
+}
+
+template <int EPI>
+static int gemm_f32_launch(float* out, const float* x, const float* w, const float* bias, int M, int N, int K, int act, float gate_alpha, float gate_limit, cudaStream_t stream) {
+  constexpr int NW = EPI == EPI_GATED ? 2 : 1;
+  auto launch = [&](auto kernel, int mt, int nt) {
+    const long long rows = (M + mt - 1) / mt;
+    if (rows > 65535) return ALOFA_ERR_ARGUMENT;
+    launch_dep(kernel, dim3((N + 8 * nt - 1) / (8 * nt), (unsigned)rows), 256, 0, stream, out, x, w, bias, M, N, K, act, gate_alpha, gate_limit);
+    return launch_status();
+  };
+  if (M == 1) return launch(gemm_f32_kernel<1, 1, EPI>, 1, 1);
+  if (M == 2) return launch(gemm_f32_kernel<2, 2 / NW, EPI>, 2, 2 / NW);
+  if (M <= 4) return launch(gemm_f32_kernel<4, 2 / NW, EPI>, 4, 2 / NW);
+  return launch(gemm_f32_kernel<8, 4 / NW, EPI>, 8, 4 / NW);
+}
+
 template <typename TA, typename TW, typename TO>
 static int gemm_generic_launch(void* out, const void* x, const void* w, const float* bias, int M, int N, int K, int epi,
                                float gate_alpha, float gate_limit, cudaStream_t stream) {
@@ -199,7 +350,18 @@ ALOFA_API int alofa_gemm_generic(void* out, const void* x, const void* w, const 
   const float* b = (const float*)bias;
   const int key = (x_bf16 ? 4 : 0) | (w_bf16 ? 2 : 0) | (out_bf16 ? 1 : 0);
   switch (key) {
-    case 0: return gemm_generic_launch<float, float, float>(out, x, w, b, M, N, K, epi, gate_alpha, gate_limit, stream);
+    case 0:
+      if (K % 4 == 0 && ((uintptr_t)x | (uintptr_t)w) % 16 == 0 && M <= 8 * 65535) {  // rows of whole groups of 16 bytes
+        const int act = epi >> 4;
+        if (act && (epi & 15) != EPI_STORE) return ALOFA_ERR_ARGUMENT;
+        switch (epi & 15) {
+          case EPI_STORE: return gemm_f32_launch<EPI_STORE>((float*)out, (const float*)x, (const float*)w, b, M, N, K, act, gate_alpha, gate_limit, stream);
+          case EPI_RESIDUAL: return gemm_f32_launch<EPI_RESIDUAL>((float*)out, (const float*)x, (const float*)w, b, M, N, K, act, gate_alpha, gate_limit, stream);
+          case EPI_GATED: return gemm_f32_launch<EPI_GATED>((float*)out, (const float*)x, (const float*)w, b, M, N, K, act, gate_alpha, gate_limit, stream);
+          default: return ALOFA_ERR_ARGUMENT;
+        }
+      }
+      return gemm_generic_launch<float, float, float>(out, x, w, b, M, N, K, epi, gate_alpha, gate_limit, stream);
     case 1: return gemm_generic_launch<float, float, bf16>(out, x, w, b, M, N, K, epi, gate_alpha, gate_limit, stream);
     case 2: return gemm_generic_launch<float, bf16, float>(out, x, w, b, M, N, K, epi, gate_alpha, gate_limit, stream);
     case 3: return gemm_generic_launch<float, bf16, bf16>(out, x, w, b, M, N, K, epi, gate_alpha, gate_limit, stream);
@@ -222,9 +384,10 @@ ALOFA_API int alofa_gemm_generic(void* out, const void* x, const void* w, const 
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void rope_store_kernel(T* __restrict__ q_out, T* __restrict__ k_cache, T* __restrict__ v_cache,
-                                  const T* __restrict__ qkv, const float* __restrict__ cos_sin,
+                                  const T* qkv, const float* __restrict__ cos_sin,
                                   const int* __restrict__ positions, const int* __restrict__ slot_map, int nh, int nkv,
                                   int hd, int rot, int write_cache) {
+  pdl_begin();
   const int t = blockIdx.x;
   const int head = blockIdx.y;  // 0..nh-1 q, nh..nh+nkv-1 k, then v
   const int pos = positions[t];
@@ -268,12 +431,11 @@ ALOFA_API int alofa_rope_store(void* q_out, void* k_cache, void* v_cache, const 
   dim3 grid(n_tokens, nh + 2 * nkv);
   const int threads = hd <= 32 ? 32 : (hd <= 64 ? 64 : 128);
   if (is_bf16)
-    rope_store_kernel<bf16><<<grid, threads, 0, stream>>>((bf16*)q_out, (bf16*)k_cache, (bf16*)v_cache, (const bf16*)qkv,
-                                                           cos_sin, positions, slot_map, nh, nkv, hd, rot, write_cache);
+    launch_dep(rope_store_kernel<bf16>, grid, threads, 0, stream, (bf16*)q_out, (bf16*)k_cache, (bf16*)v_cache, (const bf16*)qkv,
+               cos_sin, positions, slot_map, nh, nkv, hd, rot, write_cache);
   else
-    rope_store_kernel<float><<<grid, threads, 0, stream>>>((float*)q_out, (float*)k_cache, (float*)v_cache,
-                                                            (const float*)qkv, cos_sin, positions, slot_map, nh, nkv, hd,
-                                                            rot, write_cache);
+    launch_dep(rope_store_kernel<float>, grid, threads, 0, stream, (float*)q_out, (float*)k_cache, (float*)v_cache, (const float*)qkv,
+               cos_sin, positions, slot_map, nh, nkv, hd, rot, write_cache);
   return launch_status();
 }
 
@@ -292,11 +454,12 @@ ALOFA_API int alofa_rope_store(void* q_out, void* k_cache, void* v_cache, const 
 // ---------------------------------------------------------------------------
 template <typename T, typename TO>
 __global__ void __launch_bounds__(128) paged_attention_generic_kernel(
-    TO* __restrict__ out, const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
+    TO* __restrict__ out, const T* q, const T* k_cache, const T* v_cache,
     const int* __restrict__ positions, const int* __restrict__ seq_of_token, const int* __restrict__ block_table,
     int max_blocks, int page_size, int nh, int nkv, int hd, int vd, int window, float scale, float softcap, const float* __restrict__ sink,
     int chunk, int v_share, int keep, const float* __restrict__ slopes) {
-  extern __shared__ float smem[];
+  extern __shared__ __align__(16) float smem[];
+  pdl_begin();
   float* qs = smem;          // hd
   float* ps = smem + hd;     // 128
   __shared__ float scratch[32];
@@ -359,6 +522,98 @@ __global__ void __launch_bounds__(128) paged_attention_generic_kernel(
   if (tid + 128 < vd) o[tid + 128] = from_f<TO>(acc1 / l);
 }
 
+// The same where keys and values are whole groups of four numbers: a key's row is read four numbers at a time, all of it in
+// flight at once, and the value sum is spread over all 128 threads, a group of vd / 4 threads taking every G-th key of a chunk;
+// the groups' sums are added in order at the end.  Chunks and the order within one go by the key's index alone, as above.
+// A block's time is its dependent trips to memory (one row of 14 heads over 48 keys: 21 -> 8.8 us).
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const bf16* p) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+template <typename T, typename TO>
+__global__ void __launch_bounds__(128) paged_attention_vector_kernel(
+    TO* __restrict__ out, const T* q, const T* k_cache, const T* v_cache,
+    const int* __restrict__ positions, const int* __restrict__ seq_of_token, const int* __restrict__ block_table,
+    int max_blocks, int page_size, int nh, int nkv, int hd, int vd, int window, float scale, float softcap, const float* __restrict__ sink,
+    int chunk, int v_share, int keep, const float* __restrict__ slopes) {
+  extern __shared__ __align__(16) float smem[];
+  float* qs = smem;            // hd
+  float* ps = qs + hd;         // 128
+  float* sums = ps + 128;      // [G][vd], at most 512
+  __shared__ float scratch[32];
+  __shared__ int pages[128];
+  pdl_begin();
+  const int t = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
+  const int kvh = h / (nh / nkv);
+  const int P = positions[t];
+  const int* table = block_table + (size_t)seq_of_token[t] * max_blocks;
+  for (int d = tid; d < hd; d += 128) qs[d] = to_f(q[((size_t)t * nh + h) * hd + d]);
+  int first = 0;
+  if (window > 0 && P - window + 1 > 0) first = P - window + 1;
+  if (chunk > 0) first = max(first, P - P % chunk);
+  const int vh = kvh / v_share, nv = nkv / v_share;
+  float m = sink ? sink[h] : -INFINITY, l = sink ? 1.f : 0.f;
+  const int nd = vd >> 2, G = 128 / nd;
+  const int grp = tid / nd, d4 = tid - grp * nd;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int kept = min(keep, first);
+  const float slope = slopes ? slopes[h] : 0.f;
+  __syncthreads();
+  for (int c0 = kept > 0 ? 0 : (first / 128) * 128; c0 <= P; c0 += 128) {
+    if (c0 >= kept) c0 = max(c0, (first / 128) * 128);
+    const int j = c0 + tid;
+    const bool visible = (j >= first || j < kept) && j <= P;
+    float s = -INFINITY;
+    int slot = -1;
+    if (visible) {
+      const int page = table[j / page_size];
+      slot = page * page_size + (j % page_size);
+      const T* kr = k_cache + ((size_t)slot * nkv + kvh) * hd;
+      float4 dot = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 16
+      for (int d = 0; d < hd; d += 4) {
+        const float4 a = load4(kr + d), b = *reinterpret_cast<const float4*>(qs + d);
+        dot.x = fmaf(b.x, a.x, dot.x), dot.y = fmaf(b.y, a.y, dot.y), dot.z = fmaf(b.z, a.z, dot.z), dot.w = fmaf(b.w, a.w, dot.w);
+      }
+      s = ((dot.x + dot.y) + (dot.z + dot.w)) * scale;
+      if (softcap > 0.f) s = softcap * tanhf(s / softcap);
+      s -= slope * (float)(P - j);
+    }
+    pages[tid] = slot;
+    const float cmax = block_max(s, scratch);
+    const float m_new = fmaxf(m, cmax);
+    const float p = visible ? expf(s - m_new) : 0.f;
+    ps[tid] = p;
+    const float csum = block_sum(p, scratch);  // also orders the writes of ps / pages
+    const float corr = (m == -INFINITY) ? 0.f : expf(m - m_new);
+    l = l * corr + csum;
+    acc.x *= corr, acc.y *= corr, acc.z *= corr, acc.w *= corr;
+    const int n_in = min(128, P - c0 + 1);
+    if (grp < G) {
+#pragma unroll 8
+      for (int i = grp; i < n_in; i += G) {
+        const int sl = pages[i];
+        const float4 v = sl >= 0 ? load4(v_cache + ((size_t)sl * nv + vh) * vd + 4 * d4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float pi = ps[i];
+        acc.x = fmaf(pi, v.x, acc.x), acc.y = fmaf(pi, v.y, acc.y), acc.z = fmaf(pi, v.z, acc.z), acc.w = fmaf(pi, v.w, acc.w);
+      }
+    }
+    m = m_new;
+    __syncthreads();
+  }
+  if (grp < G) *reinterpret_cast<float4*>(sums + grp * vd + 4 * d4) = acc;
+  __syncthreads();
+  TO* o = out + ((size_t)t * nh + h) * vd;
+  for (int d = tid; d < vd; d += 128) {
+    float total = 0.f;
+    for (int g = 0; g < G; ++g) total += sums[g * vd + d];
+    o[d] = from_f<TO>(total / l);
+  }
+}
+
 ALOFA_API int alofa_paged_attention_generic(void* out, const void* q, const void* k_cache, const void* v_cache,
                                             const int* positions, const int* seq_of_token, const int* block_table,
                                             int max_blocks, int page_size, int n_tokens, int nh, int nkv, int hd,
@@ -367,18 +622,18 @@ ALOFA_API int alofa_paged_attention_generic(void* out, const void* q, const void
   if (n_tokens <= 0) return ALOFA_OK;
   if (hd <= 0 || vd <= 0 || vd > 256 || nkv <= 0 || nh % nkv != 0 || page_size <= 0 || chunk < 0 || v_share <= 0 || nkv % v_share != 0 || keep < 0) return ALOFA_ERR_ARGUMENT;
   dim3 grid(n_tokens, nh);
-  const size_t smem = (size_t)(hd + 128) * sizeof(float);
-  if (is_bf16 && out_f32)
-    paged_attention_generic_kernel<bf16, float><<<grid, 128, smem, stream>>>(
-        (float*)out, (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, positions, seq_of_token, block_table,
-        max_blocks, page_size, nh, nkv, hd, vd, window, scale, softcap, sink, chunk, v_share, keep, slopes);
-  else if (is_bf16)
-    paged_attention_generic_kernel<bf16, bf16><<<grid, 128, smem, stream>>>(
-        (bf16*)out, (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, positions, seq_of_token, block_table,
-        max_blocks, page_size, nh, nkv, hd, vd, window, scale, softcap, sink, chunk, v_share, keep, slopes);
-  else
-    paged_attention_generic_kernel<float, float><<<grid, 128, smem, stream>>>(
-        (float*)out, (const float*)q, (const float*)k_cache, (const float*)v_cache, positions, seq_of_token, block_table,
-        max_blocks, page_size, nh, nkv, hd, vd, window, scale, softcap, sink, chunk, v_share, keep, slopes);
+  auto launch = [&](auto* o, const auto* queries) {
+    using TO = std::remove_pointer_t<decltype(o)>;
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(queries)>>;
+    // rows of whole groups of four numbers, which then lie on the 16 (bfloat16: 8) bytes a load takes
+    const bool vector = hd % 4 == 0 && vd % 4 == 0 && ((uintptr_t)k_cache | (uintptr_t)v_cache) % (4 * sizeof(T)) == 0;
+    const size_t smem = (size_t)(hd + 128 + (vector ? 128 / (vd / 4) * vd : 0)) * sizeof(float);
+    launch_dep(vector ? paged_attention_vector_kernel<T, TO> : paged_attention_generic_kernel<T, TO>, grid, 128, smem, stream,
+               o, queries, (const T*)k_cache, (const T*)v_cache, positions, seq_of_token, block_table,
+               max_blocks, page_size, nh, nkv, hd, vd, window, scale, softcap, sink, chunk, v_share, keep, slopes);
+  };
+  if (is_bf16 && out_f32) launch((float*)out, (const bf16*)q);
+  else if (is_bf16) launch((bf16*)out, (const bf16*)q);
+  else launch((float*)out, (const float*)q);
   return launch_status();
 }

@@ -640,3 +640,26 @@ def test_sample_chain_against_plain(ops, vocab):
         if g != w:  # allowed only when u sits within fp32 rounding of a CDF step
             cdf = np.cumsum(dist)
             assert dist[g] > 0 and min(abs(u - cdf[w]), abs(u - (cdf[w - 1] if w else 0.0))) < 1e-5, (g, w)
+
+
+@pytest.mark.parametrize("k", [4, 128, 132, 2048, 2052, 4864])
+def test_32_bit_products_sum_a_row_the_same_way_in_every_batch(ops, k):
+    """One, two, up to four and up to eight rows a warp, with columns left over in the last warp and depths either side of a
+    run of 128 and of a round of 16 runs: every row as in the plain implementation, and bit for bit what it is alone."""
+    rng = np.random.default_rng(k)
+    for n in (1, 9, 37):
+        x, w = rng.normal(size=(19, k)).astype(np.float32), (rng.normal(size=(2 * n, k)) / np.sqrt(k)).astype(np.float32)
+        bias, res = rng.normal(size=2 * n).astype(np.float32), rng.normal(size=(19, n)).astype(np.float32)
+        first = None
+        for m in (1, 2, 3, 4, 5, 8, 19):
+            store, gated, add = torch.empty(m, n, device="cuda"), torch.empty(m, n, device="cuda"), dev(res[:m])
+            ops.gemm_generic(store, dev(x[:m]), dev(w[:n]), dev(bias[:n]), ops.EPI_STORE, ops.ACTIVATIONS["relu"])
+            ops.gemm_generic(gated, dev(x[:m]), dev(w), dev(bias), ops.EPI_GATED)
+            ops.gemm_generic(add, dev(x[:m]), dev(w[:n]), None, ops.EPI_RESIDUAL)
+            rows = [t.cpu().numpy() for t in (store, gated, add)]
+            first = first or [r[0] for r in rows]
+            assert all(np.array_equal(r[0], f) for r, f in zip(rows, first)), f"m={m} n={n}: row 0 depends on the rows beside it"
+        sums = plain.linear(x, w, bias)
+        assert_close(rows[0], np.maximum(sums[:, :n], 0), TOL[F32], f"store n={n}")
+        assert_close(rows[1], plain.silu(sums[:, :n]) * sums[:, n:], TOL[F32], f"gated n={n}")
+        assert_close(rows[2], res + plain.linear(x, w[:n]), TOL[F32], f"residual n={n}")
