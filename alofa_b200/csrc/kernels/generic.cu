@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(256) gemm_generic_kernel(TO* __restrict__ out,
 // bytes: one row takes one column a warp, with up to 16 loads of 16 bytes a lane in flight and the first of them ahead of
 // the dependency wait, where the 64 x 64 tiles above kept 14 of 148 SMs busy (one row, output and down projection of 896
 // columns: 318 -> 3.7 us on average; gate and up 244 -> 6.5 us, 5.4 TB/s).  Many rows are bound by the reads of x and w
-// through L1: 8 x 4 sums a lane from 12 such reads (40 rows, gate and up: 57 us).
+// through L1: 8 x 4 sums a lane from 12 such reads (40 rows, gate and up: 57 us), 16 x 8 from 24 over the rows of a prompt.
 template <int V>
 __device__ __forceinline__ float reduce_across_lanes(float (&v)[V], int lane) {  // value i ends in the lanes i * (32 / V) ..
   int o = 16;
@@ -247,13 +247,13 @@ __device__ __forceinline__ float reduce_across_lanes(float (&v)[V], int lane) { 
   return s;
 }
 
-template <int MT, int NT, int EPI>
+template <int MT, int NT, int EPI, int WM = 1>  // WM: warps of a block side by side along the rows of x, the other 8 / WM along the columns
 __global__ void __launch_bounds__(256) gemm_f32_kernel(float* out, const float* x, const float* __restrict__ w, const float* __restrict__ bias, int M, int N, int K, int act,
                                                        float gate_alpha, float gate_limit) {
   constexpr int NW = EPI == EPI_GATED ? 2 : 1, R = NT * NW, V = MT * R;
   constexpr int U = V == 1 ? 16 : R >= 8 ? 1 : 8 / R;  // runs of 128 whose weights are asked for together
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = (blockIdx.x * 8 + warp) * NT, m0 = blockIdx.y * MT;
+  const int n0 = (blockIdx.x * (8 / WM) + warp / WM) * NT, m0 = (blockIdx.y * WM + warp % WM) * MT;
   const int k4 = K >> 2;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   const float4* wr[R];  // columns past the last read the last one's weights, and are not stored
@@ -291,35 +291,48 @@ __global__ void __launch_bounds__(256) gemm_f32_kernel(float* out, const float* 
     }
     load_weights(c + 32 * U);
   }
-  float v = reduce_across_lanes<V>(acc, lane);
-  const int i = lane / (32 / V);  // the value this lane holds: row i / R, column (i % R) / NW, its gate or up sum
-  const int m = m0 + i / R, n = n0 + (i % R) / NW;
-  if (EPI == EPI_GATED) {
-    float u = __shfl_xor_sync(0xffffffffu, v, 32 / V);  // the up sum beside the gate's
-    if (i % NW || m >= M || n >= N || lane % (32 / V)) return;
-    if (bias) v += bias[n], u += bias[N + n];
-    out[(size_t)m * N + n] = gate_times(v, u, gate_alpha, gate_limit);
-    return;
+  constexpr int G = V > 32 ? 32 : V;  // values reduced together: value i of a group ends in the lanes i * (32 / G) ..
+#pragma unroll
+  for (int g = 0; g < V; g += G) {
+    float part[G];
+#pragma unroll
+    for (int j = 0; j < G; ++j) part[j] = acc[g + j];
+    float v = reduce_across_lanes<G>(part, lane);
+    const int i = g + lane / (32 / G);  // the value this lane holds: row i / R, column (i % R) / NW, its gate or up sum
+    const int m = m0 + i / R, n = n0 + (i % R) / NW;
+    float u = 0.f;
+    if (EPI == EPI_GATED) u = __shfl_xor_sync(0xffffffffu, v, 32 / G);  // the up sum beside the gate's
+    if (m >= M || n >= N || lane % (32 / G) || (EPI == EPI_GATED && i % NW)) continue;
+    float* o = out + (size_t)m * N + n;
+    if (EPI == EPI_GATED) {
+      if (bias) v += bias[n], u += bias[N + n];
+      *o = gate_times(v, u, gate_alpha, gate_limit);
+    } else {
+      if (bias) v += bias[n];
+      *o = EPI == EPI_RESIDUAL ? *o + v : activate(v, act);
+    }
   }
-  if (m >= M || n >= N || lane % (32 / V)) return;
-  if (bias) v += bias[n];
-  float* o = out + (size_t)m * N + n;
-  *o = EPI == EPI_RESIDUAL ? *o + v : activate(v, act);
 }
 
 template <int EPI>
 static int gemm_f32_launch(float* out, const float* x, const float* w, const float* bias, int M, int N, int K, int act, float gate_alpha, float gate_limit, cudaStream_t stream) {
   constexpr int NW = EPI == EPI_GATED ? 2 : 1;
-  auto launch = [&](auto kernel, int mt, int nt) {
-    const long long rows = (M + mt - 1) / mt;
+  auto launch = [&](auto kernel, int mt, int nt, int wm) {
+    const long long rows = (M + mt * wm - 1) / (mt * wm);
     if (rows > 65535) return ALOFA_ERR_ARGUMENT;
-    launch_dep(kernel, dim3((N + 8 * nt - 1) / (8 * nt), (unsigned)rows), 256, 0, stream, out, x, w, bias, M, N, K, act, gate_alpha, gate_limit);
+    const int columns = 8 / wm * nt;
+    launch_dep(kernel, dim3((N + columns - 1) / columns, (unsigned)rows), 256, 0, stream, out, x, w, bias, M, N, K, act, gate_alpha, gate_limit);
     return launch_status();
   };
-  if (M == 1) return launch(gemm_f32_kernel<1, 1, EPI>, 1, 1);
-  if (M == 2) return launch(gemm_f32_kernel<2, 2 / NW, EPI>, 2, 2 / NW);
-  if (M <= 4) return launch(gemm_f32_kernel<4, 2 / NW, EPI>, 4, 2 / NW);
-  return launch(gemm_f32_kernel<8, 4 / NW, EPI>, 8, 4 / NW);
+  if (M == 1) return launch(gemm_f32_kernel<1, 1, EPI>, 1, 1, 1);
+  if (M == 2) return launch(gemm_f32_kernel<2, 2 / NW, EPI>, 2, 2 / NW, 1);
+  if (M <= 4) return launch(gemm_f32_kernel<4, 2 / NW, EPI>, 4, 2 / NW, 1);
+  // Prompts: 16 x 8 sums a lane, 32 x 32 outputs a block, once such blocks come near filling the SMs and their rows are mostly
+  // there (us at 8 x 4 / 16 x 8 sums: 40 x 9,728 of depth 896 45 / 50, 64 rows 69 / 50; 128 x 896 of depth 896 17.7 / 14.9;
+  // 64 x 896 of depth 4,864, 56 blocks, 39 / 48, 128 rows, 112 blocks, 74 / 48; 2,048 rows 1,139 / 649).
+  const long long blocks = (long long)((N + 32 / NW - 1) / (32 / NW)) * ((M + 31) / 32);
+  if (M >= 48 && blocks >= 112) return launch(gemm_f32_kernel<16, 8 / NW, EPI, 2>, 16, 8 / NW, 2);
+  return launch(gemm_f32_kernel<8, 4 / NW, EPI>, 8, 4 / NW, 1);
 }
 
 template <typename TA, typename TW, typename TO>

@@ -663,3 +663,27 @@ def test_32_bit_products_sum_a_row_the_same_way_in_every_batch(ops, k):
         assert_close(rows[0], np.maximum(sums[:, :n], 0), TOL[F32], f"store n={n}")
         assert_close(rows[1], plain.silu(sums[:, :n]) * sums[:, n:], TOL[F32], f"gated n={n}")
         assert_close(rows[2], res + plain.linear(x, w[:n]), TOL[F32], f"residual n={n}")
+
+
+@pytest.mark.parametrize("k", [4, 132, 896])
+def test_32_bit_products_over_prompts(ops, k):
+    """The blocks of 32 x 32 outputs that many rows take, with rows and columns left over: as the plain implementation, and
+    bit for bit what a row is alone."""
+    rng = np.random.default_rng(k)
+    m, n = 53, 1797
+    x, w = rng.normal(size=(m, k)).astype(np.float32), (rng.normal(size=(2 * n, k)) / np.sqrt(k)).astype(np.float32)
+    bias, res = rng.normal(size=2 * n).astype(np.float32), rng.normal(size=(m, n)).astype(np.float32)
+    sums, got = plain.linear(x, w, bias), {}
+    for rows in (slice(0, m), slice(0, 1), slice(m - 1, m)):
+        count = rows.stop - rows.start
+        store, gated, add = torch.empty(count, n, device="cuda"), torch.empty(count, n, device="cuda"), dev(res[rows])
+        ops.gemm_generic(store, dev(x[rows]), dev(w[:n]), dev(bias[:n]), ops.EPI_STORE)
+        ops.gemm_generic(gated, dev(x[rows]), dev(w), dev(bias), ops.EPI_GATED)
+        ops.gemm_generic(add, dev(x[rows]), dev(w[:n]), None, ops.EPI_RESIDUAL)
+        got[rows.start, count] = [t.cpu().numpy() for t in (store, gated, add)]
+    whole = got[0, m]
+    for (at, count), alone in got.items():
+        assert all(np.array_equal(a, b[at : at + count]) for a, b in zip(alone, whole)), f"row {at} depends on the rows beside it"
+    assert_close(whole[0], sums[:, :n], TOL[F32], "store")
+    assert_close(whole[1], plain.silu(sums[:, :n]) * sums[:, n:], TOL[F32], "gated")
+    assert_close(whole[2], res + plain.linear(x, w[:n]), TOL[F32], "residual")
