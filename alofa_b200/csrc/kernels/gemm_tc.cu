@@ -672,8 +672,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
 // The epilogue of a 128-token tile whose width is a multiple of 4: warp q owns
 // rows [32q, 32q + 32) of the accumulator at `tmem_acc`; `staging` holds
-// 4 x 32 rows of 132 floats.  Two warps share a quarter: `half` (0 or 1) takes columns
-// [64 half, 64 half + 64) of every 128 and rows [16 half, 16 half + 16) of the stores; they meet
+// 4 x 32 rows of 64 floats.  Two warps share a quarter: `half` (0 or 1) takes columns
+// [32 half, 32 half + 32) of every 64 and rows [16 half, 16 half + 16) of the stores; they meet
 // on the named barrier 8 + q.  `release` (optional, one arrival per warp) is signalled once the
 // accumulator has been read out.
 __device__ __forceinline__ void quarter_sync(int q) { asm volatile("bar.sync %0, 64;" ::"r"(8 + q) : "memory"); }
@@ -692,27 +692,36 @@ __device__ __forceinline__ bool epilogue_warps_agree(bool ok) {
   return any_bad == 0;
 }
 
-template <int BNF, int EPI>
-__device__ __forceinline__ void tokens_epilogue_staged(const GemmArgs& args, uint32_t tmem_base, float* staging, int q, int half, int lane, int f0,
+template <int EPI>
+__device__ __forceinline__ void tokens_epilogue_staged(const GemmArgs& args, const int FEATS, uint32_t tmem_base, float* staging, int q, int half, int lane, int f0,
                                                        int t0, int n_splits, int split_index, uint64_t* release, uint32_t release_in_cluster = 0) {
-  constexpr bool GATED = EPI == EPI_GATED;
-  constexpr int FEATS = GATED ? BNF / 2 : BNF;
-  // The accumulator rows go through shared memory so
-  // that global memory is written a whole row of 128 features at a time:
-  // each thread drops its row's values into a padded tile, then the warp
-  // walks the 32 rows with one 16-byte access per lane.
-  constexpr int PITCH = 132;  // floats per staged row: 128 + padding against bank conflicts
-  float* stage = staging + (size_t)q * 32 * PITCH;
+  constexpr bool GATED = EPI == EPI_GATED;  // FEATS: output features of the tile, a multiple of 16
+  // The accumulator rows go through shared memory so that global memory is written whole rows of 64 features at a time:
+  // each thread drops its row's values into a tile whose groups of four are permuted by the row (no bank is hit twice, and
+  // no padding takes room from the ring), then the warps walk the rows with one 16-byte access per lane, two rows at once.
+  float* stage = staging + (size_t)q * 32 * 64;
+  auto group = [&](int row, int c) { return reinterpret_cast<float4*>(stage + row * 64 + ((c ^ (row & 15)) << 2)); };
   const bool split = n_splits > 1;
   const int N = args.N;
   const size_t plane = (size_t)args.T * N;
+  const int sub = lane >> 4, c4 = lane & 15;
+  const int r_lo = half * 16 + sub, rows = args.T - (t0 + q * 32);  // this lane stores rows r_lo, r_lo + 2, .. r_lo + 14 below `rows`
 #pragma unroll 1
-  for (int cb = 0; cb < FEATS; cb += 128) {
+  for (int cb = 0; cb < FEATS; cb += 64) {
     if (f0 + cb >= N) break;
+    const int f = f0 + cb + c4 * 4;  // this lane's four features of the rows it stores
+    const bool f_ok = f < N && cb + c4 * 4 < FEATS;  // N % 4 == 0: a group is inside or outside as a whole
+    const size_t at = (size_t)(t0 + q * 32) * N + f;
+    float4 b[EPI == EPI_RESIDUAL ? 8 : 1];
+    if (EPI == EPI_RESIDUAL && !split && f_ok) {  // the rows to add to: their loads run beside the staging
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (r_lo + 2 * i < rows) b[i] = *reinterpret_cast<const float4*>((float*)args.out + at + (size_t)(r_lo + 2 * i) * N);
+    }
 #pragma unroll 1
-    for (int c0 = half * 64; c0 < half * 64 + 64 && cb + c0 < FEATS; c0 += 16) {
-      const int f = f0 + cb + c0;
-      if (f >= N) break;
+    for (int c0 = half * 32; c0 < half * 32 + 32 && cb + c0 < FEATS; c0 += 16) {
+      const int g = f0 + cb + c0;
+      if (g >= N) break;
       uint32_t r0[16], r1[16];
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(cb + c0);
       tmem_ld16(taddr, r0);
@@ -723,17 +732,17 @@ __device__ __forceinline__ void tokens_epilogue_staged(const GemmArgs& args, uin
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           float a = __uint_as_float(r0[j]), u = __uint_as_float(r1[j]);
-          if (args.bias && f + j < N) a += args.bias[f + j], u += args.bias[N + f + j];
+          if (args.bias && g + j < N) a += args.bias[g + j], u += args.bias[N + g + j];
           v[j] = clamped_gate_times(a, u, args.gate_alpha, args.gate_limit);
         }
       } else {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           float a = __uint_as_float(r0[j]);
-          if (!split && args.bias && f + j < N) a += args.bias[f + j];
+          if (!split && args.bias && g + j < N) a += args.bias[g + j];
           if (GATED) {
             float u = __uint_as_float(r1[j]);
-            if (args.bias && f + j < N) u += args.bias[N + f + j];
+            if (args.bias && g + j < N) u += args.bias[N + g + j];
             a = silu_times(a, u);
           }
           v[j] = a;
@@ -741,9 +750,9 @@ __device__ __forceinline__ void tokens_epilogue_staged(const GemmArgs& args, uin
       }
       if (EPI == EPI_STORE && !split && args.act) activate_sixteen(v, args.act);
 #pragma unroll
-      for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(stage + lane * PITCH + c0 + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+      for (int j = 0; j < 16; j += 4) *group(lane, (c0 + j) >> 2) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
     }
-    const bool read_out = (release || release_in_cluster) && (cb + 128 >= FEATS || f0 + cb + 128 >= N);
+    const bool read_out = (release || release_in_cluster) && (cb + 64 >= FEATS || f0 + cb + 64 >= N);
     if (read_out) tc_fence_before();  // the accumulator is read out: the next tile but one may have it
     __syncwarp();
     if (read_out && lane == 0) {  // one arrival per warp: arrivals at a barrier of the other CTA are dear
@@ -751,45 +760,30 @@ __device__ __forceinline__ void tokens_epilogue_staged(const GemmArgs& args, uin
       else mbar_arrive(release);
     }
     quarter_sync(q);  // both halves of the columns are staged
-    const int f = f0 + cb + lane * 4;  // this lane's four features of every row
-    const bool f_ok = f < N && cb + lane * 4 < FEATS;  // N % 4 == 0: a group is inside or outside as a whole
-    const int r_lo = half * 16;
-    const int rows = min(r_lo + 16, args.T - (t0 + q * 32));  // this warp stores rows [r_lo, rows)
     if (f_ok) {
-      if (split) {
-        float* p = args.partial + (size_t)split_index * plane + (size_t)(t0 + q * 32) * N + f;
-#pragma unroll 4
-        for (int r = r_lo; r < rows; ++r) *reinterpret_cast<float4*>(p + (size_t)r * N) = *reinterpret_cast<const float4*>(stage + r * PITCH + lane * 4);
-      } else if (EPI == EPI_RESIDUAL) {
-        float* o = (float*)args.out + (size_t)(t0 + q * 32) * N + f;
-        {  // sixteen rows: all their loads in flight, then the stores
-          const int rb = r_lo;
-          float4 b[16];
+      if (split || EPI == EPI_RESIDUAL || !args.out_bf16) {
+        float* o = (split ? args.partial + (size_t)split_index * plane : (float*)args.out) + at;
 #pragma unroll
-          for (int r = 0; r < 16; ++r)
-            if (rb + r < rows) b[r] = *reinterpret_cast<float4*>(o + (size_t)(rb + r) * N);
-#pragma unroll
-          for (int r = 0; r < 16; ++r)
-            if (rb + r < rows) {
-              const float4 a = *reinterpret_cast<const float4*>(stage + (rb + r) * PITCH + lane * 4);
-              *reinterpret_cast<float4*>(o + (size_t)(rb + r) * N) = make_float4(b[r].x + a.x, b[r].y + a.y, b[r].z + a.z, b[r].w + a.w);
-            }
+        for (int i = 0; i < 8; ++i) {
+          const int r = r_lo + 2 * i;
+          if (r >= rows) break;
+          float4 a = *group(r, c4);
+          if (EPI == EPI_RESIDUAL && !split) a = make_float4(b[i].x + a.x, b[i].y + a.y, b[i].z + a.z, b[i].w + a.w);
+          *reinterpret_cast<float4*>(o + (size_t)r * N) = a;
         }
-      } else if (args.out_bf16) {
-        bf16* o = (bf16*)args.out + (size_t)(t0 + q * 32) * N + f;
-#pragma unroll 4
-        for (int r = r_lo; r < rows; ++r) {
-          const float4 a = *reinterpret_cast<const float4*>(stage + r * PITCH + lane * 4);
+      } else {
+        bf16* o = (bf16*)args.out + at;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int r = r_lo + 2 * i;
+          if (r >= rows) break;
+          const float4 a = *group(r, c4);
           __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);
           *reinterpret_cast<uint2*>(o + (size_t)r * N) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
         }
-      } else {
-        float* o = (float*)args.out + (size_t)(t0 + q * 32) * N + f;
-#pragma unroll 4
-        for (int r = r_lo; r < rows; ++r) *reinterpret_cast<float4*>(o + (size_t)r * N) = *reinterpret_cast<const float4*>(stage + r * PITCH + lane * 4);
       }
     }
-    quarter_sync(q);  // the staged rows are stored: the next 128 columns, or the next tile, may overwrite them
+    quarter_sync(q);  // the staged rows are stored: the next 64 columns, or the next tile, may overwrite them
   }
 }
 
@@ -914,7 +908,7 @@ gemm_tc_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     if (no_tile) {
       // nothing to store
     } else if (ok && staged && t0 + q * 32 < args.T) {
-      tokens_epilogue_staged<BNF, EPI>(args, tmem_base, reinterpret_cast<float*>(tiles), q, half, lane, f0, t0, (int)gridDim.z, (int)blockIdx.z, nullptr);
+      tokens_epilogue_staged<EPI>(args, FEATS, tmem_base, reinterpret_cast<float*>(tiles), q, half, lane, f0, t0, (int)gridDim.z, (int)blockIdx.z, nullptr);
     } else if (ok && t0 + q * 32 < args.T) {
       // widths that are no multiple of 4 (or gated partial sums): element-wise, straight from the registers
       const bool split = gridDim.z > 1;
@@ -1031,15 +1025,17 @@ gemm_tc_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
 // beside the MMAs of the next.  Tiles are taken feature-tile first, so CTAs
 // that run side by side read the same tokens and neighbouring weights.
 // ---------------------------------------------------------------------------
-constexpr int STAGING_BYTES = 4 * 32 * 132 * 4;  // the epilogue's padded rows
+constexpr int STAGING_BYTES = 4 * 32 * 64 * 4;  // the epilogue's rows
 // ROWS (32 or 64 instead of 128: an output head in a decode step of up to that many tokens): only
 // ROWS rows of the token tile are fetched - the MMA reads 128, the rest from whatever follows in
 // shared memory, and their accumulator rows are never read - and only ROWS / 32 quarters of the
-// epilogue have rows, so a stage is 36 or 40 KB instead of 48 and the ring five or four deep
-// instead of three: more weight bytes in flight per SM.
+// epilogue have rows, so a stage is 36 or 40 KB instead of 48 and the ring six or five deep
+// instead of four: more weight bytes in flight per SM.  (With 128 rows a ring of four stages, which
+// the staging tile's 32 KB leave room for, against three beside 67 KB: 2,048 tokens, depth 896, 9,728
+// weight rows 33.0 -> 31.4 us.)
 template <int ROWS>
 struct PersistentRing {
-  static constexpr int STAGES = ROWS == 32 ? 5 : ROWS == 64 ? 4 : 3;
+  static constexpr int STAGES = ROWS == 32 ? 6 : ROWS == 64 ? 5 : 4;
   static constexpr uint32_t A_BYTES = ROWS * BK * 2;
   static constexpr uint32_t STAGING = STAGING_BYTES / 128 * ROWS;
 };
@@ -1166,7 +1162,7 @@ gemm_tc_tokens_persistent_kernel(const __grid_constant__ CUtensorMap map_w, cons
       if (!epilogue_warps_agree(ok)) break;
       tc_fence_after();
       if (t0 + q * 32 < args.T) {
-        tokens_epilogue_staged<BNF, EPI>(args, tmem_base + buf * BNF, staging, q, half, lane, f0, t0, 1, 0, &acc_free[buf]);
+        tokens_epilogue_staged<EPI>(args, FEATS, tmem_base + buf * BNF, staging, q, half, lane, f0, t0, 1, 0, &acc_free[buf]);
       } else {
         tc_fence_before();
         __syncwarp();
@@ -1191,12 +1187,12 @@ gemm_tc_tokens_persistent_kernel(const __grid_constant__ CUtensorMap map_w, cons
 // half of the weight rows (for EPI_GATED the first CTA the gate rows, the
 // second the matching up rows), 32 KB per k-slice where the single CTA fetches
 // 48 KB for the same MMA time: the product is no longer bound by what an SM can
-// pull out of L2, and the ring is four stages deep.  The first CTA's full
+// pull out of L2, and the ring is six stages deep.  The first CTA's full
 // barrier counts the bytes of both CTAs' copies; the MMAs' completion is
 // signalled on the barriers of both; both CTAs' epilogue warps free an
 // accumulator on the first CTA's barrier.
 // ---------------------------------------------------------------------------
-constexpr int PAIR_STAGES = 4;
+constexpr int PAIR_STAGES = 6;
 
 template <int EPI>
 __global__ void __launch_bounds__(TOKENS_THREADS, 1)
@@ -1221,8 +1217,12 @@ gemm_tc_tokens_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
   const bool first = rank == 0;
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const int n_ftiles = (args.N + FEATS - 1) / FEATS, n_ttiles = (args.T + 255) / 256;
-  const int n_tiles = n_ftiles * n_ttiles;
-  const int n_slices = (args.K + BK - 1) / BK;
+  const int total_slices = (args.K + BK - 1) / BK, per_split = args.k_slices_per_split;
+  const int n_splits = (total_slices + per_split - 1) / per_split;
+  const int n_tiles = n_ftiles * n_ttiles * n_splits;  // feature tiles innermost, parts of the depth outermost
+  auto split_of = [&](int tile) { return tile / (n_ftiles * n_ttiles); };
+  auto token_of = [&](int tile) { return tile / n_ftiles % n_ttiles * 256 + (int)rank * 128; };
+  auto slices_of = [&](int tile) { return min(per_split, total_slices - split_of(tile) * per_split); };
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
@@ -1243,7 +1243,7 @@ gemm_tc_tokens_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
   const uint32_t tmem_base = tmem_base_smem;
   // this CTA's weight rows of a tile that starts at feature f0
   auto weight_row = [&](int f0) { return GATED ? (first ? f0 : args.N + f0) : f0 + (int)rank * (BNF / 2); };
-  auto load_weights = [&](int it, int i, int f0) {  // the weight tile of slice i of a tile into the stage of ring position it
+  auto load_weights = [&](int it, int i, int f0) {  // the weight tile of slice i of the depth into the stage of ring position it
     const int s = it % PAIR_STAGES;
     if (first) mbar_expect_tx(&full_bar[s], 2 * STAGE_BYTES);
     tma_load_2d_pair(tiles + (size_t)s * STAGE_BYTES + A_BYTES, &map_w, in_cluster_cta(&full_bar[s], 0), i * BK, weight_row(f0));
@@ -1253,8 +1253,8 @@ gemm_tc_tokens_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
   if (threadIdx.x == 0) {
     asm volatile("griddepcontrol.launch_dependents;");
     if (pair < n_tiles) {
-      early_slices = min(PAIR_STAGES, n_slices);
-      for (int i = 0; i < early_slices; ++i) load_weights(i, i, (pair % n_ftiles) * FEATS);
+      early_slices = min(PAIR_STAGES, slices_of(pair));
+      for (int i = 0; i < early_slices; ++i) load_weights(i, split_of(pair) * per_split + i, (pair % n_ftiles) * FEATS);
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
   } else {
@@ -1265,12 +1265,13 @@ gemm_tc_tokens_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
     if (lane == 0) {
       int it = 0;  // slices asked for so far, over all tiles
       for (int tile = pair; tile < n_tiles; tile += n_pairs) {
-        const int f0 = (tile % n_ftiles) * FEATS, t0 = (tile / n_ftiles) * 256 + (int)rank * 128;
+        const int f0 = (tile % n_ftiles) * FEATS, t0 = token_of(tile);
+        const int slice0 = split_of(tile) * per_split, n_slices = slices_of(tile);
         for (int i = 0; i < n_slices; ++i, ++it) {
           const int s = it % PAIR_STAGES;
           if (it >= PAIR_STAGES && !mbar_wait(&empty_bar[s], ((it / PAIR_STAGES) - 1) & 1, &abort_flag)) break;
-          if (it >= early_slices) load_weights(it, i, f0);
-          tma_load_2d_pair(tiles + (size_t)s * STAGE_BYTES, &map_x, in_cluster_cta(&full_bar[s], 0), i * BK, t0);
+          if (it >= early_slices) load_weights(it, slice0 + i, f0);
+          tma_load_2d_pair(tiles + (size_t)s * STAGE_BYTES, &map_x, in_cluster_cta(&full_bar[s], 0), (slice0 + i) * BK, t0);
         }
         if (abort_flag) break;
       }
@@ -1284,6 +1285,7 @@ gemm_tc_tokens_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
         if (j >= 2) ok = mbar_wait(&acc_free[buf], ((j >> 1) - 1) & 1, &abort_flag);
         if (!ok) break;
         tc_fence_after();
+        const int n_slices = slices_of(tile);
         for (int i = 0; i < n_slices; ++i, ++it) {
           const int s = it % PAIR_STAGES;
           ok = mbar_wait(&full_bar[s], (it / PAIR_STAGES) & 1, &abort_flag);
@@ -1304,14 +1306,14 @@ gemm_tc_tokens_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
     int j = 0;
     for (int tile = pair; tile < n_tiles; tile += n_pairs, ++j) {
       const int buf = j & 1;
-      const int f0 = (tile % n_ftiles) * FEATS, t0 = (tile / n_ftiles) * 256 + (int)rank * 128;
+      const int f0 = (tile % n_ftiles) * FEATS, t0 = token_of(tile), split = split_of(tile);
       bool ok = mbar_wait(&acc_full[buf], (j >> 1) & 1, &abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       if (!epilogue_warps_agree(ok)) break;
       tc_fence_after();
       const uint32_t free_bar = in_cluster_cta(&acc_free[buf], 0);
       if (t0 + q * 32 < args.T) {
-        tokens_epilogue_staged<BNF, EPI>(args, tmem_base + buf * BNF, staging, q, half, lane, f0, t0, 1, 0, nullptr, free_bar);
+        tokens_epilogue_staged<EPI>(args, FEATS, tmem_base + buf * BNF, staging, q, half, lane, f0, t0, n_splits, split, nullptr, free_bar);
       } else {
         tc_fence_before();
         __syncwarp();
@@ -1469,26 +1471,6 @@ static int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const GemmArg
   return launch_status();
 }
 
-// Whether a tokens-on-M product runs on pairs of CTAs: a wide product over at least two token
-// tiles with more tiles than SMs, and deep (ALOFA_GEMM_PAIR=0 keeps one CTA per tile).  Measured
-// on 2,048 tokens: depth 3,584 x 37,888 weight rows 477 against 540 us, 18,944 x 3,584 233 against
-// 238 us, depth 1,536 x 17,920 rows 85 against 92 us; at depth 896 the pair's epilogue is not
-// hidden behind its shorter MMA phase and one CTA per tile is as fast or faster (32.7 against
-// 33.9 us for 9,728 weight rows), so shallow products stay there.
-constexpr int PAIR_MIN_DEPTH = 1024;
-static bool pair_product(int bnf, int splits, int T, int N, int K, int epi) {
-  static int sms = 0, allowed = -1;
-  if (allowed < 0) {
-    const char* env = getenv("ALOFA_GEMM_PAIR");
-    allowed = (env && env[0] == '0') ? 0 : 1;
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) sms = 0;
-  }
-  if (!allowed || sms < 2 || bnf != 256 || splits != 1 || (N & 3) || T <= 128 || K < PAIR_MIN_DEPTH) return false;
-  const int feats = epi == EPI_GATED ? 128 : 256;
-  return (long long)((N + feats - 1) / feats) * ((T + 127) / 128) > sms;
-}
-
 template <int EPI, int ROWS>
 static int launch_persistent(int sms, const CUtensorMap& mw, const CUtensorMap& mx, const GemmArgs& args, cudaStream_t stream) {
   static bool configured = false;
@@ -1553,7 +1535,7 @@ static int launch_tokens(const CUtensorMap& mw, const CUtensorMap& mx, const Gem
     prefer_max_shared(gemm_tc_tokens_kernel<BNF, EPI>);
     configured = true;
   }
-  if (BNF == 256 && splits == 1 && (args.N & 3) == 0 && (args.K <= 2048 || args.pair) && (!args.tile_batch || args.T >= BY_TILE_PERSISTENT_ROWS)) {
+  if (BNF == 256 && splits == 1 && (args.N & 3) == 0 && args.K <= 2048 && (!args.tile_batch || args.T >= BY_TILE_PERSISTENT_ROWS)) {
     // More tiles than SMs and a shallow depth, where a tile's epilogue is a large share of its
     // time: one resident CTA per SM works through the tiles, epilogues beside MMAs.  (Deep
     // products measured faster as two CTAs per SM, which keep four stages in flight per SM.)
@@ -1565,43 +1547,37 @@ static int launch_tokens(const CUtensorMap& mw, const CUtensorMap& mx, const Gem
       if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) sms = 0;
     }
     const int n_tiles = (int)(grid.x * grid.y);
-    if (args.pair) {
-      static bool configured_2 = false;
-      constexpr size_t SMEM_2 = (size_t)PAIR_STAGES * ((size_t)128 * BK * 2 + (size_t)128 * BK * 2) + STAGING_BYTES + 1024;
-      if (!configured_2) {
-        if (cudaFuncSetAttribute(gemm_tc_tokens_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_2) != cudaSuccess)
-          return ALOFA_ERR_LAUNCH;
-        prefer_max_shared(gemm_tc_tokens_pair_kernel<EPI>);
-        configured_2 = true;
-      }
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(sms / 2 * 2);
-      cfg.blockDim = dim3(TOKENS_THREADS);
-      cfg.dynamicSmemBytes = SMEM_2;
-      cfg.stream = stream;
-      cudaLaunchAttribute attr[2];
-      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
-      attr[1].id = cudaLaunchAttributeClusterDimension;
-      attr[1].val.clusterDim.x = 2;
-      attr[1].val.clusterDim.y = 1;
-      attr[1].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 2;
-      cudaLaunchKernelEx(&cfg, gemm_tc_tokens_pair_kernel<EPI>, mw, mx, args);
-      return launch_status();
-    }
     if (persistent && sms > 0 && n_tiles > sms && args.few == 32) return launch_persistent<EPI, 32>(sms, mw, mx, args, stream);
     if (persistent && sms > 0 && n_tiles > sms && args.few == 64) return launch_persistent<EPI, 64>(sms, mw, mx, args, stream);
     if (persistent && sms > 0 && n_tiles > sms) return launch_persistent<EPI, 128>(sms, mw, mx, args, stream);
   }
-  if (args.few || args.pair) return ALOFA_ERR_ARGUMENT;  // their maps have other boxes than this kernel's
+  if (args.few) return ALOFA_ERR_ARGUMENT;  // its map has another box than this kernel's
   launch_dep(gemm_tc_tokens_kernel<BNF, EPI>, grid, TOKENS_THREADS, smem, stream, mw, mx, args, stages);
+  return launch_status();
+}
+
+// The kernel on pairs of CTAs: as many pairs as there are tiles, and no more than the SMs hold.
+template <int EPI>
+static int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const GemmArgs& args, int splits, cudaStream_t stream) {
+  static int sms = 0;
+  constexpr size_t SMEM = (size_t)PAIR_STAGES * 2 * 128 * BK * 2 + STAGING_BYTES + 1024;
+  if (!sms) {
+    int device = 0, count = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || count < 2) return ALOFA_ERR_LAUNCH;
+    if (cudaFuncSetAttribute(gemm_tc_tokens_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) != cudaSuccess) return ALOFA_ERR_LAUNCH;
+    prefer_max_shared(gemm_tc_tokens_pair_kernel<EPI>);
+    sms = count;
+  }
+  const int feats = EPI == EPI_GATED ? 128 : 256;
+  const long long tiles = (long long)((args.N + feats - 1) / feats) * ((args.T + 255) / 256) * splits;
+  const int pairs = (int)(tiles < sms / 2 ? tiles : sms / 2);
+  launch_dep_cluster(gemm_tc_tokens_pair_kernel<EPI>, dim3(2 * pairs), TOKENS_THREADS, SMEM, stream, 2, mw, mx, args);
   return launch_status();
 }
 
 template <int EPI>
 static int dispatch_tokens(int bnf, const CUtensorMap& mw, const CUtensorMap& mx, const GemmArgs& args, int splits, cudaStream_t stream) {
+  if (args.pair) return launch_pair<EPI>(mw, mx, args, splits, stream);
   switch (bnf) {
     case 64: return launch_tokens<64, EPI>(mw, mx, args, splits, stream);
     case 128: return launch_tokens<128, EPI>(mw, mx, args, splits, stream);
@@ -1653,7 +1629,7 @@ ALOFA_API int alofa_gemm_tc(void* out, const void* x, const void* w, const float
                             int bn, int splits, int do_reduce, int* status, int b_kind, const float* b_src, const float* b_ml,
                             const int* b_positions, int b_heads, int b_head_dim, int b_window, int b_split_keys, long long* acc,
                             const long long* n_acc, const float* n_gamma, float n_eps, float* n_out, long long* n_zero, const int* tile_batch,
-                            int batches, float gate_alpha, float gate_limit, cudaStream_t stream) {
+                            int batches, float gate_alpha, float gate_limit, int pair, cudaStream_t stream) {
   if (T <= 0 || N <= 0) return ALOFA_OK;
   const int act = epi >> 4;  // EPI_STORE | (code << 4): an activation on the sums plus bias
   epi &= 15;
@@ -1684,7 +1660,7 @@ ALOFA_API int alofa_gemm_tc(void* out, const void* x, const void* w, const float
   const bool tokens_on_m = bn < 0;
   const int bnf = -bn;
   CUtensorMap mw, mx;
-  const bool pair = tokens_on_m && !tile_batch && pair_product(bnf, splits, T, N, K, epi);
+  if (pair && (bnf != 256 || tile_batch || N % 4 || T <= 128 || (epi == EPI_GATED && splits > 1))) return ALOFA_ERR_ARGUMENT;
   const int few = (tokens_on_m && !pair && !tile_batch) ? few_tokens_product(bnf, splits, T, N, K, epi) : 0;
   if (tokens_on_m) {
     const int w_box = (epi == EPI_GATED || pair) ? bnf / 2 : bnf;

@@ -72,7 +72,7 @@ def _gemm_tc():
     if lib is None:
         lib = load_library("alofa_gemm_tc", ["kernels/gemm_tc.cu"])
         lib.alofa_gemm_tc.restype = _I
-        lib.alofa_gemm_tc.argtypes = [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _P, _P, _P, _F, _P, _P, _P, _I, _F, _F, _P]
+        lib.alofa_gemm_tc.argtypes = [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _P, _P, _P, _F, _P, _P, _P, _I, _F, _F, _I, _P]
         lib.alofa_splitk_reduce.restype = _I
         lib.alofa_splitk_reduce.argtypes = [_P, _P, _P, _I, _I, _I, _I, _I, _F, _F, _P]
         lib.alofa_gemm_tc_reduces_in_cluster.restype = _I
@@ -380,7 +380,7 @@ B_ROWS, B_MERGED_SPLITS, B_NORMED = 0, 1, 2
 
 
 def gemm_tc(out, x, w, bias, epi: int, bn: int, splits: int = 1, partial=None, status=None, reduce: bool = True, computed=None, acc=None, act: int = 0,
-            tile_batch=None, batches: int = 1, gate=SILU_GATE) -> bool:
+            tile_batch=None, batches: int = 1, gate=SILU_GATE, pair: bool = False) -> bool:
     """Tensor-core product ``out = x @ w.T`` (bf16 operands, fp32 sums) with
     the epilogue fused.  Returns False, having launched nothing, when the
     kernel does not take these sizes (depth not a multiple of 8, unaligned).
@@ -404,7 +404,10 @@ def gemm_tc(out, x, w, bias, epi: int, bn: int, splits: int = 1, partial=None, s
     no bias): ``w`` is [batches * N, K] (gated: [batches * 2N, K], a batch's
     gate rows before its up rows) and the i-th tile of 128 token rows multiplies
     by the rows of batch ``tile_batch[i]``; a negative entry skips the tile.
-    ``gate`` (EPI_GATED): as in :func:`gemm_generic`."""
+    ``gate`` (EPI_GATED): as in :func:`gemm_generic`.
+
+    ``pair`` (``bn`` = -256, more than 128 tokens, N % 4 == 0; a gated product
+    unsplit): the kernel that runs on pairs of CTAs."""
     n = out.shape[1]
     rows_w = (2 * n if epi == EPI_GATED else n) * (batches if tile_batch is not None else 1)
     k = w.shape[1]
@@ -435,7 +438,7 @@ def gemm_tc(out, x, w, bias, epi: int, bn: int, splits: int = 1, partial=None, s
         _dev(status, "status", torch.int32) if status is not None else None,
         b_kind, b_src, b_ml, b_pos, heads, hd, window, split_keys,
         _dev(acc, "acc", i64) if acc is not None else None, n_acc, n_gamma, float(n_eps), n_out, n_zero,
-        _dev(tile_batch, "tile_batch", torch.int32) if tile_batch is not None else None, batches, float(gate[0]), float(gate[1]), _stream(),
+        _dev(tile_batch, "tile_batch", torch.int32) if tile_batch is not None else None, batches, float(gate[0]), float(gate[1]), 1 if pair else 0, _stream(),
     )
     if rc == 1:
         return False

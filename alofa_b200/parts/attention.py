@@ -178,7 +178,7 @@ class GQAttention(PagedAttend, Part):
 
     def scratch_row_bytes(self) -> int:
         # q/k/v, q, the attention output, and the output product's split sums
-        return 4 * (self.q_dim + 2 * self.kv_dim) + 2 * 4 * self.q_dim + 2 * 4 * self.hidden
+        return 4 * (self.q_dim + 2 * self.kv_dim) + 2 * 4 * self.q_dim + 4 * 4 * self.hidden
 
     def tensors(self):
         pre = self.prefix

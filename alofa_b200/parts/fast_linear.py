@@ -12,6 +12,8 @@ through most of the 148 SMs; the split partial sums are added in a fixed
 order, so a given (tokens, weight) pair always sums the same way."""
 from __future__ import annotations
 
+import os
+
 import torch
 
 from ..csrc import ops
@@ -68,6 +70,40 @@ def _splits(ctas: int, depth: int, deferrable: bool = False) -> int:
     return max(1, min(slices, SMS // ctas))
 
 
+PAIR_ROWS = 256  # tokens and weight rows of a tile of the kernel on pairs of CTAs
+PAIRS_ALLOWED = os.environ.get("ALOFA_GEMM_PAIR", "1") != "0"
+
+
+def _pair_splits(tokens: int, features: int, depth: int, gated: bool, deferrable: bool) -> int:
+    """Into how many parts the depth of a prompt portion's product goes on the
+    kernel that runs on pairs of CTAs; 0: it runs on another kernel.
+
+    Undivided: wide products with more tiles than SMs even of one CTA each,
+    and deep: 2,048 tokens, depth 3,584 x 37,888 weight rows 477 against 540 us
+    on single CTAs, depth 1,536 x 17,920 rows 85 against 92 us; at depth 896 the
+    pair's epilogue is not hidden behind its shorter MMA phase (9,728 rows: 33.9
+    against 32.7 us).  In up to four parts, added up by the consumer: deep, narrow
+    products, whose tiles of 256 x 256 leave most of the pairs idle or a last
+    round nearly empty, where that takes a quarter off the busiest pair's work
+    and seven of ten pairs have some.  Depth 8,960 x 1,536 rows, us on single
+    CTAs (with their own splits) and in parts on pairs: 532 tokens 34.1 and 20.4,
+    905 tokens 36.3 and 24.4, 2,048 tokens 68.1 and 46.5; depth 4,864 x 896 rows,
+    905 tokens 21.2 and 14.7, 2,048 tokens 23.4 and 21.0, but 532 tokens, 48
+    tiles on 74 pairs, 13.1 and 13.8; depth 18,944 x 3,584 rows, 1,400 tokens
+    216 and 172 - at 2,048 tokens a sixth less work for the busiest pair (242
+    and 218) goes into writing and reading the parts."""
+    if not PAIRS_ALLOWED or tokens <= 128 or features % 4:
+        return 0
+    undivided = 1 if depth >= 1024 and -(-features // (128 if gated else 256)) * -(-tokens // 128) > SMS else 0
+    slices, pairs = -(-depth // K_SLICE), SMS // 2
+    if gated or not deferrable or tokens <= 256 or slices < 32:
+        return undivided
+    tiles = -(-features // PAIR_ROWS) * -(-tokens // PAIR_ROWS)
+    rounds = lambda s: -(-tiles * s // pairs) * -(-slices // s)  # k-slices that the busiest pair works through  # noqa: E731
+    s = min((1, 2, 3, 4), key=lambda s: (rounds(s), s))
+    return s if 4 * rounds(s) <= 3 * rounds(1) and 10 * tiles * s >= 7 * pairs else undivided
+
+
 def plan(linear):
     from .linear import Partial
 
@@ -89,7 +125,10 @@ def plan(linear):
         lazy = None if isinstance(x, torch.Tensor) else x
         if lazy is not None:
             x = None
-        splits = ops.gemm_tc_splits(depth, _splits(_ctas(tokens, linear.out_features, bn, gated), depth, defer and n_acc == 1 and not linear.act))
+        deferrable = defer and n_acc == 1 and not linear.act
+        pair = _pair_splits(tokens, linear.out_features, depth, gated, deferrable) if bn < 0 else 0
+        bn = -PAIR_ROWS if pair else bn
+        splits = ops.gemm_tc_splits(depth, pair or _splits(_ctas(tokens, linear.out_features, bn, gated), depth, deferrable))
         computed = None
         if lazy is not None:
             # Rows still to be made.  The weights-on-M kernel makes them as it loads, a k-slice at a
@@ -111,7 +150,7 @@ def plan(linear):
             partial = buf(shape, torch.float32) if buf is not None else torch.empty(shape, dtype=torch.float32, device=w.device)
         deferred = defer and splits > 1 and n_acc == 1 and acc is None and not linear.act  # whoever adds deferred sums up applies no activation
         dst = partial[0] if deferred else out  # a deferred product writes partial sums only
-        if not ops.gemm_tc(dst, x, w, linear.bias, linear.epi, bn, splits, partial, reduce=not deferred, computed=computed, acc=acc, act=linear.act, gate=linear.gate):
+        if not ops.gemm_tc(dst, x, w, linear.bias, linear.epi, bn, splits, partial, reduce=not deferred, computed=computed, acc=acc, act=linear.act, gate=linear.gate, pair=pair > 0):
             if normed:
                 lazy.undo()
                 return run(out, lazy.rows(), defer, buf)

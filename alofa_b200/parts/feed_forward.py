@@ -40,7 +40,7 @@ class GatedMLP(Part):
         self.down = Linear(state[pre + "down_proj.weight"], None, RESIDUAL)
 
     def scratch_row_bytes(self) -> int:
-        return 4 * self.inter + 2 * 4 * self.hidden  # the activation, and the down product's depth split in two
+        return 4 * self.inter + 4 * 4 * self.hidden  # the activation, and the down product's depth in up to four parts
 
     takes_normed_rows = True  # ``x`` may be rows still to be made: the gate/up product folds the norm in
 
@@ -115,7 +115,7 @@ class DenseMLP(Part):
         self.down = Linear(state[pre + "down"], as_float32_vector(state[pre + "down.b"]) if self.bias else None, STORE)
 
     def scratch_row_bytes(self) -> int:
-        return 4 * self.inter + 4 * self.hidden
+        return 4 * self.inter + 4 * 4 * self.hidden
 
     def forward(self, ctx, x, h, store=False, defer=False):
         n = x.shape[0]

@@ -687,3 +687,35 @@ def test_32_bit_products_over_prompts(ops, k):
     assert_close(whole[0], sums[:, :n], TOL[F32], "store")
     assert_close(whole[1], plain.silu(sums[:, :n]) * sums[:, n:], TOL[F32], "gated")
     assert_close(whole[2], res + plain.linear(x, w[:n]), TOL[F32], "residual")
+
+
+@pytest.mark.parametrize("shape", [(129, 36, 64, 1), (257, 260, 2056, 3), (513, 1540, 2048, 4), (300, 1796, 8, 1), (905, 300, 640, 2), (2048, 520, 192, 2)])
+def test_products_on_pairs_of_ctas(ops, shape):
+    """Tokens and widths that leave most of a tile of 256 x 256 empty, a second CTA of a pair without a token, fewer tiles than
+    pairs and several a pair, and the depth in parts that the caller adds up (the last one shorter): against fp64."""
+    m, n, k, splits = shape
+    assert ops.gemm_tc_splits(k, splits) == splits
+    rng = np.random.default_rng(m + n)
+    x, w = rounded(rng.normal(size=(m, k)), BF16), rounded(rng.normal(size=(2 * n, k)) / np.sqrt(k), BF16)
+    bias, res = rng.normal(size=n).astype(np.float32), rng.normal(size=(m, n)).astype(np.float32)
+    sums = plain.linear(x, w)
+    part = torch.empty(splits, m, n, device="cuda")
+    if splits > 1:
+        for epi in (ops.EPI_RESIDUAL, ops.EPI_STORE):
+            part.fill_(float("nan"))
+            assert ops.gemm_tc(part[0], dev(x, BF16), dev(w[:n], BF16), None, epi, -256, splits, part, reduce=False, pair=True)
+            assert_close(part.sum(dim=0).cpu(), sums[:, :n], 2e-5, "parts")
+        out = torch.empty(m, n, device="cuda")
+        assert ops.gemm_tc(out, dev(x, BF16), dev(w[:n], BF16), dev(bias), ops.EPI_STORE, -256, splits, part, pair=True)
+        assert_close(out.cpu(), sums[:, :n] + bias, TOL[F32], "parts added up")
+        assert not ops.gemm_tc(out, dev(x, BF16), dev(w, BF16), None, ops.EPI_GATED, -256, splits, torch.empty(2 * splits, m, n, device="cuda"), pair=True)
+        return
+    for od in (BF16, F32):
+        out = torch.empty(m, n, dtype=od, device="cuda")
+        assert ops.gemm_tc(out, dev(x, BF16), dev(w[:n], BF16), dev(bias), ops.EPI_STORE, -256, pair=True)
+        assert_close(out.float().cpu(), sums[:, :n] + bias, TOL[od], "store")
+        assert ops.gemm_tc(out, dev(x, BF16), dev(w, BF16), None, ops.EPI_GATED, -256, pair=True)
+        assert_close(out.float().cpu(), plain.silu(sums[:, :n]) * sums[:, n:], TOL[od], "gated")
+    acc = dev(res)
+    assert ops.gemm_tc(acc, dev(x, BF16), dev(w[:n], BF16), None, ops.EPI_RESIDUAL, -256, pair=True)
+    assert_close(acc.cpu(), res + sums[:, :n], 2e-5, "residual")
