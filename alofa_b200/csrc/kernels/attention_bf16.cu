@@ -43,7 +43,7 @@ struct AttnParams {
   const int* block_table;  // [R, max_blocks]
   float* partial_o;      // split mode: [splits, T * nh, VD]
   float* partial_ml;     // split mode: [splits, T * nh, 2]
-  int max_blocks, page_size, nh, nkv, window, split_keys, n_splits, n_rows_total, table_entries;
+  int max_blocks, page_size, nh, nkv, window, split_keys, n_splits, n_rows_total, table_entries, n_seqs;
   float scale_log2;      // scale * log2(e)
 #ifdef SOFTCAP
   float cap_in, cap_out;  // scale / softcap and softcap / scale: scores are cap_out * tanh(dot * cap_in) before the scale
@@ -819,6 +819,7 @@ ALOFA_API int alofa_attention_bf16(void* out, const void* q, const void* k_cache
   p.split_keys = split_keys;
   p.n_splits = n_splits > 0 ? n_splits : 1;
   p.n_rows_total = n_tokens * nh;
+  p.n_seqs = n_seqs;
   p.scale_log2 = scale * 1.4426950408889634f;
 #ifdef SOFTCAP
   p.cap_in = scale / softcap;

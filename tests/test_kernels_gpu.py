@@ -719,3 +719,15 @@ def test_products_on_pairs_of_ctas(ops, shape):
     acc = dev(res)
     assert ops.gemm_tc(acc, dev(x, BF16), dev(w[:n], BF16), None, ops.EPI_RESIDUAL, -256, pair=True)
     assert_close(acc.cpu(), res + sums[:, :n], 2e-5, "residual")
+
+
+@pytest.mark.parametrize("hd, nh, nkv", [(64, 14, 2), (128, 6, 2)])
+def test_prompt_portions_scattered_over_many_requests(ops, hd, nh, nkv):
+    """The tiles of all requests numbered through: portions of several tiles, of a tile and a row, and single tokens, the
+    requests more than a warp and more than two have lanes, and steps whose rows make fewer tiles than the grid has."""
+    for count, portions in ((71, {0: 200, 31: 19, 32: 64, 64: 5, 70: 130}), (33, {32: 129}), (65, {1: 2, 3: 2})):
+        rng = np.random.default_rng(count)
+        q_lens = [portions.get(i, 1) for i in range(count)]
+        lens = [n + int(rng.integers(0, 90)) for n in q_lens]
+        got, want = attention_case(ops, BF16, hd, nh, nkv, lens=lens, q_lens=q_lens, page=64, window=None, rng=rng, fast=True)
+        assert_close(got, want, TOL[BF16], f"hd={hd} requests={count}")
