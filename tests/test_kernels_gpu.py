@@ -731,3 +731,28 @@ def test_prompt_portions_scattered_over_many_requests(ops, hd, nh, nkv):
         lens = [n + int(rng.integers(0, 90)) for n in q_lens]
         got, want = attention_case(ops, BF16, hd, nh, nkv, lens=lens, q_lens=q_lens, page=64, window=None, rng=rng, fast=True)
         assert_close(got, want, TOL[BF16], f"hd={hd} requests={count}")
+
+
+@pytest.mark.parametrize("hidden", [2052, 3584, 4096])
+@pytest.mark.parametrize("n", [1, 5, 300])
+def test_norms_of_long_rows(ops, hidden, n):
+    """A block per row with the row in registers: rows in place and picked ones, and the stream as base + accumulator, which is
+    written whole and leaves both accumulators zero."""
+    rng = np.random.default_rng(hidden + n)
+    h, w = rng.normal(size=(n, hidden)).astype(np.float32) * 3, (1 + 0.1 * rng.normal(size=hidden)).astype(np.float32)
+    picked = np.array([n - 1, 0], dtype=np.int32)
+    for od in (BF16, F32):
+        out, hd = torch.empty(n, hidden, dtype=od, device="cuda"), dev(h)
+        assert ops.norm_fused(out, hd, dev(w), 1e-5)
+        assert_close(out.float().cpu(), plain.rmsnorm(h, w, 1e-5), TOL[od], "rows in place")
+        assert np.array_equal(hd.cpu().numpy(), h)
+        two = torch.empty(2, hidden, dtype=od, device="cuda")
+        assert ops.norm_fused(two, hd, dev(w), 1e-5, dev(picked))
+        assert torch.equal(two[0], out[n - 1]) and torch.equal(two[1], out[0])
+        extra = rng.normal(size=(n, hidden))
+        acc, other = (torch.from_numpy(np.rint(extra * 2.0**32).astype(np.int64)).cuda() for _ in range(2))
+        hd = torch.full((n, hidden), float("nan"), device="cuda")
+        assert ops.norm_fused(out, hd, dev(w), 1e-5, base=dev(h), acc=acc, other=other)
+        assert_close(hd.cpu(), h + extra, 2e-6, "base + accumulator")
+        assert_close(out.float().cpu(), plain.rmsnorm((h + extra).astype(np.float32), w, 1e-5), TOL[od], "norm of base + accumulator")
+        assert not acc.any() and not other.any()
