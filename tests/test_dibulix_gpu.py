@@ -68,7 +68,7 @@ def in_portions(lengths, cuts, slots_of, run):
 # mechanisms alone
 # ---------------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("dtype", [F32, BF16])
-@pytest.mark.parametrize("S,width", [(1, 96), (2, 100), (3, 64), (4, 1030), (8, 33)])
+@pytest.mark.parametrize("S,width", [(1, 96), (2, 100), (3, 64), (4, 1030), (8, 33), (4, 2048), (5, 1036), (8, 4096), (2, 4100), (4, 4)])
 def test_streams_are_moved_read_normed_and_summed(dtype, S, width):
     """One pass does the owed write, the next read with its norm, or the sum; every stream from the OLD ones."""
     from alofa_b200.csrc import ops
