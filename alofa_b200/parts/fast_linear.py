@@ -13,6 +13,7 @@ order, so a given (tokens, weight) pair always sums the same way."""
 from __future__ import annotations
 
 import os
+from functools import lru_cache
 
 import torch
 
@@ -95,13 +96,18 @@ def _pair_splits(tokens: int, features: int, depth: int, gated: bool, deferrable
     if not PAIRS_ALLOWED or tokens <= 128 or features % 4:
         return 0
     undivided = 1 if depth >= 1024 and -(-features // (128 if gated else 256)) * -(-tokens // 128) > SMS else 0
-    slices, pairs = -(-depth // K_SLICE), SMS // 2
+    slices = -(-depth // K_SLICE)
     if gated or not deferrable or tokens <= 256 or slices < 32:
         return undivided
-    tiles = -(-features // PAIR_ROWS) * -(-tokens // PAIR_ROWS)
+    return _depth_parts(-(-features // PAIR_ROWS) * -(-tokens // PAIR_ROWS), slices, SMS // 2) or undivided
+
+
+@lru_cache(maxsize=1024)  # two microseconds to work out, twice a layer of a step that is issued launch by launch
+def _depth_parts(tiles: int, slices: int, pairs: int) -> int:
+    """The parts of the depth by :func:`_pair_splits`'s rule, 0 where none pay."""
     rounds = lambda s: -(-tiles * s // pairs) * -(-slices // s)  # k-slices that the busiest pair works through  # noqa: E731
     s = min((1, 2, 3, 4), key=lambda s: (rounds(s), s))
-    return s if 4 * rounds(s) <= 3 * rounds(1) and 10 * tiles * s >= 7 * pairs else undivided
+    return s if 4 * rounds(s) <= 3 * rounds(1) and 10 * tiles * s >= 7 * pairs else 0
 
 
 def plan(linear):

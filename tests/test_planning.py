@@ -75,6 +75,15 @@ def test_a_deep_product_that_underfills_the_gpu_is_halved_only_for_a_consumer_th
     assert fl._splits(ctas, 896, deferrable=True) == 1  # shallow: not worth a second pass
 
 
+def test_the_depth_parts_on_pairs_are_worked_out_once_a_shape():
+    """The down projection of a prompt, layer after layer: the parts that leave the busiest of 74 pairs the fewest k-slices."""
+    fl._depth_parts.cache_clear()
+    for tokens, features, depth, parts in ((2048, 896, 4864, 2), (905, 896, 4864, 4), (532, 1536, 8960, 4), (1400, 3584, 18944, 4), (532, 896, 4864, 0), (2048, 3584, 18944, 1)):
+        before = fl._depth_parts.cache_info().misses
+        assert {fl._pair_splits(tokens, features, depth, False, True) for _ in range(24)} == {parts}, (tokens, features, depth)
+        assert fl._depth_parts.cache_info().misses - before <= 1
+
+
 def test_decode_attention_splits_keep_a_step_resident_at_once():
     """Keys per CTA of a decode-only step (GQAttention.decode_split_keys), for
     a device of 148 SMs: head size 64 has the eight-warp kernel (148 CTAs at a
