@@ -79,14 +79,17 @@ constexpr bool TMA_SIZES = HD % 64 == 0 && VD % 64 == 0;  // head sizes the kern
 
 // The blocks of N keys that queries see whose last key is k_hi and whose window starts at k_lo (0: no window, or not left
 // yet), walked as numbers lo .. hi: first the `kept` blocks that hold a request's kept first keys, then those from the
-// window's first on.  Without kept keys a number is the block's own.
-template <int N>
+// window's first on.  Without kept keys a number is the block's own.  With EVEN the gap between the two is an even number of
+// blocks, so that a number is odd where the block's own is; the last block before the window may then be walked with all of its
+// keys unseen.
+template <int N, bool EVEN = false>
 struct SeenBlocks {
   int lo, hi, kept, gap;
   __device__ __forceinline__ SeenBlocks(int keep, int k_lo, int k_hi) {
     const int first = k_lo / N;
     kept = keep > 0 ? min((keep + N - 1) / N, first) : 0;
     gap = keep > 0 ? first - kept : 0;
+    if (EVEN) gap &= ~1;
     lo = keep > 0 ? 0 : first;
     hi = k_hi / N - gap;
   }

@@ -29,7 +29,9 @@
 // is only raised (and O and the running sum rescaled, in tensor memory) when a
 // row's scores outgrow it by more than 2^8, so most blocks leave O alone; the
 // result is O / sum either way.  A block's stream goes by its number in the
-// request, so a row's result does not depend on the tile it lies in.
+// request, so a row's result does not depend on the tile it lies in (with kept
+// first keys too: the blocks left out between them and the window are an even
+// number, if need be by walking one whose keys no row sees).
 // Every wait is bounded; a wait that runs out sets the status word to 2.
 // Formulas: src/alofa/kernels/cpu/scalar.mojo:392-470.
 #pragma once
@@ -124,7 +126,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_prefill_tc_kernel(con
   const int t_first = row0 / g, t_last = last_row / g;
   const int k_hi = pos0 + t_last;  // last visible key of the tile
   const int k_lo = p.window != 0 ? max(0, pos0 + t_first - window_at(p.window, pos0 + t_first) + 1) : 0;
-  const SeenBlocks<TC_BN> walk(p.keep, k_lo, k_hi);
+  const SeenBlocks<TC_BN, true> walk(p.keep, k_lo, k_hi);
   const int jb0 = walk.lo, nblk = walk.hi - walk.lo + 1;
 
   if (threadIdx.x == 0) {
@@ -159,7 +161,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_prefill_tc_kernel(con
     __syncwarp();
     if (lane == 0) {
       auto rows_of = [&](int i, int (&slot0)[2]) {  // the cache rows of the halves of block i
-        const int j_block = walk.block(jb0 + i) * TC_BN;
+        int j_block = walk.block(jb0 + i) * TC_BN;
+        if (p.keep > 0 && j_block >= p.keep && j_block + TC_BN <= k_lo) j_block += TC_BN;  // no key of it is seen, its pages may be gone: the window's first block in its place
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           int j = j_block + half * 64;

@@ -205,6 +205,23 @@ def test_biased_attention_on_the_tensor_core_kernels(H, G, d, dv, window, keep, 
                 assert_close(got[r], want[r], KERNEL_TOL[BF16], f"{what}: request of {n} tokens")
 
 
+@pytest.mark.parametrize("d,dv", [(64, 64), (128, 128), (64, 128), (128, 64)])
+@pytest.mark.parametrize("window,keep", [(512, 17), (200, 70), (130, 129), (300, 1), (70, 64)])
+def test_a_row_does_not_depend_on_the_portion_it_comes_in(d, dv, window, keep):
+    """The tcgen05 prompt kernel with kept first tokens: rows whose window starts an odd and an even number of key blocks behind
+    the kept ones, in tiles that start elsewhere with every cut, bit for bit the rows of the whole prompt."""
+    rng = np.random.default_rng(window)
+    m = case_mixer(4, 2, d, dv, window, keep)
+    w, width = picking_weights(rng, m)
+    rows = [rounded(rng.standard_normal((n, width)), F32) for n in (1500, 700)]
+    for cuts in ((331, 130), (57, 200, 101), (450, 449)):
+        case = PagedCase(rng, m, [len(x) for x in rows], 64, BF16)
+        whole, portions = in_steps(case, w, rows, BF16, 1e-5, cuts, True)
+        for r, x in enumerate(rows):
+            changed = np.flatnonzero((whole[r] != portions[r]).any(axis=1))
+            assert changed.size == 0, f"cuts {cuts}: {changed.size} of {len(x)} rows, the first at position {changed[0]}"
+
+
 PATHS = [(F32, 16, 16, False), (BF16, 16, 24, False), (BF16, 64, 64, True), (BF16, 32, 48, True)]
 
 
