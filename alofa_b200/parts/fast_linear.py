@@ -67,11 +67,14 @@ def _splits(ctas: int, depth: int, deferrable: bool = False) -> int:
     if ctas >= SMS // 2:
         # a deep product that does not fill the GPU once: two halves of the depth
         # side by side, when the consumer adds the halves up for free
-        return 2 if deferrable and ctas < SMS and slices >= 32 else 1
+        return 2 if deferrable and ctas < SMS and slices >= DEEP_SLICES else 1
     return max(1, min(slices, SMS // ctas))
 
 
 PAIR_ROWS = 256  # tokens and weight rows of a tile of the kernel on pairs of CTAs
+SLICE_PAYS_FOR = 135_000  # sums written and read again for a k-slice less of the busiest SM's work
+MOST_PARTS = 4   # of the depth that such a product may leave to its consumer
+DEEP_SLICES = 32  # k-slices from which a product's depth goes in halves, or on pairs in parts, for a consumer that adds them up
 PAIRS_ALLOWED = os.environ.get("ALOFA_GEMM_PAIR", "1") != "0"
 
 
@@ -92,22 +95,39 @@ def _pair_splits(tokens: int, features: int, depth: int, gated: bool, deferrable
     905 tokens 21.2 and 14.7, 2,048 tokens 23.4 and 21.0, but 532 tokens, 48
     tiles on 74 pairs, 13.1 and 13.8; depth 18,944 x 3,584 rows, 1,400 tokens
     216 and 172 - at 2,048 tokens a sixth less work for the busiest pair (242
-    and 218) goes into writing and reading the parts."""
+    and 218) goes into writing and reading the parts.  A part more than the kernel
+    that would run otherwise leaves has to save the busiest SM a k-slice for every
+    135,000 sums: with the norm after it, us otherwise and in parts, depth 3,584 x
+    3,584 rows 532 tokens 33.3 and 37.5, 1,400 tokens 65.6 and 92.5; depth 2,048 x
+    2,048 rows 257 tokens 20.7 and 22.5, 1,400 tokens 29.6 and 30.4; depth 18,944 x
+    3,584 rows 532 tokens 93.1 and 101.1, but 700 tokens 152 and 102; with the
+    rotate-and-store after it, depth 2,048 x 2,560 rows, 2,048 tokens 38.4 and 55.1."""
     if not PAIRS_ALLOWED or tokens <= 128 or features % 4:
         return 0
     undivided = 1 if depth >= 1024 and -(-features // (128 if gated else 256)) * -(-tokens // 128) > SMS else 0
     slices = -(-depth // K_SLICE)
-    if gated or not deferrable or tokens <= 256 or slices < 32:
+    if gated or not deferrable or tokens <= 256 or slices < DEEP_SLICES:
         return undivided
-    return _depth_parts(-(-features // PAIR_ROWS) * -(-tokens // PAIR_ROWS), slices, SMS // 2) or undivided
+    return _depth_parts(tokens, features, depth, undivided, SMS)
 
 
-@lru_cache(maxsize=1024)  # two microseconds to work out, twice a layer of a step that is issued launch by launch
-def _depth_parts(tiles: int, slices: int, pairs: int) -> int:
-    """The parts of the depth by :func:`_pair_splits`'s rule, 0 where none pay."""
+@lru_cache(maxsize=1024)  # microseconds to work out, twice a layer of a step that is issued launch by launch
+def _depth_parts(tokens: int, features: int, depth: int, undivided: int, sms: int) -> int:
+    """The parts of a deferrable product's depth by :func:`_pair_splits`'s rule;
+    ``undivided`` where none pay."""
+    slices, pairs = -(-depth // K_SLICE), sms // 2
+    tiles = -(-features // PAIR_ROWS) * -(-tokens // PAIR_ROWS)
     rounds = lambda s: -(-tiles * s // pairs) * -(-slices // s)  # k-slices that the busiest pair works through  # noqa: E731
-    s = min((1, 2, 3, 4), key=lambda s: (rounds(s), s))
-    return s if 4 * rounds(s) <= 3 * rounds(1) and 10 * tiles * s >= 7 * pairs else 0
+    s = min(range(1, MOST_PARTS + 1), key=lambda s: (rounds(s), s))
+    if 4 * rounds(s) > 3 * rounds(1) or 10 * tiles * s < 7 * pairs:
+        return undivided
+    # what it runs on otherwise: k-slices of the busiest pair, or of the busiest SM with up to two CTAs, and the planes left
+    work, planes = rounds(1), 1
+    if not undivided:
+        ctas = _ctas(tokens, features, _tile(tokens, features, False), False)
+        planes = _splits(ctas, depth, True)
+        work = -(-slices // planes) * -(-ctas * planes // (2 * sms)) * (1.3 if ctas * planes > sms else 1.0)  # a slice of two CTAs takes 1.3 of one's
+    return s if (work - rounds(s)) * SLICE_PAYS_FOR >= (s - planes) * tokens * features else undivided
 
 
 def plan(linear):

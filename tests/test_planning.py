@@ -84,6 +84,13 @@ def test_the_depth_parts_on_pairs_are_worked_out_once_a_shape():
         assert fl._depth_parts.cache_info().misses - before <= 1
 
 
+def test_parts_that_cost_more_to_write_and_read_than_they_save_are_not_made():
+    """Measured slower in parts than on the kernel they run on otherwise: single CTAs (0) or undivided on pairs (1)."""
+    for tokens, features, depth, parts in ((532, 3584, 3584, 0), (1400, 3584, 3584, 1), (257, 2048, 2048, 0), (1400, 2048, 2048, 0), (532, 3584, 18944, 0), (700, 3584, 18944, 3),
+                                           (1200, 2560, 2048, 0), (2048, 2560, 2048, 1), (700, 4608, 3584, 0), (1200, 4608, 3584, 1)):
+        assert fl._pair_splits(tokens, features, depth, False, True) == parts, (tokens, features, depth)
+
+
 def test_decode_attention_splits_keep_a_step_resident_at_once():
     """Keys per CTA of a decode-only step (GQAttention.decode_split_keys), for
     a device of 148 SMs: head size 64 has the eight-warp kernel (148 CTAs at a
