@@ -177,8 +177,9 @@ class GQAttention(PagedAttend, Part):
         return PagedKV(self.nkv, self.hd, self.window)
 
     def scratch_row_bytes(self) -> int:
-        # q/k/v, q, the attention output, and the output product's split sums
-        return 4 * (self.q_dim + 2 * self.kv_dim) + 2 * 4 * self.q_dim + 4 * 4 * self.hidden
+        # q/k/v, q, the attention output, and both products' sums where they are left to the consumer
+        rows = self.q_dim + 2 * self.kv_dim
+        return 4 * rows + 2 * 4 * self.q_dim + fast_linear.owed_row_bytes(rows, self.hidden) + fast_linear.owed_row_bytes(self.hidden, self.q_dim)
 
     def tensors(self):
         pre = self.prefix

@@ -111,6 +111,13 @@ def _pair_splits(tokens: int, features: int, depth: int, gated: bool, deferrable
     return _depth_parts(tokens, features, depth, undivided, SMS)
 
 
+def owed_row_bytes(features: int, depth: int) -> int:
+    """Scratch a token that a product called with ``defer`` may leave as fp32
+    planes for its consumer, in steps whose rows alone fill the GPU (fewer rows
+    in more parts are a few megabytes in all)."""
+    return 4 * features * (MOST_PARTS if -(-depth // K_SLICE) >= DEEP_SLICES else 2)
+
+
 @lru_cache(maxsize=1024)  # microseconds to work out, twice a layer of a step that is issued launch by launch
 def _depth_parts(tokens: int, features: int, depth: int, undivided: int, sms: int) -> int:
     """The parts of a deferrable product's depth by :func:`_pair_splits`'s rule;

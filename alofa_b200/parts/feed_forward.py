@@ -9,6 +9,7 @@ import torch
 
 from ..csrc import ops
 from ..errors import AlofaError
+from . import fast_linear
 from .base import Part, TensorSpec, as_float32_vector, register_part
 from .linear import GATED, RESIDUAL, STORE, Linear, add_into_stream
 
@@ -40,7 +41,7 @@ class GatedMLP(Part):
         self.down = Linear(state[pre + "down_proj.weight"], None, RESIDUAL)
 
     def scratch_row_bytes(self) -> int:
-        return 4 * self.inter + 4 * 4 * self.hidden  # the activation, and the down product's depth in up to four parts
+        return 4 * self.inter + fast_linear.owed_row_bytes(self.hidden, self.inter)  # the activation, and the down product's sums where they are left to the consumer
 
     takes_normed_rows = True  # ``x`` may be rows still to be made: the gate/up product folds the norm in
 
@@ -115,7 +116,7 @@ class DenseMLP(Part):
         self.down = Linear(state[pre + "down"], as_float32_vector(state[pre + "down.b"]) if self.bias else None, STORE)
 
     def scratch_row_bytes(self) -> int:
-        return 4 * self.inter + 4 * 4 * self.hidden
+        return 4 * self.inter + 4 * self.hidden + fast_linear.owed_row_bytes(self.hidden, self.inter)  # the activation, the output, and the down product's sums where they are left to the consumer
 
     def forward(self, ctx, x, h, store=False, defer=False):
         n = x.shape[0]

@@ -113,7 +113,8 @@ class LatentAttention(Part):
     def scratch_row_bytes(self) -> int:
         h = self.heads
         unfolded = 2 * (self.kv_rank + h * (self.dim + self.vdim)) if self.tells_fresh else 0
-        return unfolded + 4 * (self.q_rank + self.width + self.gate_cols) + 4 * self.q_rank + 4 * h * (self.dim + self.rot) + 4 * h * self.width + 4 * h * self.kv_rank + 4 * h * self.vdim + 4 * self.hidden
+        return unfolded + 4 * (self.q_rank + self.width + self.gate_cols) + 4 * self.q_rank + 4 * h * (self.dim + self.rot) + 4 * h * self.width + 4 * h * self.kv_rank + 4 * h * self.vdim + \
+            4 * self.hidden + fast_linear.owed_row_bytes(self.hidden, h * self.vdim)
 
     def tensors(self):
         pre, h = self.prefix, self.heads

@@ -52,6 +52,7 @@ import torch
 
 from ..csrc import ops
 from ..errors import AlofaError
+from . import fast_linear
 from .attention import PagedAttend
 from .base import PagedKV, Part, TensorSpec, as_float32_vector, build_part, register_part
 from .linear import RESIDUAL, STORE, Linear, add_into_stream
@@ -138,7 +139,8 @@ class NormedAttention(PagedAttend, Part):
         return PagedKV(self.kv_heads * self.maps, self.dim, self.chunk or self.window, self.vdim, None if value_heads == self.kv_heads * self.maps else value_heads, self.keep_first)
 
     def scratch_row_bytes(self) -> int:
-        return 4 * self.rows + 4 * self.q_dim + 4 * (self.maps + 1) * self.heads * self.vdim + 8 * self.hidden
+        owed = fast_linear.owed_row_bytes(self.rows, self.hidden) + fast_linear.owed_row_bytes(self.hidden, self.heads * self.vdim)  # both products' sums where they are left to the consumer
+        return 4 * self.rows + 4 * self.q_dim + 4 * (self.maps + 1) * self.heads * self.vdim + 4 * self.heads + owed
 
     def tensors(self):
         pre = self.prefix

@@ -55,6 +55,7 @@ import torch
 
 from ..csrc import ops
 from ..errors import AlofaError
+from . import fast_linear
 from .base import Part, SlotState, TensorSpec, as_float32_vector, register_part
 from .linear import RESIDUAL, STORE, Linear, add_into_stream
 
@@ -100,7 +101,7 @@ class StateSpaceMixer(Part):
         return SlotState((self.scan_words + self.conv_words,), torch.float32)
 
     def scratch_row_bytes(self) -> int:
-        return 4 * (self.in_rows + self.channels + 2 * self.inner + 2 * self.heads) + 8 * self.hidden
+        return 4 * (self.in_rows + self.channels + 2 * self.inner + 2 * self.heads) + fast_linear.owed_row_bytes(self.hidden, self.inner)
 
     def tensors(self):
         pre = self.prefix
@@ -167,7 +168,7 @@ class GatedLinearAttention(Part):
         return SlotState((self.heads * self.vdim * self.dim,), torch.float32)
 
     def scratch_row_bytes(self) -> int:
-        return 4 * (self.rows + 2 * self.qk + 2 * self.v) + 8 * self.hidden + 64
+        return 4 * (self.rows + 2 * self.qk + 2 * self.v) + fast_linear.owed_row_bytes(self.hidden, self.v) + 64
 
     def tensors(self):
         pre = self.prefix
@@ -222,7 +223,7 @@ class MinGRU(Part):
         return SlotState((self.width,), torch.float32)
 
     def scratch_row_bytes(self) -> int:
-        return 4 * 3 * self.width + 4 * self.width + 8 * self.hidden
+        return 4 * 3 * self.width + 4 * self.width + fast_linear.owed_row_bytes(self.hidden, self.width)
 
     def tensors(self):
         pre = self.prefix
@@ -280,7 +281,7 @@ class GatedDelta(Part):
         return SlotState((self.scan_words + self.conv_words,), torch.float32)
 
     def scratch_row_bytes(self) -> int:
-        return 4 * (self.in_rows + self.channels + 2 * (self.decays + self.v) + 2 * self.qk + 2 * self.heads + self.kv_heads + 2 * self.v + 12 * self.heads) + 8 * self.hidden + 512
+        return 4 * (self.in_rows + self.channels + 2 * (self.decays + self.v) + 2 * self.qk + 2 * self.heads + self.kv_heads + 2 * self.v + 12 * self.heads) + fast_linear.owed_row_bytes(self.hidden, self.v) + 512
 
     def tensors(self):
         pre = self.prefix
@@ -378,7 +379,7 @@ class GatedLRU(Part):
         return SlotState((self.width * self.taps,), torch.float32)
 
     def scratch_row_bytes(self) -> int:
-        return 4 * 6 * self.width + 8 * self.hidden
+        return 4 * 6 * self.width + fast_linear.owed_row_bytes(self.hidden, self.width)
 
     def tensors(self):
         pre, w, bs = self.prefix, self.width, self.block_size

@@ -181,3 +181,56 @@ def test_decode_steps_on_the_accumulator_stream_give_the_same_bits_every_run(sha
         runs.append(torch.stack(rows))
     assert torch.equal(runs[0], runs[1]), "two runs of the same steps differ"
     assert torch.equal(runs[0], runs[2]), "graph replay and plain launches differ"
+
+
+@pytest.mark.parametrize("design", ["qwen2", "kotutar", "darolix", "dibulix", "kikerax", "pekerax", "nugopel"])
+def test_parts_take_no_more_scratch_than_they_declare(design):
+    """Prompt steps of every design at its 2k benchmark sizes: what a layer's mixer and feed-forward take from the arena, the
+    parts of deep products that their consumers add up among it, against ``scratch_row_bytes``; and no region grows."""
+    import importlib
+
+    import bench
+    from alofa_b200.engine.loading import compute_dtype
+    from alofa_b200.engine.step import StepEntry, StepRunner
+    from alofa_b200.parts import expected_tensors
+    from alofa_b200.parts.base import Runtime
+    from alofa_b200.parts.model import Model
+    from alofa_b200.weights.loader import load_state
+
+    z = dict(bench.DESIGN_SIZES["2k"], experts=8, top=2, vocab=512)
+    if design in ("qwen2", "kotutar"):
+        cfg = bench.qwen2_config_like(z) if design == "qwen2" else bench.kotutar_config(z)
+    else:
+        sizes = dict(getattr(bench, design.upper() + "_SIZES")["2k"])
+        cfg = getattr(bench, design + "_config")(z, {**sizes, **{k: v for k, v in (("groups", 2), ("keep", 1)) if k in sizes}} if design in ("kikerax", "pekerax") else sizes)
+    spec = importlib.import_module(f"alofa_b200.models.{design}").build_spec(cfg)
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    state = {}
+    for name, t in expected_tensors(spec).items():
+        shape = tuple(abs(n) for n in t.shape)
+        x = torch.randn(shape, generator=gen, device="cuda") * 0.02
+        state[name] = (x + 1 if t.init == "ones" else x + torch.eye(shape[0], device="cuda") if t.init == "identity" else x).to(torch.bfloat16)
+    model = Model(spec, Runtime(torch.device("cuda"), compute_dtype("bfloat16")))
+    model.load(load_state(model.tensors(), state, model.rt.dtype, model.rt.device))
+    over = []
+
+    def watched(part, run, arena):
+        def forward(*args, **kwargs):
+            held = lambda: sum(b.numel() for b in arena.current.blocks[: arena.current.block]) + arena.current.offset  # noqa: E731
+            before, out = held(), run(*args, **kwargs)
+            rows = args[2].shape[0]
+            if held() - before > rows * part.scratch_row_bytes() + 64 * 256:  # each buffer starts on 256 bytes
+                over.append((type(part).__name__, rows, (held() - before) // rows, part.scratch_row_bytes()))
+            return out
+
+        return forward
+
+    for tokens in (700, 1024, 2048):
+        runner = StepRunner(model, block_size=64, num_pages=80, max_requests=4, max_tokens=2048, max_step_tokens=tokens, cuda_graphs=False)
+        parts = [p for block in model.layers for p in (block.mixer, block.feed_forward) if p is not None]
+        for part in parts:
+            part.forward = watched(part, type(part).forward.__get__(part), runner.arena)
+        runner.forward([StepEntry(runner.admit(1), np.random.default_rng(0).integers(0, 512, tokens).tolist(), [tokens - 1])])
+        runner.check_status()
+        assert runner.arena.grown == 0
+    assert not over, over
