@@ -227,8 +227,8 @@ __global__ void __launch_bounds__(256) gemm_generic_kernel(TO* __restrict__ out,
 // result is the same in every tile shape below, whatever rows share the launch.  A decode step is bound by the weights'
 // bytes: one row takes one column a warp, with up to 16 loads of 16 bytes a lane in flight and the first of them ahead of
 // the dependency wait, where the 64 x 64 tiles above kept 14 of 148 SMs busy (one row, output and down projection of 896
-// columns: 318 -> 3.7 us on average; gate and up 244 -> 6.5 us, 5.4 TB/s).  Many rows are bound by the reads of x and w
-// through L1: 8 x 4 sums a lane from 12 such reads (40 rows, gate and up: 57 us), 16 x 8 from 24 over the rows of a prompt.
+// columns: 318 -> 3.7 us on average; gate and up 244 -> 6.5 us, 5.4 TB/s).  A few more rows are bound by the reads of x and w
+// through L1: 8 x 4 sums a lane from 12 such reads (16 rows, gate and up: 22 us).
 template <int V>
 __device__ __forceinline__ float reduce_across_lanes(float (&v)[V], int lane) {  // value i ends in the lanes i * (32 / V) ..
   int o = 16;
@@ -247,13 +247,38 @@ __device__ __forceinline__ float reduce_across_lanes(float (&v)[V], int lane) { 
   return s;
 }
 
-template <int MT, int NT, int EPI, int WM = 1>  // WM: warps of a block side by side along the rows of x, the other 8 / WM along the columns
+template <int MT, int R, int EPI>
+__device__ __forceinline__ void finish_f32(const float (&acc)[MT * R], int lane, float* out, const float* __restrict__ bias, int m0, int n0, int M, int N, int act, float gate_alpha, float gate_limit) {
+  constexpr int NW = EPI == EPI_GATED ? 2 : 1, V = MT * R, G = V > 32 ? 32 : V;  // values reduced together: value i of a group ends in the lanes i * (32 / G) ..
+#pragma unroll
+  for (int g = 0; g < V; g += G) {
+    float part[G];
+#pragma unroll
+    for (int j = 0; j < G; ++j) part[j] = acc[g + j];
+    float v = reduce_across_lanes<G>(part, lane);
+    const int i = g + lane / (32 / G);  // the value this lane holds: row i / R, column (i % R) / NW, its gate or up sum
+    const int m = m0 + i / R, n = n0 + (i % R) / NW;
+    float u = 0.f;
+    if (EPI == EPI_GATED) u = __shfl_xor_sync(0xffffffffu, v, 32 / G);  // the up sum beside the gate's
+    if (m >= M || n >= N || lane % (32 / G) || (EPI == EPI_GATED && i % NW)) continue;
+    float* o = out + (size_t)m * N + n;
+    if (EPI == EPI_GATED) {
+      if (bias) v += bias[n], u += bias[N + n];
+      *o = gate_times(v, u, gate_alpha, gate_limit);
+    } else {
+      if (bias) v += bias[n];
+      *o = EPI == EPI_RESIDUAL ? *o + v : activate(v, act);
+    }
+  }
+}
+
+template <int MT, int NT, int EPI>
 __global__ void __launch_bounds__(256) gemm_f32_kernel(float* out, const float* x, const float* __restrict__ w, const float* __restrict__ bias, int M, int N, int K, int act,
                                                        float gate_alpha, float gate_limit) {
   constexpr int NW = EPI == EPI_GATED ? 2 : 1, R = NT * NW, V = MT * R;
   constexpr int U = V == 1 ? 16 : R >= 8 ? 1 : 8 / R;  // runs of 128 whose weights are asked for together
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = (blockIdx.x * (8 / WM) + warp / WM) * NT, m0 = (blockIdx.y * WM + warp % WM) * MT;
+  const int n0 = (blockIdx.x * 8 + warp) * NT, m0 = blockIdx.y * MT;
   const int k4 = K >> 2;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   const float4* wr[R];  // columns past the last read the last one's weights, and are not stored
@@ -291,25 +316,150 @@ __global__ void __launch_bounds__(256) gemm_f32_kernel(float* out, const float* 
     }
     load_weights(c + 32 * U);
   }
-  constexpr int G = V > 32 ? 32 : V;  // values reduced together: value i of a group ends in the lanes i * (32 / G) ..
+  finish_f32<MT, R, EPI>(acc, lane, out, bias, m0, n0, M, N, act, gate_alpha, gate_limit);
+}
+
+// The same over prompts: blocks of 32 rows and 32 rows of the weight, a warp 16 x 8 sums a lane.  Runs of 128 numbers of the
+// depth come into shared memory three deep: read straight from L2 through L1, the rows of x stood in the way of 512
+// multiply-adds a lane and run, and what two warps a scheduler could not hide made long prompts slower than the 64 x 64 tiles
+// above (2,048 rows, gate and up of the 0.5B shape: 1,392 us there, 1,627 straight from L2, now 1,212; output head, 40 rows 683,
+// 787 and 575).  Depths a little over a run or two leave lanes idle: from 4,096 rows on the tiles, whose order of summation is another
+// one, are still faster at depth 260 (x 257, gated: 72 us there, 82 here).
+constexpr int F32_ROWS = 32, F32_WEIGHT_ROWS = 32, F32_STAGES = 3;
+constexpr size_t F32_SMEM = (size_t)F32_STAGES * (F32_ROWS + F32_WEIGHT_ROWS) * 128 * sizeof(float);
+__device__ __forceinline__ void fetch16(float4* to, const float4* from, bool there) {  // zeros where nothing is there
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from), "r"(there ? 16 : 0) : "memory");
+}
+
+template <int EPI>
+__global__ void __launch_bounds__(256) gemm_f32_prompt_kernel(float* out, const float* x, const float* __restrict__ w, const float* __restrict__ bias, int M, int N, int K, int act,
+                                                              float gate_alpha, float gate_limit) {
+  constexpr int NW = EPI == EPI_GATED ? 2 : 1, MT = 16, R = 8, NT = R / NW;
+  extern __shared__ float4 stages[];  // [stage][rows of x, rows of the weight][lane]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row0 = blockIdx.y * F32_ROWS, column0 = blockIdx.x * (F32_WEIGHT_ROWS / NW);
+  const int k4 = K >> 2, runs = (k4 + 31) >> 5;
+  // this warp fetches every eighth row of both; rows and columns past the last read the last one's, and are not stored
+  const float4 *wr[4], *xr[4];
 #pragma unroll
-  for (int g = 0; g < V; g += G) {
-    float part[G];
+  for (int i = 0; i < 4; ++i) {
+    const int r = warp + 8 * i;
+    wr[i] = reinterpret_cast<const float4*>(w + ((size_t)(r % NW) * N + min(column0 + r / NW, N - 1)) * K);
+    xr[i] = reinterpret_cast<const float4*>(x + (size_t)min(row0 + r, M - 1) * K);
+  }
+  auto stage = [&](int run) { return stages + (size_t)(run % F32_STAGES) * (F32_ROWS + F32_WEIGHT_ROWS) * 32; };
+  auto fetch = [&](const float4* const (&rows)[4], int run, int to) {
+    const int c = run * 32 + lane;
 #pragma unroll
-    for (int j = 0; j < G; ++j) part[j] = acc[g + j];
-    float v = reduce_across_lanes<G>(part, lane);
-    const int i = g + lane / (32 / G);  // the value this lane holds: row i / R, column (i % R) / NW, its gate or up sum
-    const int m = m0 + i / R, n = n0 + (i % R) / NW;
-    float u = 0.f;
-    if (EPI == EPI_GATED) u = __shfl_xor_sync(0xffffffffu, v, 32 / G);  // the up sum beside the gate's
-    if (m >= M || n >= N || lane % (32 / G) || (EPI == EPI_GATED && i % NW)) continue;
-    float* o = out + (size_t)m * N + n;
-    if (EPI == EPI_GATED) {
-      if (bias) v += bias[n], u += bias[N + n];
-      *o = gate_times(v, u, gate_alpha, gate_limit);
-    } else {
-      if (bias) v += bias[n];
-      *o = EPI == EPI_RESIDUAL ? *o + v : activate(v, act);
+    for (int i = 0; i < 4; ++i) fetch16(stage(run) + (to + warp + 8 * i) * 32 + lane, rows[i] + (c < k4 ? c : 0), c < k4);
+  };
+#pragma unroll
+  for (int run = 0; run < F32_STAGES - 1; ++run)
+    if (run < runs) fetch(wr, run, F32_ROWS);
+  pdl_begin();
+#pragma unroll
+  for (int run = 0; run < F32_STAGES - 1; ++run) {
+    if (run < runs) fetch(xr, run, 0);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  float acc[MT * R];
+#pragma unroll
+  for (int v = 0; v < MT * R; ++v) acc[v] = 0.f;
+  const int mine = (warp % 2) * MT, theirs = F32_ROWS + (warp / 2) * R;  // this warp's rows of x and of the weight
+  for (int run = 0; run < runs; ++run) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(F32_STAGES - 2) : "memory");
+    __syncthreads();  // the run is here, and every warp is done with the one whose stage is fetched into next
+    if (run + F32_STAGES - 1 < runs) fetch(wr, run + F32_STAGES - 1, F32_ROWS), fetch(xr, run + F32_STAGES - 1, 0);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const float4* here = stage(run) + lane;
+    float4 wv[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) wv[r] = here[(theirs + r) * 32];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      const float4 xv = here[(mine + m) * 32];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        float& a = acc[m * R + r];
+        a = fmaf(xv.x, wv[r].x, a), a = fmaf(xv.y, wv[r].y, a), a = fmaf(xv.z, wv[r].z, a), a = fmaf(xv.w, wv[r].w, a);
+      }
+    }
+  }
+  finish_f32<MT, R, EPI>(acc, lane, out, bias, row0 + mine, column0 + (warp / 2) * NT, M, N, act, gate_alpha, gate_limit);
+}
+
+// The pairwise sum of COUNT lanes' products, STRIDE apart from lane l on: 4 rows of x 16 apart by 4 rows of the weight 16 apart.
+template <int COUNT, int STRIDE, int PITCH>
+struct LaneSums {
+  __device__ static __forceinline__ void of(float (&s)[16], const float4* xs, const float4* ws, int l) {
+    float t[16];
+    LaneSums<COUNT / 2, STRIDE * 2, PITCH>::of(s, xs, ws, l);
+    LaneSums<COUNT / 2, STRIDE * 2, PITCH>::of(t, xs, ws, l + STRIDE);
+#pragma unroll
+    for (int v = 0; v < 16; ++v) s[v] += t[v];
+  }
+};
+template <int STRIDE, int PITCH>
+struct LaneSums<1, STRIDE, PITCH> {
+  __device__ static __forceinline__ void of(float (&s)[16], const float4* xs, const float4* ws, int l) {
+    float4 a[4], b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = xs[16 * i * PITCH + l], b[i] = ws[16 * i * PITCH + l];
+#pragma unroll
+    for (int v = 0; v < 16; ++v) {
+      const float4 p = a[v >> 2], q = b[v & 3];
+      s[v] = fmaf(p.w, q.w, fmaf(p.z, q.z, fmaf(p.y, q.y, fmaf(p.x, q.x, 0.f))));
+    }
+  }
+};
+
+// The same for depths of up to 4 GROUPS over many rows: blocks of 64 rows and 64 rows of the weight, whole in shared memory, a thread
+// 4 x 4 sums of its own.  What lane l would sum is summed for one l after the other, in the order in which the pairwise sums close:
+// 0 and half of the lanes on, a quarter on and three quarters on, and so forth.  (With the depth over the lanes a depth of 16 leaves 28
+// of 32 idle and a block has little to do between its start and its end: 2,048 rows x 2,048 of depth 16 79 us, here 10.6, and 10.1 in
+// the 64 x 64 tiles further up.)
+template <int EPI, int GROUPS>
+__global__ void __launch_bounds__(256, 2) gemm_f32_short_kernel(float* out, const float* x, const float* __restrict__ w, const float* __restrict__ bias, int M, int N, int K, int act,
+                                                                float gate_alpha, float gate_limit) {
+  constexpr int NW = EPI == EPI_GATED ? 2 : 1, COLUMNS = 64 / NW, PITCH = GROUPS + 1;  // odd: eight neighbouring rows lie in different banks
+  extern __shared__ float4 stages[];  // 64 rows of x, 64 of the weight (gated: 32 columns' gate rows, then their up rows)
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int row0 = blockIdx.y * 64, column0 = blockIdx.x * COLUMNS, k4 = K >> 2;
+  const float4 *xs = stages + ty * PITCH, *ws = stages + (64 + tx) * PITCH;
+#pragma unroll
+  for (int i = threadIdx.x; i < 64 * GROUPS; i += 256) {  // rows and columns past the last read the last one's, and are not stored
+    const int r = i / GROUPS, c = i % GROUPS;
+    const float4* row = reinterpret_cast<const float4*>(w + ((size_t)(r / COLUMNS) * N + min(column0 + r % COLUMNS, N - 1)) * K);
+    fetch16(stages + (64 + r) * PITCH + c, row + min(c, k4 - 1), c < k4);
+  }
+  pdl_begin();
+#pragma unroll
+  for (int i = threadIdx.x; i < 64 * GROUPS; i += 256) {
+    const int r = i / GROUPS, c = i % GROUPS;
+    fetch16(stages + r * PITCH + c, reinterpret_cast<const float4*>(x + (size_t)min(row0 + r, M - 1) * K) + min(c, k4 - 1), c < k4);
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  float acc[16];
+  LaneSums<GROUPS, 1, PITCH>::of(acc, xs, ws, 0);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int m = row0 + ty + 16 * i;
+    if (m >= M) continue;
+#pragma unroll
+    for (int j = 0; j < 4 / NW; ++j) {
+      const int n = column0 + tx + 16 * j;
+      if (n >= N) continue;
+      float* o = out + (size_t)m * N + n;
+      float v = acc[4 * i + j];
+      if (EPI == EPI_GATED) {
+        float u = acc[4 * i + j + 2];
+        if (bias) v += bias[n], u += bias[N + n];
+        *o = gate_times(v, u, gate_alpha, gate_limit);
+      } else {
+        if (bias) v += bias[n];
+        *o = EPI == EPI_RESIDUAL ? *o + v : activate(v, act);
+      }
     }
   }
 }
@@ -317,22 +467,41 @@ __global__ void __launch_bounds__(256) gemm_f32_kernel(float* out, const float* 
 template <int EPI>
 static int gemm_f32_launch(float* out, const float* x, const float* w, const float* bias, int M, int N, int K, int act, float gate_alpha, float gate_limit, cudaStream_t stream) {
   constexpr int NW = EPI == EPI_GATED ? 2 : 1;
-  auto launch = [&](auto kernel, int mt, int nt, int wm) {
-    const long long rows = (M + mt * wm - 1) / (mt * wm);
+  auto launch = [&](auto kernel, int mt, int columns, size_t smem) {
+    const long long rows = (M + mt - 1) / mt;
     if (rows > 65535) return ALOFA_ERR_ARGUMENT;
-    const int columns = 8 / wm * nt;
-    launch_dep(kernel, dim3((N + columns - 1) / columns, (unsigned)rows), 256, 0, stream, out, x, w, bias, M, N, K, act, gate_alpha, gate_limit);
+    launch_dep(kernel, dim3((N + columns - 1) / columns, (unsigned)rows), 256, smem, stream, out, x, w, bias, M, N, K, act, gate_alpha, gate_limit);
     return launch_status();
   };
-  if (M == 1) return launch(gemm_f32_kernel<1, 1, EPI>, 1, 1, 1);
-  if (M == 2) return launch(gemm_f32_kernel<2, 2 / NW, EPI>, 2, 2 / NW, 1);
-  if (M <= 4) return launch(gemm_f32_kernel<4, 2 / NW, EPI>, 4, 2 / NW, 1);
-  // Prompts: 16 x 8 sums a lane, 32 x 32 outputs a block, once such blocks come near filling the SMs and their rows are mostly
-  // there (us at 8 x 4 / 16 x 8 sums: 40 x 9,728 of depth 896 45 / 50, 64 rows 69 / 50; 128 x 896 of depth 896 17.7 / 14.9;
-  // 64 x 896 of depth 4,864, 56 blocks, 39 / 48, 128 rows, 112 blocks, 74 / 48; 2,048 rows 1,139 / 649).
-  const long long blocks = (long long)((N + 32 / NW - 1) / (32 / NW)) * ((M + 31) / 32);
-  if (M >= 48 && blocks >= 112) return launch(gemm_f32_kernel<16, 8 / NW, EPI, 2>, 16, 8 / NW, 2);
-  return launch(gemm_f32_kernel<8, 4 / NW, EPI>, 8, 4 / NW, 1);
+  if (M == 1) return launch(gemm_f32_kernel<1, 1, EPI>, 1, 8, 0);
+  if (M == 2) return launch(gemm_f32_kernel<2, 2 / NW, EPI>, 2, 16 / NW, 0);
+  if (M <= 4) return launch(gemm_f32_kernel<4, 2 / NW, EPI>, 4, 16 / NW, 0);
+  static int sms = 0;
+  if (!sms) {
+    int device = 0, count = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+        cudaFuncSetAttribute(gemm_f32_prompt_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F32_SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(gemm_f32_short_kernel<EPI, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(128 * 33 * sizeof(float4))) != cudaSuccess)
+      return ALOFA_ERR_LAUNCH;
+    sms = count;
+  }
+  // Blocks of 32 rows once they come to half of the SMs and most of the rows are there (us with 8 x 4 sums a warp / in such blocks:
+  // depth 896 x 4,864 gated 16 rows 22.3 / 29.5, 24 rows 30.7 / 29.0; depth 4,864 x 896, 28 column blocks, 64 rows 38.5 / 40.6, 96
+  // rows 56.5 / 41.6; depth 896 x 1,152, 64 rows 10.3 / 9.6).
+  const int columns = F32_WEIGHT_ROWS / NW;
+  const long long blocks = (long long)((N + columns - 1) / columns) * ((M + F32_ROWS - 1) / F32_ROWS);
+  if (M > 16 && 2 * blocks >= sms) {
+    // Short depths: blocks of 64 rows, at depths of more than 32 once they too come to half of the SMs (us in blocks of 32 / of 64:
+    // depth 16 x 2,048 40 rows 6.0 / 3.5, 2,048 rows 79 / 10.6; depth 128 x 128 1,024 rows 4.3 / 7.7, 4,096 rows 12.6 / 9.0).
+    const long long blocks64 = (long long)((N + 64 / NW - 1) / (64 / NW)) * ((M + 63) / 64);
+    if (K > 128 || K == 0 || (K > 32 && 2 * blocks64 < sms)) return launch(gemm_f32_prompt_kernel<EPI>, F32_ROWS, columns, F32_SMEM);
+    auto launch_short = [&](auto kernel, int groups) { return launch(kernel, 64, 64 / NW, (size_t)128 * (groups + 1) * sizeof(float4)); };
+    if (K > 64) return launch_short(gemm_f32_short_kernel<EPI, 32>, 32);
+    if (K > 32) return launch_short(gemm_f32_short_kernel<EPI, 16>, 16);
+    if (K > 16) return launch_short(gemm_f32_short_kernel<EPI, 8>, 8);
+    return launch_short(gemm_f32_short_kernel<EPI, 4>, 4);
+  }
+  return launch(gemm_f32_kernel<8, 4 / NW, EPI>, 8, 32 / NW, 0);
 }
 
 template <typename TA, typename TW, typename TO>

@@ -665,12 +665,13 @@ def test_32_bit_products_sum_a_row_the_same_way_in_every_batch(ops, k):
         assert_close(rows[2], res + plain.linear(x, w[:n]), TOL[F32], f"residual n={n}")
 
 
-@pytest.mark.parametrize("k", [4, 132, 896])
-def test_32_bit_products_over_prompts(ops, k):
-    """The blocks of 32 x 32 outputs that many rows take, with rows and columns left over: as the plain implementation, and
+@pytest.mark.parametrize("m, k", [(53, 4), (53, 16), (17, 20), (130, 52), (17, 52), (65, 100), (130, 128), (53, 128), (53, 132), (53, 896), (17, 384), (65, 260)])
+def test_32_bit_products_over_prompts(ops, m, k):
+    """The blocks of 32 x 32 outputs that many rows take, and those of 64 x 64 at depths of up to 16, 32, 64 and 128, with rows and
+    columns left over, whole runs of 128 numbers and not, one of them, a ring's three and more: as the plain implementation, and
     bit for bit what a row is alone."""
     rng = np.random.default_rng(k)
-    m, n = 53, 1797
+    n = 2405
     x, w = rng.normal(size=(m, k)).astype(np.float32), (rng.normal(size=(2 * n, k)) / np.sqrt(k)).astype(np.float32)
     bias, res = rng.normal(size=2 * n).astype(np.float32), rng.normal(size=(m, n)).astype(np.float32)
     sums, got = plain.linear(x, w, bias), {}
