@@ -154,9 +154,10 @@ ALOFA_API int alofa_hyper_connect(float* streams, long long plane, const float* 
   const size_t smem = x_out ? (size_t)width * sizeof(float) : 0;
   if (smem > 200 * 1024) return ALOFA_ERR_ARGUMENT;
   HyperArgs a = {streams, plane, y, mix, out_w, in_w, norm_w, eps, x_out, sum_out, S, width};
-  // rows of whole groups of four that lie on 16 bytes (8 for bfloat16 rows), a group per thread
+  // rows of whole groups of four that lie on 16 bytes (8 for bfloat16 rows), a group per thread; not where half a warp would move
+  // more than four streams of a row (eight streams of 64, one token: 2.5 us in the other kernel, 3.1 in this one; of 100: 3.7 and 3.4)
   const uintptr_t places = (uintptr_t)streams | (uintptr_t)y | (uintptr_t)norm_w | (uintptr_t)sum_out | ((uintptr_t)x_out << (out_bf16 ? 1 : 0));
-  if (width % 4 == 0 && width <= 4096 && plane % 4 == 0 && places % 16 == 0) {
+  if (width % 4 == 0 && width <= 4096 && plane % 4 == 0 && places % 16 == 0 && (S <= 4 || width > 64)) {
     const int block = (width / 4 + 31) / 32 * 32;
     if (out_bf16) launch_dep(S <= 4 ? hyper_connect_vector_kernel<bf16, 4> : hyper_connect_vector_kernel<bf16, 8>, n_tokens, block, 0, stream, a);
     else launch_dep(S <= 4 ? hyper_connect_vector_kernel<float, 4> : hyper_connect_vector_kernel<float, 8>, n_tokens, block, 0, stream, a);
