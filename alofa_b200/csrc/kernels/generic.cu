@@ -810,8 +810,11 @@ ALOFA_API int alofa_paged_attention_generic(void* out, const void* q, const void
     using TO = std::remove_pointer_t<decltype(o)>;
     using T = std::remove_const_t<std::remove_pointer_t<decltype(queries)>>;
     // rows of whole groups of four numbers, which then lie on the 16 (bfloat16: 8) bytes a load takes
-    const bool vector = hd % 4 == 0 && vd % 4 == 0 && ((uintptr_t)k_cache | (uintptr_t)v_cache) % (4 * sizeof(T)) == 0;
-    const size_t smem = (size_t)(hd + 128 + (vector ? 128 / (vd / 4) * vd : 0)) * sizeof(float);
+    bool vector = hd % 4 == 0 && vd % 4 == 0 && ((uintptr_t)k_cache | (uintptr_t)v_cache) % (4 * sizeof(T)) == 0;
+    size_t smem = (size_t)(hd + 128) * sizeof(float);
+    const size_t sums = vector ? (size_t)(128 / (vd / 4)) * vd * sizeof(float) : 0;
+    vector = vector && smem + sums <= 47 * 1024;  // beside the static part, within what a launch has without asking for more
+    if (vector) smem += sums;
     launch_dep(vector ? paged_attention_vector_kernel<T, TO> : paged_attention_generic_kernel<T, TO>, grid, 128, smem, stream,
                o, queries, (const T*)k_cache, (const T*)v_cache, positions, seq_of_token, block_table,
                max_blocks, page_size, nh, nkv, hd, vd, window, scale, softcap, sink, chunk, v_share, keep, slopes);

@@ -734,6 +734,21 @@ def test_prompt_portions_scattered_over_many_requests(ops, hd, nh, nkv):
         assert_close(got, want, TOL[BF16], f"hd={hd} requests={count}")
 
 
+@pytest.mark.parametrize("hd", [11392, 11396, 11900])
+def test_attention_of_heads_that_fill_shared_memory(ops, hd):
+    """The longest head the kernel with whole groups of four has room for, and longer ones that only the other takes."""
+    rng = np.random.default_rng(hd)
+    n, vd = 9, 8
+    q, k, v = rng.normal(size=(n, hd)).astype(np.float32), rng.normal(size=(16, 1, hd)).astype(np.float32), rng.normal(size=(16, 1, vd)).astype(np.float32)
+    out = torch.empty(n, vd, device="cuda")
+    zero = np.zeros(n, dtype=np.int32)
+    ops.paged_attention_generic(out, dev(q), dev(k), dev(v), dev(np.arange(n, dtype=np.int32)), dev(zero), dev(zero[:1].reshape(1, 1)), 16, 1, 1, hd, None, hd**-0.5, vd=vd)
+    scores = q.astype(np.float64) @ k[:n, 0].astype(np.float64).T * hd**-0.5
+    scores[np.triu_indices(n, 1)] = -np.inf
+    w = np.exp(scores - scores.max(axis=1, keepdims=True))
+    assert_close(out.cpu(), w / w.sum(axis=1, keepdims=True) @ v[:n, 0].astype(np.float64), TOL[F32], f"heads of {hd}")
+
+
 @pytest.mark.parametrize("hidden", [2052, 3584, 4096])
 @pytest.mark.parametrize("n", [1, 5, 300])
 def test_norms_of_long_rows(ops, hidden, n):
