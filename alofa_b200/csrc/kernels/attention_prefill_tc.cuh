@@ -23,8 +23,8 @@
 // different streams: while one waits, reads tensor memory or looks for its
 // maximum, the other exponentiates.  (With both groups of warps on the same
 // block, half a row a thread, they met once a block to exchange maxima and did
-// everything at the same time.  2,048 tokens from the start, 12 heads of 128 on 2, and 2,048 behind 2,048 others: 62 -> 47 us on
-// average; 905 behind 4,096: 114 -> 68; 1,999, 28 heads on 4: 104 -> 79; 2,048, 14 heads of 64 on 2: 27.5 -> 26.)
+// everything at the same time.  Repeated in a graph, operands warm: 2,048 tokens, 12 heads of 128 on 2: 36.9 -> 29.0 us, behind
+// 2,048 others 85.4 -> 65.2; 905 behind 4,096: 115 -> 68; 1,999, 28 heads on 4: 83.7 -> 62.2; 2,048, 14 heads of 64 on 2: 28.7 -> 27.0.)
 // The running maximum is kept lazily: P is scaled by 2^-m for a maximum m that
 // is only raised (and O and the running sum rescaled, in tensor memory) when a
 // row's scores outgrow it by more than 2^8, so most blocks leave O alone; the
