@@ -672,10 +672,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
 // The epilogue of a 128-token tile whose width is a multiple of 4: warp q owns
 // rows [32q, 32q + 32) of the accumulator at `tmem_acc`; `staging` holds
-// 4 x 32 rows of COLS floats.  Two warps share a quarter: `half` (0 or 1) takes half of every COLS
-// columns and rows [16 half, 16 half + 16) of the stores; they meet on the named barrier 8 + q.
-// COLS is 128, half as many meetings, where shared memory has the room (one CTA per tile: 65 tokens,
-// depth 8,192 x 100 rows 25.0 us with 64 and 24.4 with 128), and 64 where a deeper ring is worth more.  `release` (optional, one arrival per warp) is signalled once the
+// 4 x 32 rows of 64 floats.  Two warps share a quarter: `half` (0 or 1) takes columns
+// [32 half, 32 half + 32) of every 64 and rows [16 half, 16 half + 16) of the stores; they meet
+// on the named barrier 8 + q.  `release` (optional, one arrival per warp) is signalled once the
 // accumulator has been read out.
 __device__ __forceinline__ void quarter_sync(int q) { asm volatile("bar.sync %0, 64;" ::"r"(8 + q) : "memory"); }
 // All eight epilogue warps: true when every thread brought true (one verdict for all, so that they
@@ -693,35 +692,34 @@ __device__ __forceinline__ bool epilogue_warps_agree(bool ok) {
   return any_bad == 0;
 }
 
-template <int EPI, int COLS>
+template <int EPI>
 __device__ __forceinline__ void tokens_epilogue_staged(const GemmArgs& args, const int FEATS, uint32_t tmem_base, float* staging, int q, int half, int lane, int f0,
                                                        int t0, int n_splits, int split_index, uint64_t* release, uint32_t release_in_cluster = 0) {
   constexpr bool GATED = EPI == EPI_GATED;  // FEATS: output features of the tile, a multiple of 16
-  // The accumulator rows go through shared memory so that global memory is written whole rows of COLS features at a time:
+  // The accumulator rows go through shared memory so that global memory is written whole rows of 64 features at a time:
   // each thread drops its row's values into a tile whose groups of four are permuted by the row (no bank is hit twice, and
-  // no padding takes room from the ring), then the warps walk the rows with one 16-byte access per lane.
-  float* stage = staging + (size_t)q * 32 * COLS;
-  auto group = [&](int row, int c) { return reinterpret_cast<float4*>(stage + row * COLS + ((c ^ (row & 15)) << 2)); };
+  // no padding takes room from the ring), then the warps walk the rows with one 16-byte access per lane, two rows at once.
+  float* stage = staging + (size_t)q * 32 * 64;
+  auto group = [&](int row, int c) { return reinterpret_cast<float4*>(stage + row * 64 + ((c ^ (row & 15)) << 2)); };
   const bool split = n_splits > 1;
   const int N = args.N;
   const size_t plane = (size_t)args.T * N;
-  constexpr int AT_ONCE = 128 / COLS, EACH = 16 / AT_ONCE;  // rows a warp stores at once, rows a lane stores
-  const int sub = lane / (COLS / 4), c4 = lane % (COLS / 4);
-  const int r_lo = half * 16 + sub, rows = args.T - (t0 + q * 32);  // this lane stores rows r_lo, r_lo + AT_ONCE, .. below `rows`
+  const int sub = lane >> 4, c4 = lane & 15;
+  const int r_lo = half * 16 + sub, rows = args.T - (t0 + q * 32);  // this lane stores rows r_lo, r_lo + 2, .. r_lo + 14 below `rows`
 #pragma unroll 1
-  for (int cb = 0; cb < FEATS; cb += COLS) {
+  for (int cb = 0; cb < FEATS; cb += 64) {
     if (f0 + cb >= N) break;
     const int f = f0 + cb + c4 * 4;  // this lane's four features of the rows it stores
     const bool f_ok = f < N && cb + c4 * 4 < FEATS;  // N % 4 == 0: a group is inside or outside as a whole
     const size_t at = (size_t)(t0 + q * 32) * N + f;
-    float4 b[EPI == EPI_RESIDUAL ? EACH : 1];
-    if (EPI == EPI_RESIDUAL && !split && f_ok) {  // the rows to add to: the first eight loads run beside the staging, as many as registers hold there
+    float4 b[EPI == EPI_RESIDUAL ? 8 : 1];
+    if (EPI == EPI_RESIDUAL && !split && f_ok) {  // the rows to add to: their loads run beside the staging
 #pragma unroll
       for (int i = 0; i < 8; ++i)
-        if (r_lo + AT_ONCE * i < rows) b[i] = *reinterpret_cast<const float4*>((float*)args.out + at + (size_t)(r_lo + AT_ONCE * i) * N);
+        if (r_lo + 2 * i < rows) b[i] = *reinterpret_cast<const float4*>((float*)args.out + at + (size_t)(r_lo + 2 * i) * N);
     }
 #pragma unroll 1
-    for (int c0 = half * (COLS / 2); c0 < (half + 1) * (COLS / 2) && cb + c0 < FEATS; c0 += 16) {
+    for (int c0 = half * 32; c0 < half * 32 + 32 && cb + c0 < FEATS; c0 += 16) {
       const int g = f0 + cb + c0;
       if (g >= N) break;
       uint32_t r0[16], r1[16];
@@ -754,25 +752,20 @@ __device__ __forceinline__ void tokens_epilogue_staged(const GemmArgs& args, con
 #pragma unroll
       for (int j = 0; j < 16; j += 4) *group(lane, (c0 + j) >> 2) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
     }
-    const bool read_out = (release || release_in_cluster) && (cb + COLS >= FEATS || f0 + cb + COLS >= N);
+    const bool read_out = (release || release_in_cluster) && (cb + 64 >= FEATS || f0 + cb + 64 >= N);
     if (read_out) tc_fence_before();  // the accumulator is read out: the next tile but one may have it
     __syncwarp();
     if (read_out && lane == 0) {  // one arrival per warp: arrivals at a barrier of the other CTA are dear
       if (release_in_cluster) mbar_arrive_in_cluster(release_in_cluster);
       else mbar_arrive(release);
     }
-    if (EACH > 8 && EPI == EPI_RESIDUAL && !split && f_ok) {
-#pragma unroll
-      for (int i = 8; i < EACH; ++i)
-        if (r_lo + AT_ONCE * i < rows) b[i] = *reinterpret_cast<const float4*>((float*)args.out + at + (size_t)(r_lo + AT_ONCE * i) * N);
-    }
     quarter_sync(q);  // both halves of the columns are staged
     if (f_ok) {
       if (split || EPI == EPI_RESIDUAL || !args.out_bf16) {
         float* o = (split ? args.partial + (size_t)split_index * plane : (float*)args.out) + at;
 #pragma unroll
-        for (int i = 0; i < EACH; ++i) {
-          const int r = r_lo + AT_ONCE * i;
+        for (int i = 0; i < 8; ++i) {
+          const int r = r_lo + 2 * i;
           if (r >= rows) break;
           float4 a = *group(r, c4);
           if (EPI == EPI_RESIDUAL && !split) a = make_float4(b[i].x + a.x, b[i].y + a.y, b[i].z + a.z, b[i].w + a.w);
@@ -780,9 +773,9 @@ __device__ __forceinline__ void tokens_epilogue_staged(const GemmArgs& args, con
         }
       } else {
         bf16* o = (bf16*)args.out + at;
-#pragma unroll 8
-        for (int i = 0; i < EACH; ++i) {
-          const int r = r_lo + AT_ONCE * i;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int r = r_lo + 2 * i;
           if (r >= rows) break;
           const float4 a = *group(r, c4);
           __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);
@@ -790,7 +783,7 @@ __device__ __forceinline__ void tokens_epilogue_staged(const GemmArgs& args, con
         }
       }
     }
-    quarter_sync(q);  // the staged rows are stored: the next COLS columns, or the next tile, may overwrite them
+    quarter_sync(q);  // the staged rows are stored: the next 64 columns, or the next tile, may overwrite them
   }
 }
 
@@ -915,7 +908,7 @@ gemm_tc_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     if (no_tile) {
       // nothing to store
     } else if (ok && staged && t0 + q * 32 < args.T) {
-      tokens_epilogue_staged<EPI, 128>(args, FEATS, tmem_base, reinterpret_cast<float*>(tiles), q, half, lane, f0, t0, (int)gridDim.z, (int)blockIdx.z, nullptr);
+      tokens_epilogue_staged<EPI>(args, FEATS, tmem_base, reinterpret_cast<float*>(tiles), q, half, lane, f0, t0, (int)gridDim.z, (int)blockIdx.z, nullptr);
     } else if (ok && t0 + q * 32 < args.T) {
       // widths that are no multiple of 4 (or gated partial sums): element-wise, straight from the registers
       const bool split = gridDim.z > 1;
@@ -1169,7 +1162,7 @@ gemm_tc_tokens_persistent_kernel(const __grid_constant__ CUtensorMap map_w, cons
       if (!epilogue_warps_agree(ok)) break;
       tc_fence_after();
       if (t0 + q * 32 < args.T) {
-        tokens_epilogue_staged<EPI, 64>(args, FEATS, tmem_base + buf * BNF, staging, q, half, lane, f0, t0, 1, 0, &acc_free[buf]);
+        tokens_epilogue_staged<EPI>(args, FEATS, tmem_base + buf * BNF, staging, q, half, lane, f0, t0, 1, 0, &acc_free[buf]);
       } else {
         tc_fence_before();
         __syncwarp();
@@ -1194,19 +1187,17 @@ gemm_tc_tokens_persistent_kernel(const __grid_constant__ CUtensorMap map_w, cons
 // half of the weight rows (for EPI_GATED the first CTA the gate rows, the
 // second the matching up rows), 32 KB per k-slice where the single CTA fetches
 // 48 KB for the same MMA time: the product is no longer bound by what an SM can
-// pull out of L2, and the ring is six stages deep (four beside a staging tile of 128 columns instead
-// of 64: launch_pair).  The first CTA's full
+// pull out of L2, and the ring is six stages deep.  The first CTA's full
 // barrier counts the bytes of both CTAs' copies; the MMAs' completion is
 // signalled on the barriers of both; both CTAs' epilogue warps free an
 // accumulator on the first CTA's barrier.
 // ---------------------------------------------------------------------------
-template <int COLS>
-constexpr int PAIR_RING = COLS == 128 ? 4 : 6;
+constexpr int PAIR_STAGES = 6;
 
-template <int EPI, int COLS>
+template <int EPI>
 __global__ void __launch_bounds__(TOKENS_THREADS, 1)
 gemm_tc_tokens_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const GemmArgs args) {
-  constexpr int BNF = 256, PAIR_STAGES = PAIR_RING<COLS>;
+  constexpr int BNF = 256;
   constexpr bool GATED = EPI == EPI_GATED;
   constexpr int FEATS = GATED ? BNF / 2 : BNF;
   constexpr uint32_t A_BYTES = 128 * BK * 2;
@@ -1227,11 +1218,11 @@ gemm_tc_tokens_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const int n_ftiles = (args.N + FEATS - 1) / FEATS, n_ttiles = (args.T + 255) / 256;
   const int total_slices = (args.K + BK - 1) / BK, per_split = args.k_slices_per_split;
-  const int n_splits = GATED ? 1 : (total_slices + per_split - 1) / per_split;  // a gated product goes undivided
+  const int n_splits = (total_slices + per_split - 1) / per_split;
   const int n_tiles = n_ftiles * n_ttiles * n_splits;  // feature tiles innermost, parts of the depth outermost
-  auto split_of = [&](int tile) { return GATED ? 0 : tile / (n_ftiles * n_ttiles); };
-  auto token_of = [&](int tile) { return (GATED ? tile / n_ftiles : tile / n_ftiles % n_ttiles) * 256 + (int)rank * 128; };
-  auto slices_of = [&](int tile) { return GATED ? total_slices : min(per_split, total_slices - split_of(tile) * per_split); };
+  auto split_of = [&](int tile) { return tile / (n_ftiles * n_ttiles); };
+  auto token_of = [&](int tile) { return tile / n_ftiles % n_ttiles * 256 + (int)rank * 128; };
+  auto slices_of = [&](int tile) { return min(per_split, total_slices - split_of(tile) * per_split); };
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
@@ -1322,7 +1313,7 @@ gemm_tc_tokens_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
       tc_fence_after();
       const uint32_t free_bar = in_cluster_cta(&acc_free[buf], 0);
       if (t0 + q * 32 < args.T) {
-        tokens_epilogue_staged<EPI, COLS>(args, FEATS, tmem_base + buf * BNF, staging, q, half, lane, f0, t0, n_splits, split, nullptr, free_bar);
+        tokens_epilogue_staged<EPI>(args, FEATS, tmem_base + buf * BNF, staging, q, half, lane, f0, t0, n_splits, split, nullptr, free_bar);
       } else {
         tc_fence_before();
         __syncwarp();
@@ -1566,33 +1557,22 @@ static int launch_tokens(const CUtensorMap& mw, const CUtensorMap& mx, const Gem
 }
 
 // The kernel on pairs of CTAs: as many pairs as there are tiles, and no more than the SMs hold.
-template <int EPI, int COLS>
-static int launch_pair_as(const CUtensorMap& mw, const CUtensorMap& mx, const GemmArgs& args, int splits, cudaStream_t stream) {
+template <int EPI>
+static int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const GemmArgs& args, int splits, cudaStream_t stream) {
   static int sms = 0;
-  constexpr size_t SMEM = (size_t)PAIR_RING<COLS> * 2 * 128 * BK * 2 + (size_t)4 * 32 * COLS * 4 + 1024;
+  constexpr size_t SMEM = (size_t)PAIR_STAGES * 2 * 128 * BK * 2 + STAGING_BYTES + 1024;
   if (!sms) {
     int device = 0, count = 0;
     if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || count < 2) return ALOFA_ERR_LAUNCH;
-    if (cudaFuncSetAttribute(gemm_tc_tokens_pair_kernel<EPI, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) != cudaSuccess) return ALOFA_ERR_LAUNCH;
-    prefer_max_shared(gemm_tc_tokens_pair_kernel<EPI, COLS>);
+    if (cudaFuncSetAttribute(gemm_tc_tokens_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) != cudaSuccess) return ALOFA_ERR_LAUNCH;
+    prefer_max_shared(gemm_tc_tokens_pair_kernel<EPI>);
     sms = count;
   }
   const int feats = EPI == EPI_GATED ? 128 : 256;
   const long long tiles = (long long)((args.N + feats - 1) / feats) * ((args.T + 255) / 256) * splits;
   const int pairs = (int)(tiles < sms / 2 ? tiles : sms / 2);
-  launch_dep_cluster(gemm_tc_tokens_pair_kernel<EPI, COLS>, dim3(2 * pairs), TOKENS_THREADS, SMEM, stream, 2, mw, mx, args);
+  launch_dep_cluster(gemm_tc_tokens_pair_kernel<EPI>, dim3(2 * pairs), TOKENS_THREADS, SMEM, stream, 2, mw, mx, args);
   return launch_status();
-}
-
-// A gated product of a small depth waits for its epilogue, the others for their loads.  Depth 1,536 x 17,920 rows, us with a ring of
-// six beside 64 staged columns and of four beside 128: 512 tokens 27.4 and 26.6, 2,048 tokens 83.9 and 83.2; at depth 3,584 x
-// 37,888 rows a ring of four alone costs 113.6 -> 118.0 over 512 tokens.
-template <int EPI>
-static int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const GemmArgs& args, int splits, cudaStream_t stream) {
-  if constexpr (EPI == EPI_GATED) {
-    if (args.K <= 2048) return launch_pair_as<EPI, 128>(mw, mx, args, splits, stream);
-  }
-  return launch_pair_as<EPI, 64>(mw, mx, args, splits, stream);
 }
 
 template <int EPI>
