@@ -1218,11 +1218,11 @@ gemm_tc_tokens_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const int n_ftiles = (args.N + FEATS - 1) / FEATS, n_ttiles = (args.T + 255) / 256;
   const int total_slices = (args.K + BK - 1) / BK, per_split = args.k_slices_per_split;
-  const int n_splits = (total_slices + per_split - 1) / per_split;
+  const int n_splits = GATED ? 1 : (total_slices + per_split - 1) / per_split;  // a gated product goes undivided
   const int n_tiles = n_ftiles * n_ttiles * n_splits;  // feature tiles innermost, parts of the depth outermost
-  auto split_of = [&](int tile) { return tile / (n_ftiles * n_ttiles); };
-  auto token_of = [&](int tile) { return tile / n_ftiles % n_ttiles * 256 + (int)rank * 128; };
-  auto slices_of = [&](int tile) { return min(per_split, total_slices - split_of(tile) * per_split); };
+  auto split_of = [&](int tile) { return GATED ? 0 : tile / (n_ftiles * n_ttiles); };
+  auto token_of = [&](int tile) { return (GATED ? tile / n_ftiles : tile / n_ftiles % n_ttiles) * 256 + (int)rank * 128; };
+  auto slices_of = [&](int tile) { return GATED ? total_slices : min(per_split, total_slices - split_of(tile) * per_split); };
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
