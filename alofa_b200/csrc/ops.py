@@ -87,6 +87,24 @@ def _gemm_tc():
     return lib
 
 
+def _decode_stack():
+    lib = _libs.get("decode_stack")
+    if lib is None:
+        lib = load_library("alofa_decode_stack", ["kernels/decode_stack.cu"])
+        sigs = {
+            "alofa_decode_stack_layer_bytes": [],
+            "alofa_decode_stack_ctas": [_I, _I, _I, _I, _I, _I, _I],
+            "alofa_decode_stack_layer": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _F, _F, _I, _I, _I, _I, _I],
+            "alofa_decode_stack": [_P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P],
+        }
+        for name, args in sigs.items():
+            fn = getattr(lib, name)
+            fn.restype = _I
+            fn.argtypes = args
+        _libs["decode_stack"] = lib
+    return lib
+
+
 def _attention(head_dim: int, capped: bool = False, v_dim=None, distance: bool = False):
     """The attention library of one size of key heads and (``v_dim``, when it differs) value heads; ``capped``: the build
     whose scores are bounded by softcap * tanh(. / softcap); ``distance``: the one that takes a distance bias off them."""
@@ -1514,3 +1532,58 @@ def lru_scan(out, a, b, y, y_off: int, act: str, state, q_start, state_slots, n_
     _done(_gated_lru().alofa_lru_scan(_dev(out, "out"), _dev(a, "a", f32), _dev(b, "b", f32), _dev(y, "y", f32), y.shape[1], y_off, ACTIVATIONS[act], state.data_ptr(),
                                       state.stride(0), _dev(q_start, "q_start", i32), _dev(state_slots, "state_slots", i32), n_seqs, n, width, _is_bf16(out, "out"),
                                       _stream()), "lru_scan")
+
+
+def decode_stack_ctas(tokens: int, hidden: int, heads: int, kv_heads: int, head_dim: int, inter: int, page: int) -> int:
+    """How many CTAs run all layers of a decode step of so many tokens at these
+    sizes (:func:`decode_stack`); 0 where that kernel does not take them."""
+    return _decode_stack().alofa_decode_stack_ctas(tokens, hidden, heads, kv_heads, head_dim, inter, page)
+
+
+def decode_stack_act_numbers(tokens: int, inter: int, ctas: int) -> int:
+    """How many numbers the activation takes in :func:`decode_stack`: every CTA
+    has whole 128-byte lines of its own."""
+    tiles = -(-(inter // 8) // ctas)
+    return ctas * (-(-tiles * tokens * 8 // 64) * 64)
+
+
+def decode_stack_layer(qkv, out, gate_up, down, gamma_mixer, gamma_ff, qkv_bias, k_cache, v_cache, eps_mixer: float, eps_ff: float, hidden: int, heads: int, kv_heads: int, head_dim: int, inter: int) -> bytes:
+    """One layer's entry of the table that :func:`decode_stack` reads: where
+    its weights and caches lie."""
+    q_dim, rows = heads * head_dim, (heads + 2 * kv_heads) * head_dim
+    bf16 = torch.bfloat16
+    if tuple(qkv.shape) != (rows, hidden) or tuple(out.shape) != (hidden, q_dim) or tuple(gate_up.shape) != (2 * inter, hidden) or tuple(down.shape) != (hidden, inter):
+        raise AlofaError("invalid_argument", "decode_stack sizes disagree", f"qkv={tuple(qkv.shape)} out={tuple(out.shape)} gate_up={tuple(gate_up.shape)} down={tuple(down.shape)}")
+    if gamma_mixer.shape[0] != hidden or gamma_ff.shape[0] != hidden or (qkv_bias is not None and qkv_bias.shape[0] != rows) or tuple(k_cache.shape[1:]) != (kv_heads, head_dim) or k_cache.shape != v_cache.shape:
+        raise AlofaError("invalid_argument", "decode_stack sizes disagree", f"k={tuple(k_cache.shape)} v={tuple(v_cache.shape)}")
+    lib = _decode_stack()
+    entry = ctypes.create_string_buffer(lib.alofa_decode_stack_layer_bytes())
+    rc = lib.alofa_decode_stack_layer(
+        ctypes.addressof(entry), _dev(qkv, "qkv", bf16), _dev(out, "out", bf16), _dev(gate_up, "gate_up", bf16), _dev(down, "down", bf16), _dev(gamma_mixer, "gamma_mixer", torch.float32),
+        _dev(gamma_ff, "gamma_ff", torch.float32), _dev(qkv_bias, "qkv_bias", torch.float32) if qkv_bias is not None else None, _dev(k_cache, "k_cache", bf16), _dev(v_cache, "v_cache", bf16),
+        float(eps_mixer), float(eps_ff), hidden, heads, kv_heads, head_dim, inter,
+    )
+    if rc:
+        raise AlofaError("state", "decode_stack: a layer's weights could not be described to the copy engine", f"rc={rc}")
+    return entry.raw
+
+
+def decode_stack(table, n_layers: int, ctas: int, sizes: tuple, page: int, scale: float, base, acc, positions, block_table, slot_map, rope, q, part_o, part_ml, act, barrier, status) -> None:
+    """All layers of a decode step, one token per request: what they add to the
+    stream ``base`` goes into the accumulator ``acc`` (zero before).  ``table``:
+    the entries of :func:`decode_stack_layer` one after the other; ``sizes``:
+    (hidden, heads, kv_heads, head_dim, inter); ``barrier``: a word that only
+    this kernel writes, zero at first."""
+    tokens, hidden = base.shape
+    hd, kv = sizes[3], sizes[2]
+    if hidden != sizes[0] or tuple(acc.shape) != (tokens, hidden) or block_table.shape[0] != tokens or q.shape[0] < tokens or act.numel() < decode_stack_act_numbers(tokens, sizes[4], ctas) or part_o.shape[0] < ctas or tokens * kv > ctas:
+        raise AlofaError("invalid_argument", "decode_stack sizes disagree", f"base={tuple(base.shape)} acc={tuple(acc.shape)} tables={tuple(block_table.shape)} ctas={ctas}")
+    _done(
+        _decode_stack().alofa_decode_stack(
+            _dev(table, "table"), n_layers, ctas, tokens, *sizes, page, block_table.shape[1], float(scale), _dev(base, "base", torch.float32), _dev(acc, "acc", torch.int64),
+            _dev(positions, "positions", torch.int32), _dev(block_table, "block_table", torch.int32), _dev(slot_map, "slot_map", torch.int32), _dev(rope, "rope", torch.float32),
+            _dev(q, "q", torch.bfloat16), _dev(part_o, "part_o", torch.float32), _dev(part_ml, "part_ml", torch.float32), _dev(act, "act", torch.bfloat16), _dev(barrier, "barrier", torch.int32),
+            _dev(status, "status", torch.int32), _stream(),
+        ),
+        "decode_stack", f"tokens={tokens} hidden={hidden} head_dim={hd}",
+    )

@@ -30,6 +30,7 @@ from ..cache.storage import CacheStorage, flat_specs, group_windows
 from ..csrc import ops
 from ..errors import AlofaError
 from ..parts.base import PagedKV, PagedRows
+from ..parts.decode_stack import DecodeStack
 from ..parts.model import Model
 from .arena import Arena
 from .context import GroupView, Layout, StepContext
@@ -103,6 +104,8 @@ class StepRunner:
         self._stream_acc = None
         if on_gpu and self.rt.dtype == torch.bfloat16 and os.environ.get("ALOFA_STREAM_ACC", "1") != "0":
             self._stream_acc = torch.zeros((2, self.STREAM_TOKENS, model.spec.hidden_size), dtype=torch.int64, device=self.rt.device)
+        # all layers of a decode step of a few tokens in one kernel, for models it is built for
+        self.decode_stack = DecodeStack.build(model, self.storage.caches, block_size) if self._stream_acc is not None else None
         self._layouts = {}
         self.cuda_graphs = cuda_graphs and on_gpu and model.graph_safe()
         self._graphs = {}  # decode steps by batch size; steps with prompt portions by (tokens, requests, wanted rows), and apart for those whose requests all start in them where a mixer tells them apart
@@ -205,6 +208,7 @@ class StepRunner:
         self.arena.begin_step()
         ctx.fed_tokens = self._fed if self.feeds_tokens else None
         ctx.stream_acc = self._stream_acc
+        ctx.decode_stack = self.decode_stack
         ctx.max_q_len, ctx.max_kv_len = max_q, max_kv
         ctx.decode_only = max_q == 1
         ctx.fresh = self.model.tells_fresh and not ctx.decode_only and lengths_fresh
@@ -352,6 +356,8 @@ class StepRunner:
         self._status.zero_()
         if self._stream_acc is not None:
             self._stream_acc.zero_()  # a kernel that gave up may have left the step half done
+        if self.decode_stack is not None:
+            self.decode_stack.reset()
         if code == 2:
             raise AlofaError("state", "a kernel gave up waiting on its own pipeline")
         raise AlofaError("out_of_range", "a kernel met a token id outside the vocabulary")

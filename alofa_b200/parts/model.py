@@ -89,7 +89,10 @@ class Model:
         # every row wanted, in order (a decode step): no picking, and the last block or a norm that reads the stream as base + accumulator may make them
         all_rows = ctx.n_out == ctx.n_tokens and bool((ctx.host_field("logit_rows") == np.arange(ctx.n_tokens, dtype=np.int32)).all())
         last = len(self.run) - 1
-        for i, (layer, cache) in enumerate(self.run):
+        whole = ctx.decode_stack is not None and ctx.decode_stack.takes(ctx, h)
+        if whole:
+            ctx.decode_stack.forward(ctx, h)
+        for i, (layer, cache) in enumerate(() if whole else self.run):
             block = self.layers[layer]
             if not getattr(block, "absorbs_pending", False):
                 ctx.flush_pending()

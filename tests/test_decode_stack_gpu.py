@@ -1,0 +1,114 @@
+"""All layers of a small decode step in one kernel, against float64 and against the same step layer by layer.
+
+Sizes go to the edges of what the kernel divides: one token to sixteen (eight fill a group of token columns), heads of 64
+and 128 in groups of one to eight, widths with an odd and an even number of 64-column chunks, a tile a CTA and several;
+contexts of one key, on either side of a page and of a granule of sixteen keys, and of several splits."""
+import numpy as np
+import pytest
+import torch
+
+import plain_qwen2 as plain
+
+pytestmark = pytest.mark.gpu
+
+# layers, hidden, heads, kv heads, head size, inter
+SHAPES = {
+    "h64_odd": (2, 192, 3, 3, 64, 576),  # chunks of 64 columns, one head a group
+    "h64_even": (3, 256, 8, 2, 64, 640),
+    "h64_group8": (2, 512, 8, 1, 64, 2560),
+    "h128": (2, 384, 6, 2, 128, 640),
+    "h128_group7": (2, 896, 7, 1, 128, 2432),
+}
+
+
+@pytest.fixture(scope="module")
+def folders(tmp_path_factory):
+    from alofa_b200.models.qwen2 import NAME, Qwen2Config
+    from alofa_b200.weights.random_init import write_random_model
+
+    base = tmp_path_factory.mktemp("decode_stack_models")
+    out = {}
+    for i, (name, (n, h, nh, nkv, hd, f)) in enumerate(SHAPES.items()):
+        out[name] = write_random_model(base / name, NAME, Qwen2Config(n, h, nh, nkv, hd, f, 300, 1e-6, 1e4, True, 4096), 40 + i, torch.bfloat16)
+    return out
+
+
+def decode(folder, contexts, steps, stacked, graphs=True, page=64):
+    """Logits of ``steps`` decode steps behind prompts of the given lengths, and whether the one kernel ran."""
+    from alofa_b200.csrc import ops
+    from alofa_b200.engine.loading import load_model
+    from alofa_b200.engine.step import StepEntry, StepRunner
+
+    model, _, _ = load_model(folder, "bfloat16")
+    runner = StepRunner(model, block_size=page, num_pages=sum((c + steps) // page + 1 for c in contexts) + 2, max_requests=len(contexts), max_tokens=4096, max_step_tokens=2048, cuda_graphs=graphs)
+    assert runner.decode_stack is not None
+    runner.decode_stack.FEWEST_TOKENS = 1
+    if not stacked:
+        runner.decode_stack = None
+    rng = np.random.default_rng(5)
+    seqs = [[int(t) for t in rng.integers(0, 300, c + steps)] for c in contexts]
+    slots = [runner.admit(i) for i in range(len(contexts))]
+    for slot, ids, c in zip(slots, seqs, contexts):
+        if c:
+            for lo in range(0, c, 2048):
+                runner.forward([StepEntry(slot, ids[lo : min(c, lo + 2048)])])
+    out = []
+    for t in range(steps):
+        before = ops.launch_count()
+        out.append(runner.forward([StepEntry(s, [ids[c + t]], [0]) for s, ids, c in zip(slots, seqs, contexts)]).clone())
+        launched = ops.launch_count() - before
+    runner.check_status()
+    assert runner._stream_acc.abs().sum().item() == 0
+    return torch.stack(out), launched, seqs
+
+
+@pytest.mark.parametrize("name", list(SHAPES))
+@pytest.mark.parametrize("contexts", [[0], [1], [63, 15], [16, 64, 17], [0, 127, 300, 1, 640, 255, 256, 257], [5] * 9, [3000, 20] + [33 * i for i in range(14)]])
+def test_matches_layer_by_layer(folders, name, contexts):
+    got, launched, _ = decode(folders[name], contexts, 3, True)
+    want, more, _ = decode(folders[name], contexts, 3, False)
+    assert launched < more, "the step did not run as one kernel"
+    # both round the same operands to bfloat16 (2^-9) and differ in the order of fp32 sums alone, so in which way close cases round:
+    # a few roundings a layer, each 2^-9 of a row's size at most and mostly averaged out over the products they go into
+    assert (got - want).norm() <= 2**-8 * want.norm()
+    assert (got - want).abs().max() <= 2**-4 * want.abs().max()
+
+
+def test_against_plain_and_repeats_bit_for_bit(folders):
+    contexts = [0, 70, 513]
+    got, _, seqs = decode(folders["h64_even"], contexts, 4, True)
+    again, _, _ = decode(folders["h64_even"], contexts, 4, True, graphs=False)
+    assert torch.equal(got, again)
+    wts, cfg = plain.load(folders["h64_even"])
+    for i, (c, ids) in enumerate(zip(contexts, seqs)):
+        want = torch.from_numpy(np.asarray(plain.forward(ids, wts, cfg)))[c:].float()
+        have = got[:, i].cpu().float()
+        assert (have - want).norm() <= 1e-2 * want.norm()  # bfloat16 operands
+
+
+def test_smaller_pages(folders):
+    contexts = [31, 200]
+    got, _, _ = decode(folders["h128"], contexts, 2, True, page=16)
+    want, _, _ = decode(folders["h128"], contexts, 2, True, page=64)
+    assert torch.equal(got, want)  # keys are taken sixteen at a time whatever the pages
+
+
+def test_model_loaded_again(folders):
+    """The kernel's table of weights follows a model that is loaded again behind the runner's back."""
+    from alofa_b200.engine.loading import load_model
+    from alofa_b200.engine.step import StepEntry, StepRunner
+    from alofa_b200.parts.linear import RESIDUAL, Linear
+
+    model, _, _ = load_model(folders["h64_even"], "bfloat16")
+    runner = StepRunner(model, block_size=64, num_pages=4, max_requests=1, max_tokens=128, max_step_tokens=64, cuda_graphs=False)
+    runner.decode_stack.FEWEST_TOKENS = 1
+    first = runner.forward([StepEntry(runner.admit(1), [7], [0])]).clone()
+    for block in model.layers:
+        block.mixer.out = Linear(block.mixer.out.weight * 2, None, RESIDUAL)
+    runner.release(0)
+    changed = runner.forward([StepEntry(runner.admit(2), [7], [0])]).clone()
+    runner.release(0)
+    runner.decode_stack = None
+    want = runner.forward([StepEntry(runner.admit(3), [7], [0])]).clone()
+    assert (first - want).norm() > 0.01 * want.norm()
+    assert (changed - want).norm() <= 2**-8 * want.norm()
