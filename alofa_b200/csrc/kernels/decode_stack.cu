@@ -28,6 +28,7 @@
 //
 // Every wait is bounded: after the limit the status word is raised, every CTA skips what is left, waits
 // for its own copies in flight and returns.
+#include <stddef.h>
 #include <string.h>
 
 #include "common.cuh"
@@ -146,10 +147,13 @@ struct Small {  // of shared memory
   int splits[MAX_TOKENS];
   int per_split, item_token, item_group, item_first, item_last;  // granules of keys a split has at most; this CTA's item
   int first_row[WARPS];      // of the cache: where the warp's first granule lies
-  float wm[WARPS][8], wl[WARPS][8];
+  alignas(16) float wm[WARPS][8];  // attention: each warp's maxima and sums, by head
+  alignas(16) float wl[WARPS][8];
   alignas(8) LayerVectors layer[2];  // of this layer and the next
   int abort_flag;
 };
+
+static_assert(sizeof(Small) % 16 == 0 && offsetof(Small, wm) % 16 == 0 && offsetof(Small, wl) % 16 == 0 && offsetof(Small, layer) % 8 == 0, "vector loads");
 
 // The next phase in which a warp has pieces.
 __device__ __forceinline__ void next_piece(Loader& ld, const Small& sm, int warp, int n_layers) {
