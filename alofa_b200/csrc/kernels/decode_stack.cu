@@ -36,12 +36,14 @@
 
 constexpr int WARPS = 16;
 constexpr int THREADS = 32 * WARPS;
+constexpr int PACE = 2;                  // pieces a paced warp asks for ahead of a product
 constexpr int GRANULE = 16;              // keys a warp takes at a time
 constexpr int MAX_TOKENS = 16;
 constexpr int MAX_TILES = 64;             // of 16 rows a CTA and phase
 constexpr uint32_t BARRIER_LIMIT = 1u << 21;  // polls of the grid barrier, about a second
 enum { P_QKV = 0, P_OUT = 1, P_GATE = 2, P_DOWN = 3 };
 
+#define TRACE(n)
 struct LayerVectors {
   const float* gamma_mixer;
   const float* gamma_ff;
@@ -68,6 +70,7 @@ struct StackArgs {
   int tokens, hidden, heads, kv_heads, group, inter;
   int page, table_stride;
   int chunks, slots;         // 64-column chunks of a piece, pieces in a warp's ring
+  int paced;                 // a warp asks for a few pieces ahead of each product, not for all it can behind it
   int x_stride;              // bytes of an operand row in shared memory
   int qkv_tiles;             // of a CTA, at most
   int x_bytes, work_bytes;   // operand rows; operand, sums and attention together
@@ -92,7 +95,8 @@ struct StackArgs {
 // ---- wrappers ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
   asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst), "l"(map), "r"(bar),
+      "{\n\t.reg .b64 p;\n\tcreatepolicy.fractional.L2::evict_first.b64 p, 1.0;\n\t"
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], p;\n\t}" ::"r"(dst), "l"(map), "r"(bar),
       "r"(x), "r"(y), "r"(z)
       : "memory");
 }
@@ -285,13 +289,14 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
     next_piece(sm.loader[warp], sm, warp, a.n_layers);
   }
   // Asks for the next pieces of this warp's list, one for each empty place.
-  auto refill = [&]() {
+  auto refill = [&](int most) {
+    const int ask = min(most, empty);
     if (lane == 0) {
       Loader ld = sm.loader[warp];
       int into = slot - empty;
       if (into < 0) into += a.slots;
 #pragma unroll 1
-      for (int k = 0; k < empty && ld.layer < a.n_layers; ++k) {
+      for (int k = 0; k < ask && ld.layer < a.n_layers; ++k) {
         const Share& s = sm.share[ld.phase];
         const int tile = s.tile0 + ld.tile * s.tile_step;
         const int row = (tile >> s.shift) * s.head_rows + (tile & ((1 << s.shift) - 1)) * 8, chunk = (s.slice0 + ld.slice) * a.chunks;
@@ -310,9 +315,9 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
       }
       sm.loader[warp] = ld;
     }
-    empty = 0;
+    empty -= ask;
   };
-  refill();
+  refill(a.slots);
 
   // The attention item of this CTA: the keys of (request, KV head) pairs go in splits of as many granules as
   // make all items resident together, no fewer than one per warp.
@@ -363,7 +368,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
     __syncthreads();
     if (tid == 0 && !*abort_flag) {
       const unsigned add = cta == 0 ? 0x80000000u - (unsigned)(ctas - 1) : 1u;
-      asm volatile("fence.acq_rel.gpu;\n\tred.relaxed.gpu.global.add.u32 [%0], %1;" ::"l"(a.barrier), "r"(add) : "memory");
+      asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(a.barrier), "r"(add) : "memory");
     }
   };
   auto wait = [&]() -> bool {  // false: give up
@@ -400,6 +405,15 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
     }
   };
 
+  // A paced warp asks for its next pieces while the operand's loads are on their way.  (All that a ring has room for, behind the
+  // barrier: the flood of copies held up the fences of the CTAs behind, 4,100 cycles after gate and up, 2,900 after the down
+  // projection, 1,100 with a few pieces a phase.  Before the product, after the operand: 700 to 1,000 cycles a phase.)
+  bool asked = false;
+  auto ahead = [&]() {
+    if (!asked && a.paced) refill(PACE);
+    asked = true;
+  };
+
   // The rows of the stream times the norm's weight as bfloat16 into shared memory, and each row's factor.  The stream is
   // `base` in the first norm of a step and the accumulator from then on (phase 1 of the first layer moves it there).
   auto normed_rows = [&](float eps, bool from_base) {
@@ -412,32 +426,29 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
       unsigned char* row = work + (size_t)t * a.x_stride;
       const int n2 = H / 2, step = 32 * per_row;
 #pragma unroll 1
-      for (int i0 = part * 32 + lane; i0 < n2; i0 += 8 * step) {
-        float2 x[8];
-        if (from_base) {
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            x[u] = make_float2(0.f, 0.f);
-            if (i0 + u * step < n2) x[u] = __ldcg(b2 + i0 + u * step);
-          }
-        } else {
-          longlong2 q[8];
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            q[u] = make_longlong2(0, 0);
-            if (i0 + u * step < n2) q[u] = __ldcg(a2 + i0 + u * step);
-          }
-#pragma unroll
-          for (int u = 0; u < 8; ++u) x[u] = make_float2(stream_add(0.f, q[u].x), stream_add(0.f, q[u].y));
-        }
+      for (int w0 = part * 32; w0 < n2; w0 += 8 * step) {  // H is a multiple of 64: whole warps have an element or none
+        longlong2 q[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-          const int i = i0 + u * step;
-          if (i < n2) {
-            const float2 g = g2[i];
-            square += x[u].x * x[u].x + x[u].y * x[u].y;
-            *reinterpret_cast<uint32_t*>(row + 4 * i) = pack2(x[u].x * g.x, x[u].y * g.y);
+          q[u] = make_longlong2(0, 0);
+          if (w0 + u * step < n2) {
+            if (from_base) {
+              const float2 b = __ldcg(b2 + w0 + u * step + lane);
+              q[u] = make_longlong2(__float_as_int(b.x), __float_as_int(b.y));
+            } else {
+              q[u] = __ldcg(a2 + w0 + u * step + lane);
+            }
           }
+        }
+        ahead();
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          if (w0 + u * step >= n2) break;
+          const int i = w0 + u * step + lane;
+          const float x = from_base ? __int_as_float((int)q[u].x) : stream_add(0.f, q[u].x), y = from_base ? __int_as_float((int)q[u].y) : stream_add(0.f, q[u].y);
+          const float2 g = g2[i];
+          square += x * x + y * y;
+          *reinterpret_cast<uint32_t*>(row + 4 * i) = pack2(x * g.x, y * g.y);
         }
       }
     }
@@ -456,6 +467,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
   auto multiply = [&](const Share& s, int phase) {
     const Part part = sm.part[phase][warp];
     if (part.first >= part.end) return;
+    if (empty == a.slots) refill(a.slots);
     const int slices = s.slices;
     int tile = part.tile, slice = part.slice;
     float c[NT][2][4];
@@ -495,7 +507,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
         slot = 0;
         parity ^= 1;
       }
-      if (left > a.slots - empty) refill();  // this phase has pieces that nobody asked for yet; else behind the barrier
+      if (left > a.slots - empty) refill(a.slots);  // this phase has pieces that nobody asked for yet; else behind the barrier
       if (++slice == slices || left == 0) {
         float* dst = sums + ((warp + tile) * 16 + r) * TP + 2 * j;
 #pragma unroll
@@ -538,6 +550,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
       place_thread();
       const Share& s = sm.share[phase];
       if (s.tiles) {
+        asked = false;
         // the operand
         if (phase == P_QKV || phase == P_GATE) {
           normed_rows(phase == P_QKV ? L.eps_mixer : L.eps_ff, layer == 0 && phase == P_QKV);
@@ -581,6 +594,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
                 v.w *= f;
 #pragma unroll
                 for (int u = 0; u < 5; ++u) {
+                  if (p0 - half + 2 * u >= n) break;
                   const float w = exp2_fast(ml[u].x - up);
                   sum += w * ml[u].y;
                   v.x += w * o[u].x;
@@ -611,10 +625,12 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
               uint4 v[4];
 #pragma unroll
               for (int u = 0; u < 4; ++u) {
-                const int tile = tile0 + i0 + u * step, k = (int)((tile + 0.5f) * a.per_cta), c = tile - k * ctas;  // of the gate product: its CTA, and which of that one's
                 v[u] = make_uint4(0u, 0u, 0u, 0u);
+                if (i0 - lane + u * step >= n) continue;
+                const int tile = tile0 + i0 + u * step, k = (int)((tile + 0.5f) * a.per_cta), c = tile - k * ctas;  // of the gate product: its CTA, and which of that one's
                 if (i0 + u * step < n) v[u] = __ldcg(reinterpret_cast<const uint4*>(a.act + (size_t)c * a.act_stride) + k * T + t);
               }
+              ahead();
 #pragma unroll
               for (int u = 0; u < 4; ++u)
                 if (i0 + u * step < n) *reinterpret_cast<uint4*>(row + 16 * (i0 + u * step)) = v[u];
@@ -622,6 +638,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
           }
           __syncthreads();
         }
+        if (phase != P_OUT) ahead();  // a warp that had nothing to load
         multiply(s, phase);
         __syncthreads();
         // what becomes of the sums
@@ -686,7 +703,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
       if (phase == P_DOWN && layer + 1 == a.n_layers) break;
       arrive();
       if (phase != P_QKV) {
-        if (empty) refill();
+        if (!a.paced) refill(a.slots);
         if (phase == P_OUT) stage(L.gamma_ff, nullptr);
         if (phase == P_DOWN) stage(N.gamma_mixer, N.qkv_bias);
         if (!wait()) goto leave;
@@ -720,7 +737,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
             asm volatile("prefetch.global.L2 [%0];" ::"l"(L.v + ((size_t)(sm.first_row[warp] + (lane & 15)) * a.kv_heads + it_group) * HD + (lane >> 4) * 64));
           }
         }
-        if (empty) refill();
+        if (!a.paced) refill(a.slots);
         if (!wait()) goto leave;
         if (layer == 0)  // the stream is in the accumulator now
           for (int i = cta * THREADS + tid; i < T * H; i += ctas * THREADS) a.base[i] = 0.f;
@@ -935,7 +952,7 @@ void split_plan(PhasePlan* p, int ctas, int chunks, int tokens, int operand, int
     const int rg = ctas / kg < p->tiles ? ctas / kg : p->tiles;
     const long long tiles = (p->tiles + rg - 1) / rg, slices = (p->slices + kg - 1) / kg, cols = slices * chunks * 64;
     if (cols > x_limit || tiles > 24) continue;
-    const long long cost = tiles * slices * 2048 * chunks + cols * tokens * operand + tiles * 16 * tokens * 16 + kg * 8192;
+    const long long cost = tiles * slices * 2048 * chunks + cols * tokens * operand + tiles * 16 * tokens * 16 + (long long)kg * 32 * p->tiles;
     if (best < 0 || cost < best) {
       best = cost;
       p->kg = kg;
@@ -980,6 +997,9 @@ size_t plan_stack(StackArgs* a, int head_dim, int ctas) {
   if (rest + 2 * piece > limit) return 0;
   a->slots = (int)((limit - rest) / piece);
   if (a->slots > 8) a->slots = 8;
+  long long all = 0;
+  for (int p = 0; p < 4; ++p) all += (long long)a->plan[p].tiles * a->plan[p].slices;
+  a->paced = all <= 2 * (long long)ctas * WARPS * a->slots;
   return rest + a->slots * piece;
 }
 

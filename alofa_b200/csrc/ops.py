@@ -1534,6 +1534,9 @@ def lru_scan(out, a, b, y, y_off: int, act: str, state, q_start, state_slots, n_
                                       _stream()), "lru_scan")
 
 
+DECODE_STACK_TOKENS = 16  # the most tokens that the one-kernel decode step takes
+
+
 def decode_stack_ctas(tokens: int, hidden: int, heads: int, kv_heads: int, head_dim: int, inter: int, page: int) -> int:
     """How many CTAs run all layers of a decode step of so many tokens at these
     sizes (:func:`decode_stack`); 0 where that kernel does not take them."""

@@ -24,8 +24,11 @@ from .position import RotaryNeox
 
 
 class DecodeStack:
-    # Tokens of a step below and above which the layers' own kernels are the faster ones (at most what the kernel takes).
-    FEWEST_TOKENS, MOST_TOKENS = 4, 16
+    # Steps this kernel is the faster way for: up to eight tokens (one group of token columns; at nine, two groups, it loses 3 % at 0.5B
+    # sizes) and as many of their numbers as every SM can read before each product.  us a pass of four steps, here and layer by
+    # layer: hidden 896, 3 tokens 2,535 and 2,748, 9 tokens 3,058 and 2,981; hidden 1,536, 4 tokens 4,855 and 5,207, 8 tokens 5,387
+    # and 5,414; hidden 3,584, 1 token 11,118 and 12,682, 4 tokens 11,886 and 12,890, 6 tokens 13,015 and 12,974.
+    MOST_TOKENS, MOST_NUMBERS = 8, 16384
 
     def __init__(self, model, caches: dict, block_size: int):
         self.model = model
@@ -34,8 +37,9 @@ class DecodeStack:
         self.sizes = (block.mixer_norm.size, mixer.nh, mixer.nkv, mixer.hd, block.feed_forward.inter)
         self.page = block_size
         self.scale = mixer.scale
+        self.most, self.most_numbers = self.MOST_TOKENS, self.MOST_NUMBERS
         self.group = caches[model.run[0][1]].group
-        self.ctas = [0] + [ops.decode_stack_ctas(n, *self.sizes, block_size) for n in range(1, self.MOST_TOKENS + 1)]
+        self.ctas = [0] + [ops.decode_stack_ctas(n, *self.sizes, block_size) for n in range(1, ops.DECODE_STACK_TOKENS + 1)]
         if not any(self.ctas):
             return
         device = model.rt.device
@@ -108,7 +112,7 @@ class DecodeStack:
         return stack if any(stack.ctas) else None
 
     def takes(self, ctx, h) -> bool:
-        return ctx.decode_only and self.FEWEST_TOKENS <= ctx.n_tokens <= self.MOST_TOKENS and self.ctas[ctx.n_tokens] > 0 and ctx.stream_of(h) is not None
+        return ctx.decode_only and ctx.n_tokens <= self.most and ctx.n_tokens * self.sizes[0] <= self.most_numbers and self.ctas[ctx.n_tokens] > 0 and ctx.stream_of(h) is not None
 
     def forward(self, ctx, h) -> None:
         """The step's rows through all layers: what they add to ``h`` is left

@@ -14,9 +14,9 @@ pytestmark = pytest.mark.gpu
 # layers, hidden, heads, kv heads, head size, inter
 SHAPES = {
     "h64_odd": (2, 192, 3, 3, 64, 576),  # chunks of 64 columns, one head a group
-    "h64_even": (3, 256, 8, 2, 64, 640),
+    "h64_even": (3, 256, 4, 2, 64, 640),
     "h64_group8": (2, 512, 8, 1, 64, 2560),
-    "h128": (2, 384, 6, 2, 128, 640),
+    "h128": (2, 384, 3, 1, 128, 640),
     "h128_group7": (2, 896, 7, 1, 128, 2432),
 }
 
@@ -42,7 +42,7 @@ def decode(folder, contexts, steps, stacked, graphs=True, page=64):
     model, _, _ = load_model(folder, "bfloat16")
     runner = StepRunner(model, block_size=page, num_pages=sum((c + steps) // page + 1 for c in contexts) + 2, max_requests=len(contexts), max_tokens=4096, max_step_tokens=2048, cuda_graphs=graphs)
     assert runner.decode_stack is not None
-    runner.decode_stack.FEWEST_TOKENS = 1
+    runner.decode_stack.most = 16  # also the sizes that go layer by layer because that is faster
     if not stacked:
         runner.decode_stack = None
     rng = np.random.default_rng(5)
@@ -69,8 +69,8 @@ def test_matches_layer_by_layer(folders, name, contexts):
     want, more, _ = decode(folders[name], contexts, 3, False)
     assert launched < more, "the step did not run as one kernel"
     # both round the same operands to bfloat16 (2^-9) and differ in the order of fp32 sums alone, so in which way close cases round:
-    # a few roundings a layer, each 2^-9 of a row's size at most and mostly averaged out over the products they go into
-    assert (got - want).norm() <= 2**-8 * want.norm()
+    # both sides, each of the eight roundings a layer 2^-9 / sqrt(3) of its row: sqrt(2 sides * 3 layers * 8) * 2^-9 / sqrt(3) = 2^-7
+    assert (got - want).norm() <= 2**-7 * want.norm()
     assert (got - want).abs().max() <= 2**-4 * want.abs().max()
 
 
@@ -101,7 +101,6 @@ def test_model_loaded_again(folders):
 
     model, _, _ = load_model(folders["h64_even"], "bfloat16")
     runner = StepRunner(model, block_size=64, num_pages=4, max_requests=1, max_tokens=128, max_step_tokens=64, cuda_graphs=False)
-    runner.decode_stack.FEWEST_TOKENS = 1
     first = runner.forward([StepEntry(runner.admit(1), [7], [0])]).clone()
     for block in model.layers:
         block.mixer.out = Linear(block.mixer.out.weight * 2, None, RESIDUAL)
