@@ -6,13 +6,17 @@
 // kernels, even with programmatic launch, a hand-over costs 1.0 to 1.9 us and a product's body starts
 // on a cold pipeline.  Here one CTA per SM stays resident for the whole step (a cooperative launch).
 // Each of its 16 warps owns a list of weight pieces, known from the shapes alone, and a ring in shared
-// memory that it keeps full by TMA: weights of later phases and of the next layer arrive
+// memory that TMA fills ahead of the product: weights of later phases and of the next layer arrive
 // while a phase waits for the one before it.  Five phases a layer, a barrier over the grid between them:
 //   1  norm, q/k/v product, bias, rotation, cache write
 //   2  attention, a request's keys split over CTAs
 //   3  merge of the key splits, output projection, added into the stream
 //   4  norm, gate and up product, silu(gate) * up
 //   5  down projection, added into the stream
+// A layer of 0.5B sizes takes 39,000 to 46,000 cycles at one to eight tokens (20 to 24 us; 23 to 28 as kernels, 4.5 for the
+// weights alone): per phase 1,100 for the barrier's fence, 800 for the wait of the last CTA, 1,500 to 3,700 for the operand
+// (a trip to L2 and the work on it), 800 to 1,500 for the product, 600 to 1,600 for what becomes of its sums.  us a pass of
+// perf/cases.py, layer by layer and here: decode_05b_1 4,866 and 4,747, decode_05b_8 5,949 and 5,430, decode_7b_4 12,890 and 11,836.
 // Products run on mma.sync m16n8k16 with the weights as the 16-row operand and 8 tokens as the other:
 // a warp multiplies straight from its ring, without the tensor-memory round trip of tcgen05 (which for a
 // handful of tokens took 70 to 110 ns per 128 x 16 x 16 instruction); at up to 16 tokens the math is a
@@ -36,14 +40,13 @@
 
 constexpr int WARPS = 16;
 constexpr int THREADS = 32 * WARPS;
-constexpr int PACE = 2;                  // pieces a paced warp asks for ahead of a product
+constexpr int PACE = 3;                  // pieces a paced warp asks for ahead of a product
 constexpr int GRANULE = 16;              // keys a warp takes at a time
 constexpr int MAX_TOKENS = 16;
 constexpr int MAX_TILES = 64;             // of 16 rows a CTA and phase
 constexpr uint32_t BARRIER_LIMIT = 1u << 21;  // polls of the grid barrier, about a second
 enum { P_QKV = 0, P_OUT = 1, P_GATE = 2, P_DOWN = 3 };
 
-#define TRACE(n)
 struct LayerVectors {
   const float* gamma_mixer;
   const float* gamma_ff;
@@ -53,7 +56,7 @@ struct LayerVectors {
   float eps_mixer, eps_ff;
 };
 struct alignas(64) StackLayer {
-  CUtensorMap maps[4];  // q/k/v, output, gate and up, down: boxes of 8 rows x `chunks` x 64 columns
+  CUtensorMap maps[4];  // q/k/v, output, gate and up, down: boxes of 8 rows x 2 x `chunks` x 64 columns
   LayerVectors vectors;
   int pad[4];
 };
@@ -93,11 +96,13 @@ struct StackArgs {
 };
 
 // ---- wrappers ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
+// A piece: both groups of rows at once, marked to leave L2 first (a weight is read once a step; without the mark what the phases
+// hand over was driven out: four requests of the 7B shape 12.6 and 12.1 ms a pass of four steps).
+__device__ __forceinline__ void tma_load_piece(uint32_t dst, const CUtensorMap* map, uint32_t bar, int row, int chunk) {
   asm volatile(
       "{\n\t.reg .b64 p;\n\tcreatepolicy.fractional.L2::evict_first.b64 p, 1.0;\n\t"
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], p;\n\t}" ::"r"(dst), "l"(map), "r"(bar),
-      "r"(x), "r"(y), "r"(z)
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %3, %5}], [%2], p;\n\t}" ::"r"(dst), "l"(map), "r"(bar),
+      "r"(0), "r"(row), "r"(chunk)
       : "memory");
 }
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
@@ -128,11 +133,13 @@ struct Share {
   int tile0, tile_step, tiles;  // local tile i is tile0 + i * tile_step
   int slice0, slices;
   int pieces, warps;            // tiles * slices, dealt to so many warps: warp w has pieces [w * pieces / warps, (w + 1) * pieces / warps)
-  int shift, head_rows, second; // a tile's rows: 8 from (tile >> shift) * head_rows + (tile & mask) * 8, and 8 from `second` further on
+  int shift, head_rows; // a tile's rows: 8 from (tile >> shift) * head_rows + (tile & mask) * 8, and 8 as far on as the map's second group is
 };
 
-struct Loader {  // a warp's place in its list of pieces, and how many it has asked for
-  int layer, phase, piece, end, tile, slice, asked;
+struct alignas(16) Loader {  // a warp's next piece and its place in the list of them, how many it has asked for
+  int row, chunk, layer, phase;
+  int piece, end, tile, slice;
+  int slices, asked, pad[2];
 };
 struct Part {  // of a phase, for one warp: its pieces, and tile and slice of the first
   short first, end, tile, slice;
@@ -141,7 +148,7 @@ struct Part {  // of a phase, for one warp: its pieces, and tile and slice of th
 struct Small {  // of shared memory
   Share share[4];
   Part part[4][WARPS];
-  Loader loader[WARPS];
+  alignas(16) Loader loader[WARPS];
   unsigned char first_warp[4][MAX_TILES], last_warp[4][MAX_TILES];  // of the warps with pieces of a tile
   float square[WARPS];       // each warp's sum of squares in a norm
   float factor[MAX_TOKENS];  // 1 / sqrt(mean square + eps)
@@ -157,10 +164,16 @@ struct Small {  // of shared memory
   int abort_flag;
 };
 
-static_assert(sizeof(Small) % 16 == 0 && offsetof(Small, wm) % 16 == 0 && offsetof(Small, wl) % 16 == 0 && offsetof(Small, layer) % 8 == 0, "vector loads");
+static_assert(sizeof(Small) % 16 == 0 && offsetof(Small, loader) % 16 == 0 && offsetof(Small, wm) % 16 == 0 && offsetof(Small, wl) % 16 == 0 && offsetof(Small, layer) % 8 == 0, "vector loads");
 
+// Where a piece lies in its weight.
+__device__ __forceinline__ void place_piece(Loader& ld, const Share& s, int chunks) {
+  const int tile = s.tile0 + ld.tile * s.tile_step;
+  ld.row = (tile >> s.shift) * s.head_rows + (tile & ((1 << s.shift) - 1)) * 8;
+  ld.chunk = (s.slice0 + ld.slice) * chunks;
+}
 // The next phase in which a warp has pieces.
-__device__ __forceinline__ void next_piece(Loader& ld, const Small& sm, int warp, int n_layers) {
+__device__ __forceinline__ void next_phase(Loader& ld, const Small& sm, int warp, int n_layers, int chunks) {
   do {
     if (++ld.phase == 4) {
       ld.phase = 0;
@@ -172,6 +185,8 @@ __device__ __forceinline__ void next_piece(Loader& ld, const Small& sm, int warp
     ld.tile = p.tile;
     ld.slice = p.slice;
   } while (ld.piece >= ld.end);
+  ld.slices = sm.share[ld.phase].slices;
+  place_piece(ld, sm.share[ld.phase], chunks);
 }
 
 // A register that only some paths write counts as held from the start of the loop over layers to its end; that is why what a
@@ -231,7 +246,6 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
     s.warps = min(WARPS, s.pieces);  // each of them has a piece
     s.shift = tid == P_QKV ? (HD == 128 ? 3 : 2) : tid == P_GATE ? 30 : 0;
     s.head_rows = tid == P_QKV ? HD : 16;
-    s.second = tid == P_QKV ? HD / 2 : tid == P_GATE ? a.inter : 8;
     sm.share[tid] = s;
   }
   if (tid < (int)(sizeof(LayerVectors) / 4)) reinterpret_cast<int*>(&sm.layer[0])[tid] = reinterpret_cast<const int*>(&a.layers[0].vectors)[tid];
@@ -285,8 +299,10 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
   int taken = 0;        // pieces multiplied
   int empty = a.slots;  // places of the ring that nothing is on its way to, the last of them before `slot`
   if (lane == 0) {
-    sm.loader[warp] = {0, -1, 0, 0, 0, 0, 0};
-    next_piece(sm.loader[warp], sm, warp, a.n_layers);
+    Loader ld = {};
+    ld.phase = -1;
+    next_phase(ld, sm, warp, a.n_layers, a.chunks);
+    sm.loader[warp] = ld;
   }
   // Asks for the next pieces of this warp's list, one for each empty place.
   auto refill = [&](int most) {
@@ -297,20 +313,18 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
       if (into < 0) into += a.slots;
 #pragma unroll 1
       for (int k = 0; k < ask && ld.layer < a.n_layers; ++k) {
-        const Share& s = sm.share[ld.phase];
-        const int tile = s.tile0 + ld.tile * s.tile_step;
-        const int row = (tile >> s.shift) * s.head_rows + (tile & ((1 << s.shift) - 1)) * 8, chunk = (s.slice0 + ld.slice) * a.chunks;
-        const uint32_t dst = my_ring + (uint32_t)into * piece_bytes, bar = smem_u32(my_bars + into);
-        const CUtensorMap* map = &a.layers[ld.layer].maps[ld.phase];
         mbar_expect_tx(my_bars + into, piece_bytes);
-        tma_load_3d(dst, map, bar, 0, row, chunk);
-        tma_load_3d(dst + piece_bytes / 2, map, bar, 0, row + s.second, chunk);
+        tma_load_piece(my_ring + (uint32_t)into * piece_bytes, &a.layers[ld.layer].maps[ld.phase], smem_u32(my_bars + into), ld.row, ld.chunk);
         ++ld.asked;
-        if (++ld.slice == s.slices) {
+        if (++ld.piece == ld.end) {
+          next_phase(ld, sm, warp, a.n_layers, a.chunks);
+        } else if (++ld.slice == ld.slices) {
           ld.slice = 0;
           ++ld.tile;
+          place_piece(ld, sm.share[ld.phase], a.chunks);
+        } else {
+          ld.chunk += a.chunks;
         }
-        if (++ld.piece == ld.end) next_piece(ld, sm, warp, a.n_layers);
         if (++into == a.slots) into = 0;
       }
       sm.loader[warp] = ld;
@@ -406,8 +420,10 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
   };
 
   // A paced warp asks for its next pieces while the operand's loads are on their way.  (All that a ring has room for, behind the
-  // barrier: the flood of copies held up the fences of the CTAs behind, 4,100 cycles after gate and up, 2,900 after the down
-  // projection, 1,100 with a few pieces a phase.  Before the product, after the operand: 700 to 1,000 cycles a phase.)
+  // barrier: that flood of copies held up the fences of the CTAs behind, 4,100 cycles after gate and up and 2,900 after the
+  // down projection, 1,100 to 1,500 this way.  Before the product, after the operand: 700 to 1,000 cycles a phase more.  0.5B sizes, us
+  // a pass of eight steps with one and eight requests: behind the barrier 5,031 and 5,658, one piece a phase 4,860 and 5,520, two
+  // 4,774 and 5,494, three 4,747 and 5,430.)
   bool asked = false;
   auto ahead = [&]() {
     if (!asked && a.paced) refill(PACE);
@@ -480,13 +496,13 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
     uint32_t x_lane[NT];
 #pragma unroll
     for (int n = 0; n < NT; ++n) x_lane[n] = smem_u32(work) + min(8 * n + (lane & 7), T - 1) * a.x_stride + (lane >> 3) * 16;  // rows past the last: a sum that nobody reads
-    const uint32_t w_half = ((lane >> 3) & 1) * (piece_bytes / 2) + (lane & 7) * 128, w_k = lane >> 4, w_x = lane & 7;
+    const uint32_t w_half = ((lane >> 3) & 1) * 1024 + (lane & 7) * 128, w_k = lane >> 4, w_x = lane & 7;
 #pragma unroll 1
     for (int left = part.end - part.first - 1; left >= 0; --left) {
       if (!__all_sync(0xffffffffu, mbar_wait(my_bars + slot, parity, abort_flag))) return;
       uint32_t w_at = my_ring + (uint32_t)slot * piece_bytes + w_half, x_at = slice * a.chunks * 128;
 #pragma unroll 1
-      for (int ch = 0; ch < a.chunks; ++ch, w_at += 1024, x_at += 128) {
+      for (int ch = 0; ch < a.chunks; ++ch, w_at += 2048, x_at += 128) {
         uint32_t b[NT][2][4], w[4][4];
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
@@ -925,15 +941,15 @@ leave:
 // ---------------------------------------------------------------------------------------------------------
 namespace {
 
-// A [rows, 64 * n] bf16 row-major matrix as boxes of 8 rows x `chunks` x 64 columns, 128-byte swizzle.
-bool make_piece_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, int chunks) {
+// A [rows, 64 * n] bf16 row-major matrix as boxes of 8 rows, 8 rows `second` further on, and `chunks` x 64 columns; 128-byte swizzle.
+bool make_piece_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t second, int chunks) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
-  cuuint64_t dims[3] = {64, (cuuint64_t)rows, (cuuint64_t)(cols / 64)};
-  cuuint64_t strides[2] = {(cuuint64_t)cols * 2, 128};
-  cuuint32_t box[3] = {64, 8, (cuuint32_t)chunks};
-  cuuint32_t elem[3] = {1, 1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  cuuint64_t dims[4] = {64, (cuuint64_t)(rows - second), 2, (cuuint64_t)(cols / 64)};
+  cuuint64_t strides[3] = {(cuuint64_t)cols * 2, (cuuint64_t)(second * cols * 2), 128};
+  cuuint32_t box[4] = {64, 8, 2, (cuuint32_t)chunks};
+  cuuint32_t elem[4] = {1, 1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -999,6 +1015,8 @@ size_t plan_stack(StackArgs* a, int head_dim, int ctas) {
   if (a->slots > 8) a->slots = 8;
   long long all = 0;
   for (int p = 0; p < 4; ++p) all += (long long)a->plan[p].tiles * a->plan[p].slices;
+  // a ring that holds half a layer or more keeps up at that pace; larger models are bound by their weights (7B sizes: a layer is 24
+  // rings) and ask for all they can as soon as they can
   a->paced = all <= 2 * (long long)ctas * WARPS * a->slots;
   return rest + a->slots * piece;
 }
@@ -1060,8 +1078,8 @@ ALOFA_API int alofa_decode_stack_layer(void* entry, const void* qkv, const void*
   memset(&L, 0, sizeof(L));
   const int q_dim = heads * head_dim, chunks = (hidden / 64) % 2 || (q_dim / 64) % 2 || (inter / 64) % 2 ? 1 : 2;
   if (((uintptr_t)qkv | (uintptr_t)out | (uintptr_t)gate_up | (uintptr_t)down | (uintptr_t)gamma_mixer | (uintptr_t)gamma_ff | (uintptr_t)k | (uintptr_t)v) & 15) return ALOFA_ERR_ARGUMENT;
-  if (!make_piece_map(&L.maps[P_QKV], qkv, q_dim + 2 * kv_heads * head_dim, hidden, chunks) || !make_piece_map(&L.maps[P_OUT], out, hidden, q_dim, chunks) ||
-      !make_piece_map(&L.maps[P_GATE], gate_up, 2 * (uint64_t)inter, hidden, chunks) || !make_piece_map(&L.maps[P_DOWN], down, hidden, inter, chunks))
+  if (!make_piece_map(&L.maps[P_QKV], qkv, q_dim + 2 * kv_heads * head_dim, hidden, head_dim / 2, chunks) || !make_piece_map(&L.maps[P_OUT], out, hidden, q_dim, 8, chunks) ||
+      !make_piece_map(&L.maps[P_GATE], gate_up, 2 * (uint64_t)inter, hidden, inter, chunks) || !make_piece_map(&L.maps[P_DOWN], down, hidden, inter, 8, chunks))
     return ALOFA_ERR_LAUNCH;
   L.vectors.gamma_mixer = gamma_mixer;
   L.vectors.gamma_ff = gamma_ff;
