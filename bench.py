@@ -816,7 +816,8 @@ class KernelClock:
         self.pairs, self.windowed = pairs, windowed
         names = [n for n in dir(ops) if not n.startswith("_") and callable(getattr(ops, n)) and getattr(getattr(ops, n), "__module__", "") == ops.__name__
                  and n not in ("launch_count", "count_launches", "bound_stream", "attention_decode_wide_warps", "attention_decode_slots", "attention_bf16_supported",
-                               "gemm_tc_rope_splits", "gemm_tc_splits", "delta_pair_words", "latent_attention_bf16_supported", "load_library", "gemm_by_tile")]  # gemm_by_tile only chooses: its product is timed
+                               "gemm_tc_rope_splits", "gemm_tc_splits", "delta_pair_words", "latent_attention_bf16_supported", "load_library", "gemm_by_tile",
+                               "decode_stack_ctas", "decode_stack_layer", "decode_stack_act_numbers")]  # gemm_by_tile only chooses: its product is timed
         originals = {n: getattr(ops, n) for n in names}
         records = []
 
