@@ -1,4 +1,4 @@
-// All layers of a small decode step in one persistent kernel (sm_100a): up to 16 tokens, one per
+// All layers of a small decode step in one persistent kernel (sm_100a): up to eight tokens, one per
 // request, through a stack of layers  h += attention(rmsnorm(h)); h += feed_forward(rmsnorm(h))
 // with grouped-query attention over a paged cache, NeoX rotation of whole heads and a silu gate.
 //
@@ -16,10 +16,10 @@
 // A layer of 0.5B sizes takes 39,000 to 46,000 cycles at one to eight tokens (20 to 24 us; 23 to 28 as kernels, 4.5 for the
 // weights alone): per phase 1,100 for the barrier's fence, 800 for the wait of the last CTA, 1,500 to 3,700 for the operand
 // (a trip to L2 and the work on it), 800 to 1,500 for the product, 600 to 1,600 for what becomes of its sums.  us a pass of
-// perf/cases.py, layer by layer and here: decode_05b_1 4,866 and 4,747, decode_05b_8 5,949 and 5,430, decode_7b_4 12,890 and 11,836.
+// perf/cases.py, layer by layer and here: decode_05b_1 4,834 and 4,551, decode_05b_8 5,903 and 5,300, decode_7b_4 12,920 and 11,680.
 // Products run on mma.sync m16n8k16 with the weights as the 16-row operand and 8 tokens as the other:
 // a warp multiplies straight from its ring, without the tensor-memory round trip of tcgen05 (which for a
-// handful of tokens took 70 to 110 ns per 128 x 16 x 16 instruction); at up to 16 tokens the math is a
+// handful of tokens took 70 to 110 ns per 128 x 16 x 16 instruction); the math is a
 // few tenths of a microsecond a phase either way.  A piece is two groups of eight weight rows (the
 // two halves of a rotated head, gate and up rows of the same outputs, or neighbours) by 64 or 128
 // columns, so that both values an epilogue combines end up in one tile of 16 rows.  Sums over a tile's
@@ -42,7 +42,7 @@ constexpr int WARPS = 16;
 constexpr int THREADS = 32 * WARPS;
 constexpr int PACE = 3;                  // pieces a paced warp asks for ahead of a product
 constexpr int GRANULE = 16;              // keys a warp takes at a time
-constexpr int MAX_TOKENS = 16;
+constexpr int MAX_TOKENS = 8;             // the columns of a product (with two groups of them, 9 to 16 tokens, 0.5B sizes lost 3 % against layer by layer, 1.5B sizes 17 %)
 constexpr int MAX_TILES = 64;             // of 16 rows a CTA and phase
 constexpr uint32_t BARRIER_LIMIT = 1u << 21;  // polls of the grid barrier, about a second
 enum { P_QKV = 0, P_OUT = 1, P_GATE = 2, P_DOWN = 3 };
@@ -64,7 +64,7 @@ static_assert(sizeof(StackLayer) % 64 == 0, "tensor maps need 64-byte alignment"
 
 struct PhasePlan {
   int tiles, slices;  // tiles of 16 rows, slices of `chunks` * 64 columns
-  int kg, rg;         // 0: tiles dealt whole over the CTAs, rg neighbours at a time; else CTAs as kg ranges of slices x rg ranges of tiles
+  int kg, rg;         // 0: tiles dealt whole over the CTAs; else CTAs as kg ranges of slices x rg ranges of tiles
 };
 
 struct StackArgs {
@@ -192,9 +192,9 @@ __device__ __forceinline__ void next_phase(Loader& ld, const Small& sm, int warp
 // A register that only some paths write counts as held from the start of the loop over layers to its end; that is why what a
 // load may leave out is set to zero first.  (Loads that go to a clamped place instead all hit one line: 7,500 cycles for an
 // operand of one token.)
-template <int NT, int HD>
+template <int HD>
 __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_constant__ StackArgs a) {
-  constexpr int TP = 8 * NT, C32 = HD / 32;
+  constexpr int TP = MAX_TOKENS, C32 = HD / 32;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t piece_bytes = 2048u * a.chunks;
   unsigned char* ring = smem_raw;
@@ -230,9 +230,9 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
     s.tile0 = s.tile_step = s.tiles = s.slice0 = s.slices = 0;
     if (p.kg == 0) {
       const int c = tid == P_GATE ? ctas - 1 - cta : cta;  // the CTAs with a tile more differ between the phases
-      s.tile0 = c * p.rg;
-      s.tile_step = p.rg > 1 ? 1 : ctas;
-      s.tiles = p.rg > 1 ? (c * p.rg < p.tiles ? p.rg : 0) : c < p.tiles ? (p.tiles - 1 - c) / ctas + 1 : 0;
+      s.tile0 = c;
+      s.tile_step = ctas;
+      s.tiles = c < p.tiles ? (p.tiles - 1 - c) / ctas + 1 : 0;
       s.slices = p.slices;
     } else if (cta < p.kg * p.rg) {
       const int k = cta % p.kg, g = cta / p.kg;
@@ -486,16 +486,10 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
     if (empty == a.slots) refill(a.slots);
     const int slices = s.slices;
     int tile = part.tile, slice = part.slice;
-    float c[NT][2][4];
+    float c[2][4];
 #pragma unroll
-    for (int n = 0; n < NT; ++n)
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) c[n][h][i] = 0.f;
-    uint32_t x_lane[NT];
-#pragma unroll
-    for (int n = 0; n < NT; ++n) x_lane[n] = smem_u32(work) + min(8 * n + (lane & 7), T - 1) * a.x_stride + (lane >> 3) * 16;  // rows past the last: a sum that nobody reads
+    for (int i = 0; i < 4; ++i) c[0][i] = c[1][i] = 0.f;
+    const uint32_t x_lane = smem_u32(work) + min(lane & 7, T - 1) * a.x_stride + (lane >> 3) * 16;  // rows past the last: a sum that nobody reads
     const uint32_t w_half = ((lane >> 3) & 1) * 1024 + (lane & 7) * 128, w_k = lane >> 4, w_x = lane & 7;
 #pragma unroll 1
     for (int left = part.end - part.first - 1; left >= 0; --left) {
@@ -503,18 +497,13 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
       uint32_t w_at = my_ring + (uint32_t)slot * piece_bytes + w_half, x_at = slice * a.chunks * 128;
 #pragma unroll 1
       for (int ch = 0; ch < a.chunks; ++ch, w_at += 2048, x_at += 128) {
-        uint32_t b[NT][2][4], w[4][4];
-#pragma unroll
-        for (int n = 0; n < NT; ++n) {
-          ldsm4(b[n][0], x_lane[n] + x_at);
-          ldsm4(b[n][1], x_lane[n] + x_at + 64);
-        }
+        uint32_t b[2][4], w[4][4];
+        ldsm4(b[0], x_lane + x_at);
+        ldsm4(b[1], x_lane + x_at + 64);
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) ldsm4(w[ks], w_at + ((((uint32_t)ks * 2 + w_k) ^ w_x) << 4));
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-          for (int n = 0; n < NT; ++n) mma16816(c[n][ks & 1], w[ks][0], w[ks][1], w[ks][2], w[ks][3], b[n][ks >> 1][(ks & 1) * 2], b[n][ks >> 1][(ks & 1) * 2 + 1]);
+        for (int ks = 0; ks < 4; ++ks) mma16816(c[ks & 1], w[ks][0], w[ks][1], w[ks][2], w[ks][3], b[ks >> 1][(ks & 1) * 2], b[ks >> 1][(ks & 1) * 2 + 1]);
       }
       __syncwarp();
       ++taken;
@@ -526,15 +515,10 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
       if (left > a.slots - empty) refill(a.slots);  // this phase has pieces that nobody asked for yet; else behind the barrier
       if (++slice == slices || left == 0) {
         float* dst = sums + ((warp + tile) * 16 + r) * TP + 2 * j;
+        *reinterpret_cast<float2*>(dst) = make_float2(c[0][0] + c[1][0], c[0][1] + c[1][1]);
+        *reinterpret_cast<float2*>(dst + 8 * TP) = make_float2(c[0][2] + c[1][2], c[0][3] + c[1][3]);
 #pragma unroll
-        for (int n = 0; n < NT; ++n) {
-          *reinterpret_cast<float2*>(dst + 8 * n) = make_float2(c[n][0][0] + c[n][1][0], c[n][0][1] + c[n][1][1]);
-          *reinterpret_cast<float2*>(dst + 8 * TP + 8 * n) = make_float2(c[n][0][2] + c[n][1][2], c[n][0][3] + c[n][1][3]);
-#pragma unroll
-          for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) c[n][h][i] = 0.f;
-        }
+        for (int i = 0; i < 4; ++i) c[0][i] = c[1][i] = 0.f;
         slice = 0;
         ++tile;
       }
@@ -954,10 +938,8 @@ bool make_piece_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t 
 }
 
 typedef void (*StackKernel)(const StackArgs);
-StackKernel kernel_of(int tokens, int head_dim) {
-  if (head_dim == 64) return tokens <= 8 ? (StackKernel)decode_stack_kernel<1, 64> : (StackKernel)decode_stack_kernel<2, 64>;
-  if (head_dim == 128) return tokens <= 8 ? (StackKernel)decode_stack_kernel<1, 128> : (StackKernel)decode_stack_kernel<2, 128>;
-  return nullptr;
+StackKernel kernel_of(int head_dim) {
+  return head_dim == 64 ? (StackKernel)decode_stack_kernel<64> : head_dim == 128 ? (StackKernel)decode_stack_kernel<128> : nullptr;
 }
 
 // Ranges of slices and tiles over the CTAs for a projection whose parts are added into the stream: the fewest bytes for the
@@ -979,11 +961,11 @@ void split_plan(PhasePlan* p, int ctas, int chunks, int tokens, int operand, int
 
 // Everything of the launch that goes by the sizes: the shares, shared memory, the ring.  0: the kernel does not take them.
 size_t plan_stack(StackArgs* a, int head_dim, int ctas) {
-  const int T = a->tokens, H = a->hidden, q_dim = a->heads * head_dim, F = a->inter, tp = T <= 8 ? 8 : 16;
+  const int T = a->tokens, H = a->hidden, q_dim = a->heads * head_dim, F = a->inter;
   a->chunks = (H / 64) % 2 || (q_dim / 64) % 2 || (F / 64) % 2 ? 1 : 2;
   const int cols = a->chunks * 64;
-  a->plan[P_QKV] = {(q_dim + 2 * a->kv_heads * head_dim) / 16, H / cols, 0, 1};
-  a->plan[P_GATE] = {F / 8, H / cols, 0, 1};
+  a->plan[P_QKV] = {(q_dim + 2 * a->kv_heads * head_dim) / 16, H / cols, 0, 0};
+  a->plan[P_GATE] = {F / 8, H / cols, 0, 0};
   a->plan[P_OUT] = {H / 16, q_dim / cols, 0, 0};
   a->plan[P_DOWN] = {H / 16, F / cols, 0, 0};
   const int x_limit = H > 512 ? H : 512;  // columns of an operand row
@@ -993,7 +975,7 @@ size_t plan_stack(StackArgs* a, int head_dim, int ctas) {
   int most = 0, wide = H;
   for (int p = 0; p < 4; ++p) {
     const PhasePlan& s = a->plan[p];
-    const int tiles = s.kg ? (s.tiles + s.rg - 1) / s.rg : s.rg > 1 ? s.rg : (s.tiles + ctas - 1) / ctas;
+    const int tiles = s.kg ? (s.tiles + s.rg - 1) / s.rg : (s.tiles + ctas - 1) / ctas;
     most = tiles > most ? tiles : most;
     if (s.kg) {
       const int w = (s.slices + s.kg - 1) / s.kg * cols;
@@ -1004,8 +986,8 @@ size_t plan_stack(StackArgs* a, int head_dim, int ctas) {
   a->act_stride = ((a->plan[P_GATE].tiles + ctas - 1) / ctas * T * 8 + 63) / 64 * 64;
   a->x_stride = 2 * wide + 16;
   a->x_bytes = T * a->x_stride;
-  a->qkv_tiles = a->plan[P_QKV].rg > 1 ? a->plan[P_QKV].rg : (a->plan[P_QKV].tiles + ctas - 1) / ctas;
-  const int sums = (most + WARPS) * 16 * tp * 4, merge = WARPS / 2 * 8 * (head_dim + 1) * 4;
+  a->qkv_tiles = (a->plan[P_QKV].tiles + ctas - 1) / ctas;
+  const int sums = (most + WARPS) * 16 * MAX_TOKENS * 4, merge = WARPS / 2 * 8 * (head_dim + 1) * 4;
   a->work_bytes = a->x_bytes + sums > merge ? a->x_bytes + sums : merge;
   a->work_bytes = (a->work_bytes + 15) / 16 * 16;
   const size_t rest = (size_t)a->work_bytes + (size_t)T * head_dim * 4 + (size_t)H * 4 + 64 * (size_t)a->qkv_tiles + sizeof(Small) + 64;
@@ -1046,7 +1028,7 @@ ALOFA_API int alofa_decode_stack_plan(int tokens, int hidden, int heads, int kv_
 // How many CTAs run a step of these sizes: one per SM, all resident together; 0 where the kernel does not take them.
 ALOFA_API int alofa_decode_stack_ctas(int tokens, int hidden, int heads, int kv_heads, int head_dim, int inter, int page) {
   if (tokens < 1 || tokens > MAX_TOKENS || hidden % 64 || inter % 64 || inter < 64 || kv_heads < 1 || heads % kv_heads || heads / kv_heads > 8 || page % GRANULE || page < GRANULE) return 0;
-  StackKernel kernel = kernel_of(tokens, head_dim);
+  StackKernel kernel = kernel_of(head_dim);
   if (!kernel || (heads * head_dim) % 64) return 0;
   int device, sms, coop;
   if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
@@ -1096,7 +1078,7 @@ ALOFA_API int alofa_decode_stack(const void* layers, int n_layers, int ctas, int
                                  int table_stride, float scale, float* base, long long* acc, const int* positions, const int* block_table,
                                  const int* slot_map, const float* rope, void* q, float* part_o, float* part_ml, void* act, unsigned* barrier, int* status,
                                  cudaStream_t stream) {
-  StackKernel kernel = kernel_of(tokens, head_dim);
+  StackKernel kernel = kernel_of(head_dim);
   if (!kernel || tokens < 1 || tokens > MAX_TOKENS) return ALOFA_ERR_ARGUMENT;
   StackArgs a = {};
   a.layers = (const StackLayer*)layers;

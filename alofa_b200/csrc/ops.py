@@ -1534,7 +1534,7 @@ def lru_scan(out, a, b, y, y_off: int, act: str, state, q_start, state_slots, n_
                                       _stream()), "lru_scan")
 
 
-DECODE_STACK_TOKENS = 16  # the most tokens that the one-kernel decode step takes
+DECODE_STACK_TOKENS = 8  # the most tokens that the one-kernel decode step takes
 
 
 def decode_stack_ctas(tokens: int, hidden: int, heads: int, kv_heads: int, head_dim: int, inter: int, page: int) -> int:

@@ -1,6 +1,6 @@
 """All layers of a small decode step as one persistent kernel.
 
-A decode step of up to 16 requests (one token each) through a stack of
+A decode step of up to eight requests (one token each) through a stack of
 pre-norm layers - grouped-query attention over pages, rotation of whole heads,
 a silu-gated feed-forward - runs in ``ops.decode_stack``: one CTA per SM works
 through all layers, weights streaming ahead of the phases that wait for one
@@ -24,11 +24,10 @@ from .position import RotaryNeox
 
 
 class DecodeStack:
-    # Steps this kernel is the faster way for: up to eight tokens (one group of token columns; at nine, two groups, it loses 3 % at 0.5B
-    # sizes) and as many of their numbers as every SM can read before each product.  us a pass of four steps, here and layer by
-    # layer: hidden 896, 3 tokens 2,535 and 2,748, 9 tokens 3,058 and 2,981; hidden 1,536, 4 tokens 4,855 and 5,207, 8 tokens 5,387
-    # and 5,414; hidden 3,584, 1 token 11,118 and 12,682, 4 tokens 11,886 and 12,890, 6 tokens 13,015 and 12,974.
-    MOST_TOKENS, MOST_NUMBERS = 8, 16384
+    # Steps this kernel is the faster way for: as many numbers of the stream as every SM can read before each product.  us a pass of four
+    # steps, layer by layer and here: hidden 896, 3 tokens 2,748 and 2,535; hidden 1,536, 1 token 4,955 and 4,602, 4 tokens 5,207 and
+    # 4,855, 8 tokens 5,414 and 5,387; hidden 3,584, 1 token 12,682 and 11,118, 4 tokens 12,890 and 11,836, 6 tokens 12,974 and 13,015.
+    MOST_NUMBERS = 16384
 
     def __init__(self, model, caches: dict, block_size: int):
         self.model = model
@@ -37,15 +36,18 @@ class DecodeStack:
         self.sizes = (block.mixer_norm.size, mixer.nh, mixer.nkv, mixer.hd, block.feed_forward.inter)
         self.page = block_size
         self.scale = mixer.scale
-        self.most, self.most_numbers = self.MOST_TOKENS, self.MOST_NUMBERS
         self.group = caches[model.run[0][1]].group
-        self.ctas = [0] + [ops.decode_stack_ctas(n, *self.sizes, block_size) for n in range(1, ops.DECODE_STACK_TOKENS + 1)]
+        self.caches = caches
+        self.ctas = None  # by tokens, 0 where the kernel does not take a step; worked out at the first step it may be for
+        self.described = None  # the tensors whose addresses the table holds
+
+    def _open(self) -> None:
+        """Asks the kernel what it takes and makes its scratch (a runner that never decodes a few tokens loads no library for it)."""
+        block, device = self.model.layers[self.model.run[0][0]], self.model.rt.device
+        mixer = block.mixer
+        self.ctas = [0] + [ops.decode_stack_ctas(n, *self.sizes, self.page) for n in range(1, ops.DECODE_STACK_TOKENS + 1)]
         if not any(self.ctas):
             return
-        device = model.rt.device
-        self.caches = caches
-        self.described = None  # the tensors whose addresses the table holds
-        self._describe()
         # the kernel's own scratch: rotated queries, the key splits' outputs, the activation; and its barrier word
         most = max(n for n, c in enumerate(self.ctas) if c)
         ctas = max(self.ctas)
@@ -108,11 +110,15 @@ class DecodeStack:
         the model's layers or sizes are not ones the kernel takes."""
         if model.rt.device.type != "cuda" or not cls.fits(model, caches):
             return None
-        stack = cls(model, caches, block_size)
-        return stack if any(stack.ctas) else None
+        return cls(model, caches, block_size)
 
     def takes(self, ctx, h) -> bool:
-        return ctx.decode_only and ctx.n_tokens <= self.most and ctx.n_tokens * self.sizes[0] <= self.most_numbers and self.ctas[ctx.n_tokens] > 0 and ctx.stream_of(h) is not None
+        n = ctx.n_tokens
+        if not ctx.decode_only or n > ops.DECODE_STACK_TOKENS or n * self.sizes[0] > self.MOST_NUMBERS or ctx.stream_of(h) is None:
+            return False
+        if self.ctas is None:
+            self._open()
+        return self.ctas[n] > 0
 
     def forward(self, ctx, h) -> None:
         """The step's rows through all layers: what they add to ``h`` is left
@@ -126,4 +132,5 @@ class DecodeStack:
 
     def reset(self) -> None:
         """After a kernel gave up: its barrier may stand half way."""
-        self.barrier.zero_()
+        if self.ctas is not None and any(self.ctas):
+            self.barrier.zero_()

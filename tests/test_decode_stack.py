@@ -1,5 +1,5 @@
 """How the one-kernel decode step divides a layer's products: every weight row and column by exactly one warp, within the
-matrices and within shared memory, over shapes with odd and even chunk counts, groups of one to eight and one to sixteen
+matrices and within shared memory, over shapes with odd and even chunk counts, groups of one to eight and one to eight
 tokens."""
 import ctypes
 
@@ -24,8 +24,7 @@ def share(phase, tiles, slices, kg, rg, cta, ctas):
     """(tiles, slices) of a CTA, as the kernel deals them."""
     if kg == 0:
         c = ctas - 1 - cta if phase == 2 else cta
-        own = [t for t in range(c * rg, (c + 1) * rg) if t < tiles] if rg > 1 else list(range(c, tiles, ctas))
-        return own, list(range(slices))
+        return list(range(c, tiles, ctas)), list(range(slices))
     if cta >= kg * rg:
         return [], []
     k, g = cta % kg, cta // kg
@@ -33,13 +32,13 @@ def share(phase, tiles, slices, kg, rg, cta, ctas):
 
 
 @pytest.mark.parametrize("name", list(SHAPES))
-@pytest.mark.parametrize("tokens", [1, 4, 8, 9, 16])
+@pytest.mark.parametrize("tokens", [1, 3, 4, 7, 8])
 @pytest.mark.parametrize("ctas", [148, 132])
 def test_products_are_covered_once(name, tokens, ctas):
     hidden, heads, kv_heads, hd, inter = SHAPES[name]
     taken, p = plan(tokens, SHAPES[name], ctas)
     if not taken:
-        assert name in ("7b", "1.5b") and tokens > 8, "only wide operands of many tokens leave no room"
+        assert name == "7b" and tokens > 4, "only wide operands of many tokens leave no room"
         return
     chunks, slots, x_stride, x_bytes, work_bytes, smem = p[16:22]
     assert slots >= 2 and smem <= LIMIT and x_bytes >= tokens * x_stride
@@ -62,7 +61,7 @@ def test_products_are_covered_once(name, tokens, ctas):
                     entry = w + u // len(part)
                     if (w, u // len(part)) not in entries:
                         entries.append((w, u // len(part)))
-                    assert (entry + 1) * 16 * (8 if tokens <= 8 else 16) * 4 + x_bytes <= work_bytes
+                    assert (entry + 1) * 16 * 8 * 4 + x_bytes <= work_bytes
             assert len({w + t for w, t in entries}) == len(entries)
             assert not seen & set(pieces)
             seen |= set(pieces)
