@@ -251,6 +251,9 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
   if (tid < (int)(sizeof(LayerVectors) / 4)) reinterpret_cast<int*>(&sm.layer[0])[tid] = reinterpret_cast<const int*>(&a.layers[0].vectors)[tid];
   if (cta == ctas - 1)  // the table into L2
     for (int i = tid * 128; i < a.n_layers * (int)sizeof(StackLayer); i += THREADS * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(a.layers) + i));
+  // The maps lie in global memory that the host wrote: without this an SM may use what it kept of another table that lay at the same
+  // address.  A map by a thread, dealt over the warps; the __syncthreads() below hands that on to the lanes that ask for copies.
+  for (int i = warp + WARPS * lane; i < a.n_layers * 4; i += THREADS) asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(&a.layers[i >> 2].maps[i & 3]) : "memory");
   if (tid == 0) sm.abort_flag = 0;
   if (tid < WARPS * a.slots) mbar_init(bars + tid, 1);
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");

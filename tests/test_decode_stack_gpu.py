@@ -110,3 +110,27 @@ def test_model_loaded_again(folders):
     want = runner.forward([StepEntry(runner.admit(3), [7], [0])]).clone()
     assert (first - want).norm() > 0.01 * want.norm()
     assert (changed - want).norm() <= 2**-8 * want.norm()
+
+
+def test_table_at_an_address_used_before(folders):
+    """A table of layers that takes the place of a dropped one in memory describes other weights: none of the old one's maps is used."""
+    from alofa_b200.engine.loading import load_model
+    from alofa_b200.engine.step import StepEntry, StepRunner
+
+    models, places, reused = [], [], False
+    for i in range(6):
+        model, _, _ = load_model(folders["h64_even"], "bfloat16")  # earlier models stay: these weights lie elsewhere
+        for block in model.layers:
+            block.mixer.out.weight.mul_(1 + i)
+        models.append(model)
+        runner = StepRunner(model, block_size=64, num_pages=4, max_requests=1, max_tokens=128, max_step_tokens=64, cuda_graphs=False)
+        got = runner.forward([StepEntry(runner.admit(1), [7], [0])]).clone()
+        runner.check_status()
+        runner.release(0)
+        reused = reused or runner.decode_stack.table.data_ptr() in places
+        places.append(runner.decode_stack.table.data_ptr())
+        runner.decode_stack = None
+        want = runner.forward([StepEntry(runner.admit(2), [7], [0])]).clone()
+        assert (got - want).norm() <= 2**-8 * want.norm()
+        del runner
+    assert reused, "no table lay where another had been"
