@@ -138,37 +138,53 @@ def _depth_parts(tokens: int, features: int, depth: int, undivided: int, sms: in
 
 
 def plan(linear):
-    from .linear import Partial
-
+    """The tensor-core product of ``linear``'s weight, or None."""
     w = linear.weight
-    depth = linear.in_features
-    if depth % 8 or w.data_ptr() % 16:
+    if linear.in_features % 8 or w.data_ptr() % 16:
         return None
     _sms_of_device(w.device)
-    gated = linear.epi == ops.EPI_GATED
-    n_acc = 2 if gated else 1
+    return TensorCoreProduct(linear)
 
-    def run(out, x, defer: bool = False, buf=None, acc=None):
-        from .linear import ACCUMULATED
 
+class TensorCoreProduct:
+    """What :func:`plan` returns.  It holds the weight and the numbers it goes
+    by, not the :class:`~alofa_b200.parts.linear.Linear` that holds it: a
+    dropped layer gives its weight back at once, not when the cycle collector
+    next runs."""
+
+    __slots__ = ("weight", "bias", "epi", "act", "gate", "depth", "out_features")
+
+    def __init__(self, linear):
+        self.weight, self.bias, self.epi, self.act, self.gate = linear.weight, linear.bias, linear.epi, linear.act, linear.gate
+        self.depth, self.out_features = linear.in_features, linear.out_features
+
+    def weights_on_m(self, tokens: int) -> bool:
+        return _tile(tokens, self.out_features, self.epi == ops.EPI_GATED) > 0
+
+    def __call__(self, out, x, defer: bool = False, buf=None, acc=None):
+        from .linear import ACCUMULATED, Partial
+
+        w, depth, features = self.weight, self.depth, self.out_features
+        gated = self.epi == ops.EPI_GATED
+        n_acc = 2 if gated else 1
         tokens = x.shape[0]
         if tokens == 0:
             return True
-        bn = _tile(tokens, linear.out_features, gated)
+        bn = _tile(tokens, features, gated)
         lazy = None if isinstance(x, torch.Tensor) else x
         if lazy is not None:
             x = None
-        deferrable = defer and n_acc == 1 and not linear.act
-        pair = _pair_splits(tokens, linear.out_features, depth, gated, deferrable) if bn < 0 else 0
+        deferrable = defer and n_acc == 1 and not self.act
+        pair = _pair_splits(tokens, features, depth, gated, deferrable) if bn < 0 else 0
         bn = -PAIR_ROWS if pair else bn
-        splits = ops.gemm_tc_splits(depth, pair or _splits(_ctas(tokens, linear.out_features, bn, gated), depth, deferrable))
+        splits = ops.gemm_tc_splits(depth, pair or _splits(_ctas(tokens, features, bn, gated), depth, deferrable))
         computed = None
         if lazy is not None:
             # Rows still to be made.  The weights-on-M kernel makes them as it loads, a k-slice at a
             # time and each a trip to L2: worth it while a CTA has a few slices, else they are made first.
             per_cta = -(-(-(-depth // K_SLICE)) // splits)
             kind = getattr(lazy, "kind", "merged")
-            if kind == "merged" and bn == 16 and linear.epi == ops.EPI_RESIDUAL and per_cta <= 2 and lazy.fits_kernel():
+            if kind == "merged" and bn == 16 and self.epi == ops.EPI_RESIDUAL and per_cta <= 2 and lazy.fits_kernel():
                 computed = lazy.computed()
             elif kind == "normed" and bn == 16 and gated and splits <= 8 and per_cta <= 6 and lazy.fits_kernel():
                 computed = lazy.computed()  # the norm folded into a gated product whose splits are one cluster
@@ -179,14 +195,14 @@ def plan(linear):
         normed = computed is not None and computed[0] == ops.B_NORMED
         partial = None
         if splits > 1 and acc is None and not normed:
-            shape = (splits * n_acc, tokens, linear.out_features)
+            shape = (splits * n_acc, tokens, features)
             partial = buf(shape, torch.float32) if buf is not None else torch.empty(shape, dtype=torch.float32, device=w.device)
-        deferred = defer and splits > 1 and n_acc == 1 and acc is None and not linear.act  # whoever adds deferred sums up applies no activation
+        deferred = defer and splits > 1 and n_acc == 1 and acc is None and not self.act  # whoever adds deferred sums up applies no activation
         dst = partial[0] if deferred else out  # a deferred product writes partial sums only
-        if not ops.gemm_tc(dst, x, w, linear.bias, linear.epi, bn, splits, partial, reduce=not deferred, computed=computed, acc=acc, act=linear.act, gate=linear.gate, pair=pair > 0):
+        if not ops.gemm_tc(dst, x, w, self.bias, self.epi, bn, splits, partial, reduce=not deferred, computed=computed, acc=acc, act=self.act, gate=self.gate, pair=pair > 0):
             if normed:
                 lazy.undo()
-                return run(out, lazy.rows(), defer, buf)
+                return self(out, lazy.rows(), defer, buf)
             if computed is not None or acc is not None:
                 raise AlofaError("state", "the tensor-core product refused an operand it had accepted")
             return False
@@ -194,7 +210,4 @@ def plan(linear):
             lazy.done(computed)
         if acc is not None:
             return ACCUMULATED
-        return Partial(partial, splits, linear.bias) if deferred else True
-
-    run.weights_on_m = lambda tokens: _tile(tokens, linear.out_features, gated) > 0
-    return run
+        return Partial(partial, splits, self.bias) if deferred else True
