@@ -24,9 +24,12 @@
 // two halves of a rotated head, gate and up rows of the same outputs, or neighbours) by 64 or 128
 // columns, so that both values an epilogue combines end up in one tile of 16 rows.  Sums over a tile's
 // pieces go through shared memory in the order of the pieces.
-// The stream is an fp32 base (the embedding) plus the 64-bit fixed-point accumulator of common.cuh, into
-// which phases 3 and 5 add with integer atomics: the result does not depend on their order.  The
-// norm's factor 1 / sqrt(mean square + eps) is applied to a product's sums, its weight to the operand.
+// The stream is kept as layer by layer: an fp32 base plus the 64-bit fixed-point accumulator of common.cuh, into
+// which phases 3 and 5 add with integer atomics, so that the result does not depend on their order.  Phases 1 and 4
+// read base + accumulator; behind them, while the barrier is waited for, the sum becomes the other base, and once all
+// have read it the accumulator is cleared.  Only what one sublayer adds is ever in fixed point: infinities, NaN and
+// numbers of any size in an embedding reach the logits.  The norm's factor 1 / sqrt(mean square + eps) is applied to
+// a product's sums, its weight to the operand.
 // (src/alofa/kernels/cpu/scalar.mojo:93-231, 283-470 for the formulas; src/alofa/model/arch/qwen.mojo:1367-1510
 // for the order of a layer.)
 //
@@ -80,8 +83,10 @@ struct StackArgs {
   float scale;               // of the scores, times log2(e)
   float per_group, per_cta;  // 1 / group, 1 / CTAs: quotients of small numbers by a product
   PhasePlan plan[4];
-  float* base;               // [tokens, hidden]: the stream; zero afterwards
-  long long* acc;            // [tokens, hidden]: the stream with what the layers added to it
+  float* base;               // [tokens, hidden]: the stream, before phase 1 (and at the end) without what `acc` holds
+  float* base_ff;            // the same before phase 4, without what `acc_ff` holds
+  long long* acc;            // [tokens, hidden]: what the last feed-forward added; zero before, as is acc_ff
+  long long* acc_ff;         // what the attention added; zero afterwards
   const int* positions;
   const int* block_table;    // [tokens, table_stride]
   const int* slot_map;       // [tokens]
@@ -433,30 +438,39 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
     asked = true;
   };
 
-  // The rows of the stream times the norm's weight as bfloat16 into shared memory, and each row's factor.  The stream is
-  // `base` in the first norm of a step and the accumulator from then on (phase 1 of the first layer moves it there).
-  auto normed_rows = [&](float eps, bool from_base) {
+  // The stream with what a sublayer added, for the next norm: between the arrival at a barrier and its end, by all warps but the one
+  // that waits there.
+  auto settle = [&](float* to, const float* base, const long long* acc, bool added) {
+#pragma unroll 1
+    for (int i = ((warp - 1) * ctas + cta) * 32 + lane; warp > 0 && i < T * H; i += (WARPS - 1) * ctas * 32) to[i] = stream_add(__ldcg(base + i), added ? __ldcg(acc + i) : 0);
+  };
+  auto clear = [&](long long* acc) {  // the numbers that this thread settled, once all have read them
+#pragma unroll 1
+    for (int i = ((warp - 1) * ctas + cta) * 32 + lane; warp > 0 && i < T * H; i += (WARPS - 1) * ctas * 32) acc[i] = 0;
+  };
+
+  // The rows of the stream times the norm's weight as bfloat16 into shared memory, and each row's factor.  (`added`: before the first
+  // norm of a step nothing was.)
+  auto normed_rows = [&](float eps, const float* base, const long long* acc, bool added) {
     const int per_row = WARPS >> t_bits, t = warp >> (4 - t_bits), part = warp & (per_row - 1);
     float square = 0.f;
     if (t < T) {
-      const float2* b2 = reinterpret_cast<const float2*>(a.base + (size_t)t * H);
-      const longlong2* a2 = reinterpret_cast<const longlong2*>(a.acc + (size_t)t * H);
+      const float2* b2 = reinterpret_cast<const float2*>(base + (size_t)t * H);
+      const longlong2* a2 = reinterpret_cast<const longlong2*>(acc + (size_t)t * H);
       const float2* g2 = reinterpret_cast<const float2*>(gamma_s);
       unsigned char* row = work + (size_t)t * a.x_stride;
       const int n2 = H / 2, step = 32 * per_row;
 #pragma unroll 1
       for (int w0 = part * 32; w0 < n2; w0 += 8 * step) {  // H is a multiple of 64: whole warps have an element or none
         longlong2 q[8];
+        float2 b[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
           q[u] = make_longlong2(0, 0);
+          b[u] = make_float2(0.f, 0.f);
           if (w0 + u * step < n2) {
-            if (from_base) {
-              const float2 b = __ldcg(b2 + w0 + u * step + lane);
-              q[u] = make_longlong2(__float_as_int(b.x), __float_as_int(b.y));
-            } else {
-              q[u] = __ldcg(a2 + w0 + u * step + lane);
-            }
+            b[u] = __ldcg(b2 + w0 + u * step + lane);
+            if (added) q[u] = __ldcg(a2 + w0 + u * step + lane);
           }
         }
         ahead();
@@ -464,7 +478,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
         for (int u = 0; u < 8; ++u) {
           if (w0 + u * step >= n2) break;
           const int i = w0 + u * step + lane;
-          const float x = from_base ? __int_as_float((int)q[u].x) : stream_add(0.f, q[u].x), y = from_base ? __int_as_float((int)q[u].y) : stream_add(0.f, q[u].y);
+          const float x = stream_add(b[u].x, q[u].x), y = stream_add(b[u].y, q[u].y);
           const float2 g = g2[i];
           square += x * x + y * y;
           *reinterpret_cast<uint32_t*>(row + 4 * i) = pack2(x * g.x, y * g.y);
@@ -546,8 +560,6 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
           for (int i = tid * 32; i < (a.heads + 2 * a.kv_heads) * HD; i += THREADS * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(next.qkv_bias + i));
       }
     }
-    if (layer == 0)
-      for (int i = cta * THREADS + tid; i < T * H; i += ctas * THREADS) a.acc[i] = __float2ll_rn(a.base[i] * STREAM_SCALE);
 #pragma unroll 1  // one copy of the product's loop, whose instructions then stay in the cache
     for (int phase = 0; phase < 4; ++phase) {
       place_thread();
@@ -556,7 +568,8 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
         asked = false;
         // the operand
         if (phase == P_QKV || phase == P_GATE) {
-          normed_rows(phase == P_QKV ? L.eps_mixer : L.eps_ff, layer == 0 && phase == P_QKV);
+          const bool mixer = phase == P_QKV;
+          normed_rows(mixer ? L.eps_mixer : L.eps_ff, mixer ? a.base : a.base_ff, mixer ? a.acc : a.acc_ff, !mixer || layer > 0);
         } else {
           const int per_row = WARPS >> t_bits, t = warp >> (4 - t_bits), first = (warp & (per_row - 1)) * 32 + lane, step = 32 * per_row;
           const int cols = s.slices * a.chunks * 64, col0 = s.slice0 * a.chunks * 64;
@@ -662,7 +675,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
               if (rows == 3) y += from[8 * TP];
             }
             if (rows == 4)  // into the stream
-              atomicAdd(reinterpret_cast<unsigned long long*>(a.acc) + (size_t)t * H + at * 16 + e, (unsigned long long)__float2ll_rn(x * STREAM_SCALE));
+              atomicAdd(reinterpret_cast<unsigned long long*>(phase == P_OUT ? a.acc_ff : a.acc) + (size_t)t * H + at * 16 + e, (unsigned long long)__float2ll_rn(x * STREAM_SCALE));
           }
           if (rows == 4) continue;
           bf16* dst = nullptr;
@@ -708,8 +721,10 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
       if (phase != P_QKV) {
         if (!a.paced) refill(a.slots);
         if (phase == P_OUT) stage(L.gamma_ff, nullptr);
+        if (phase == P_GATE) settle(a.base, a.base_ff, a.acc_ff, true);
         if (phase == P_DOWN) stage(N.gamma_mixer, N.qkv_bias);
         if (!wait()) goto leave;
+        if (phase == P_GATE) clear(a.acc_ff);
         continue;
       }
 
@@ -741,9 +756,9 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
           }
         }
         if (!a.paced) refill(a.slots);
+        settle(a.base_ff, a.base, a.acc, layer > 0);
         if (!wait()) goto leave;
-        if (layer == 0)  // the stream is in the accumulator now
-          for (int i = cta * THREADS + tid; i < T * H; i += ctas * THREADS) a.base[i] = 0.f;
+        if (layer > 0) clear(a.acc);
         if (it_token >= 0) {
           float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;  // of heads 2j and 2j + 1 of the group
           float o[HD / 16][4];
@@ -1078,7 +1093,7 @@ ALOFA_API int alofa_decode_stack_layer(void* entry, const void* qkv, const void*
 }
 
 ALOFA_API int alofa_decode_stack(const void* layers, int n_layers, int ctas, int tokens, int hidden, int heads, int kv_heads, int head_dim, int inter, int page,
-                                 int table_stride, float scale, float* base, long long* acc, const int* positions, const int* block_table,
+                                 int table_stride, float scale, float* base, float* base_ff, long long* acc, long long* acc_ff, const int* positions, const int* block_table,
                                  const int* slot_map, const float* rope, void* q, float* part_o, float* part_ml, void* act, unsigned* barrier, int* status,
                                  cudaStream_t stream) {
   StackKernel kernel = kernel_of(head_dim);
@@ -1096,7 +1111,9 @@ ALOFA_API int alofa_decode_stack(const void* layers, int n_layers, int ctas, int
   a.table_stride = table_stride;
   a.scale = scale * 1.4426950408889634f;
   a.base = base;
+  a.base_ff = base_ff;
   a.acc = acc;
+  a.acc_ff = acc_ff;
   a.positions = positions;
   a.block_table = block_table;
   a.slot_map = slot_map;

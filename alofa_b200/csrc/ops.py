@@ -95,7 +95,7 @@ def _decode_stack():
             "alofa_decode_stack_layer_bytes": [],
             "alofa_decode_stack_ctas": [_I, _I, _I, _I, _I, _I, _I],
             "alofa_decode_stack_layer": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _F, _F, _I, _I, _I, _I, _I],
-            "alofa_decode_stack": [_P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P],
+            "alofa_decode_stack": [_P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P],
         }
         for name, args in sigs.items():
             fn = getattr(lib, name)
@@ -1571,19 +1571,20 @@ def decode_stack_layer(qkv, out, gate_up, down, gamma_mixer, gamma_ff, qkv_bias,
     return entry.raw
 
 
-def decode_stack(table, n_layers: int, ctas: int, sizes: tuple, page: int, scale: float, base, acc, positions, block_table, slot_map, rope, q, part_o, part_ml, act, barrier, status) -> None:
+def decode_stack(table, n_layers: int, ctas: int, sizes: tuple, page: int, scale: float, base, alt, acc, other, positions, block_table, slot_map, rope, q, part_o, part_ml, act, barrier, status) -> None:
     """All layers of a decode step, one token per request: what they add to the
-    stream ``base`` goes into the accumulator ``acc`` (zero before).  ``table``:
-    the entries of :func:`decode_stack_layer` one after the other; ``sizes``:
+    stream ``base`` is in ``base`` and the accumulator ``acc`` afterwards.  ``alt``:
+    like ``base``, overwritten; ``acc`` and ``other``, like it, are zero before,
+    ``other`` afterwards too.  ``table``: the entries of :func:`decode_stack_layer` one after the other; ``sizes``:
     (hidden, heads, kv_heads, head_dim, inter); ``barrier``: a word that only
     this kernel writes, zero at first."""
     tokens, hidden = base.shape
     hd, kv = sizes[3], sizes[2]
-    if hidden != sizes[0] or tuple(acc.shape) != (tokens, hidden) or block_table.shape[0] != tokens or q.shape[0] < tokens or act.numel() < decode_stack_act_numbers(tokens, sizes[4], ctas) or part_o.shape[0] < ctas or tokens * kv > ctas:
+    if hidden != sizes[0] or any(tuple(t.shape) != (tokens, hidden) for t in (alt, acc, other)) or block_table.shape[0] != tokens or q.shape[0] < tokens or act.numel() < decode_stack_act_numbers(tokens, sizes[4], ctas) or part_o.shape[0] < ctas or tokens * kv > ctas:
         raise AlofaError("invalid_argument", "decode_stack sizes disagree", f"base={tuple(base.shape)} acc={tuple(acc.shape)} tables={tuple(block_table.shape)} ctas={ctas}")
     _done(
         _decode_stack().alofa_decode_stack(
-            _dev(table, "table"), n_layers, ctas, tokens, *sizes, page, block_table.shape[1], float(scale), _dev(base, "base", torch.float32), _dev(acc, "acc", torch.int64),
+            _dev(table, "table"), n_layers, ctas, tokens, *sizes, page, block_table.shape[1], float(scale), _dev(base, "base", torch.float32), _dev(alt, "alt", torch.float32), _dev(acc, "acc", torch.int64), _dev(other, "other", torch.int64),
             _dev(positions, "positions", torch.int32), _dev(block_table, "block_table", torch.int32), _dev(slot_map, "slot_map", torch.int32), _dev(rope, "rope", torch.float32),
             _dev(q, "q", torch.bfloat16), _dev(part_o, "part_o", torch.float32), _dev(part_ml, "part_ml", torch.float32), _dev(act, "act", torch.bfloat16), _dev(barrier, "barrier", torch.int32),
             _dev(status, "status", torch.int32), _stream(),

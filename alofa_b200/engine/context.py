@@ -164,6 +164,13 @@ class StepContext:
             return None
         return st["acc"][st["next"]]
 
+    def stream_buffers(self, h):
+        """(the stream's other buffer, the accumulator to leave owed, the other
+        one), for a kernel that reads and adds to a stream that lacks nothing
+        several times over."""
+        st = self.stream_of(h)
+        return st["alt"], st["acc"][st["next"]], st["acc"][1 - st["next"]]
+
     def owe_accumulator(self, h) -> None:
         """A product has added into ``accumulator_for(h)``."""
         st = self.stream_of(h)

@@ -121,12 +121,12 @@ class DecodeStack:
         return self.ctas[n] > 0
 
     def forward(self, ctx, h) -> None:
-        """The step's rows through all layers: what they add to ``h`` is left
-        in the stream's accumulator."""
+        """The step's rows through all layers: what the last product added to
+        ``h`` is left in the stream's accumulator."""
         self._describe()
-        acc = ctx.accumulator_for(h)
+        alt, acc, other = ctx.stream_buffers(h)
         group = ctx.groups[self.group]
-        ops.decode_stack(self.table, len(self.model.run), self.ctas[ctx.n_tokens], self.sizes, self.page, self.scale, h, acc, ctx.positions, group.block_table, group.slot_map, self.rope,
+        ops.decode_stack(self.table, len(self.model.run), self.ctas[ctx.n_tokens], self.sizes, self.page, self.scale, h, alt, acc, other, ctx.positions, group.block_table, group.slot_map, self.rope,
                          self.q, self.part_o, self.part_ml, self.act, self.barrier, ctx.status)
         ctx.owe_accumulator(h)
 

@@ -134,3 +134,33 @@ def test_table_at_an_address_used_before(folders):
         assert (got - want).norm() <= 2**-8 * want.norm()
         del runner
     assert reused, "no table lay where another had been"
+
+
+def test_infinities_nan_and_large_numbers_of_an_embedding_reach_the_logits(folders):
+    """The stream of a step as one kernel loses nothing that the same step layer by layer keeps."""
+    from alofa_b200.engine.loading import load_model
+    from alofa_b200.engine.step import StepEntry, StepRunner
+
+    model, _, _ = load_model(folders["h64_even"], "bfloat16")
+    with torch.no_grad():
+        rows = model.embedding.weight
+        rows[1, 3] = float("nan")
+        rows[2, 70] = float("inf")
+        rows[3] *= 2.0**40
+        rows[4, 5] = -(2.0**33)
+    tokens = [1, 2, 3, 4, 20]
+    out = []
+    for stacked in (True, False):
+        runner = StepRunner(model, block_size=64, num_pages=10, max_requests=5, max_tokens=128, max_step_tokens=64, cuda_graphs=False)
+        if not stacked:
+            runner.decode_stack = None
+        slots = [runner.admit(i) for i in range(5)]
+        for _ in range(2):
+            got = runner.forward([StepEntry(s, [t], [0]) for s, t in zip(slots, tokens)]).clone()
+        runner.check_status()
+        out.append(got[:, 10:])  # the head has the changed rows too
+    got, want = out
+    assert torch.equal(got.isnan(), want.isnan())
+    assert want[0].isnan().all() and not want[2:].isnan().any()
+    for i in (2, 3, 4):
+        assert (got[i] - want[i]).norm() <= 2**-7 * want[i].norm()
