@@ -123,6 +123,7 @@ class StepContext:
         # Small decode steps keep the stream as base + fixed-point accumulator (see open_stream)
         self.stream_acc = None  # int64 [2, rows, hidden], given by the step runner; both zero between steps
         self._stream = None
+        self.keep = []  # device memory that a recording of this step needs as long as it is replayed, beyond the runner's and the model's own
         self.decode_stack = None  # runs all layers of a small decode step as one kernel, where the model's are of that form (set by the step runner)
         # Several copies of the residual stream (blocks that keep them): fp32 [S, tokens, hidden], and the write a
         # sublayer left owed, (y, out weights, mix weights), which the next reader of the streams does

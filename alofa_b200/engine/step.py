@@ -55,6 +55,7 @@ class DecodeGraph:
     logits: Optional[torch.Tensor]
     tokens: Optional[torch.Tensor]
     kernels: int
+    keep: list  # what the recorded kernels read that may be replaced while the recording lives
 
 
 class StepRunner:
@@ -108,6 +109,7 @@ class StepRunner:
         self.decode_stack = DecodeStack.build(model, self.storage.caches, block_size) if self._stream_acc is not None else None
         self._layouts = {}
         self.cuda_graphs = cuda_graphs and on_gpu and model.graph_safe()
+        self._graphs_of = model.loads  # the loading that the recordings below are of: their kernels hold the weights' addresses
         self._graphs = {}  # decode steps by batch size; steps with prompt portions by (tokens, requests, wanted rows), and apart for those whose requests all start in them where a mixer tells them apart
         self.prompt_graphs = self.cuda_graphs and os.environ.get("ALOFA_PROMPT_GRAPHS", "1") != "0"
         self.max_prompt_graphs = 4
@@ -233,6 +235,11 @@ class StepRunner:
 
     def _run(self, ctx: StepContext, sample: bool):
         """(logits or None, tokens or None) for a prepared step."""
+        if self._graphs_of != self.model.loads:  # the model was loaded again
+            if self._graphs:
+                torch.cuda.synchronize()  # a replay may still run
+            self._graphs.clear()
+            self._graphs_of = self.model.loads
         if self.cuda_graphs and ctx.decode_only and ctx.n_out == ctx.n_seqs:
             ctx.max_context = self._context_bucket(ctx.max_kv_len)
             key = (ctx.n_seqs, ctx.max_context, "decode")
@@ -309,7 +316,7 @@ class StepRunner:
             tokens = self._sample(ctx, logits, True) if logits is not None else None  # a replay may meet rows of any temperature
         if self.arena.grown != grown or (logits is not None and logits.data_ptr() != first_logits.data_ptr()):
             raise AlofaError("state", "recording a step asked the arena for other memory than running it did")
-        self._graphs[key] = DecodeGraph(graph, logits, tokens, ops.launch_count() - before)
+        self._graphs[key] = DecodeGraph(graph, logits, tokens, ops.launch_count() - before, ctx.keep)
         return first_logits, first_tokens
 
     def forward(self, entries: Sequence[StepEntry]) -> Optional[torch.Tensor]:

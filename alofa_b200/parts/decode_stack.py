@@ -4,12 +4,13 @@ A decode step of up to eight requests (one token each) through a stack of
 pre-norm layers - grouped-query attention over pages, rotation of whole heads,
 a silu-gated feed-forward - runs in ``ops.decode_stack``: one CTA per SM works
 through all layers, weights streaming ahead of the phases that wait for one
-another.  :meth:`DecodeStack.build` says whether a model's layers are of that
+another.  :meth:`DecodeStack.build` says whether a model's layers may be of that
 form, :meth:`DecodeStack.takes` whether a step is; every other model and step
 goes layer by layer.  (The order of a layer:
 src/alofa/model/arch/qwen.mojo:1367-1510.)"""
 from __future__ import annotations
 
+from dataclasses import dataclass
 from typing import Optional
 
 import torch
@@ -19,8 +20,21 @@ from ..csrc import ops
 from .attention import GQAttention
 from .block import PrenormResidual
 from .feed_forward import GatedMLP
+from .linear import GATED, RESIDUAL, STORE
 from .norm import RMSNorm
 from .position import RotaryNeox
+
+
+@dataclass(frozen=True)
+class Form:
+    """All that the kernel's table and launch go by, as numbers: two equal
+    ones describe the same step.  Nothing of a model is kept alive by it."""
+
+    sizes: tuple  # hidden, heads, kv heads, head size, intermediate
+    scale: float
+    group: int
+    rope: int  # the rotary table's address
+    layers: tuple  # per run entry the addresses of its weights, vectors and caches, and the norms' eps
 
 
 class DecodeStack:
@@ -31,106 +45,111 @@ class DecodeStack:
 
     def __init__(self, model, caches: dict, block_size: int):
         self.model = model
-        block = model.layers[model.run[0][0]]
-        mixer = block.mixer
-        self.sizes = (block.mixer_norm.size, mixer.nh, mixer.nkv, mixer.hd, block.feed_forward.inter)
-        self.page = block_size
-        self.scale = mixer.scale
-        self.group = caches[model.run[0][1]].group
         self.caches = caches
-        self.ctas = None  # by tokens, 0 where the kernel does not take a step; worked out at the first step it may be for
-        self.described = None  # the tensors whose addresses the table holds
+        self.page = block_size
+        self.form = None  # what the table and the scratch below were made for
+        self.ctas = [0] * (ops.DECODE_STACK_TOKENS + 1)  # by tokens, 0 where the kernel does not take a step
 
-    def _open(self) -> None:
-        """Asks the kernel what it takes and makes its scratch (a runner that never decodes a few tokens loads no library for it)."""
-        block, device = self.model.layers[self.model.run[0][0]], self.model.rt.device
-        mixer = block.mixer
-        self.ctas = [0] + [ops.decode_stack_ctas(n, *self.sizes, self.page) for n in range(1, ops.DECODE_STACK_TOKENS + 1)]
-        if not any(self.ctas):
-            return
-        # the kernel's own scratch: rotated queries, the key splits' outputs, the activation; and its barrier word
-        most = max(n for n, c in enumerate(self.ctas) if c)
-        ctas = max(self.ctas)
-        self.q = torch.empty((most, mixer.q_dim), dtype=torch.bfloat16, device=device)
-        self.act = torch.empty(ops.decode_stack_act_numbers(most, block.feed_forward.inter, ctas), dtype=torch.bfloat16, device=device)
-        self.part_o = torch.empty((ctas, 8, mixer.hd), dtype=torch.float32, device=device)
-        self.part_ml = torch.empty((ctas, 8, 2), dtype=torch.float32, device=device)
-        self.barrier = torch.zeros(32, dtype=torch.int32, device=device)
-
-    def _tensors(self) -> list:
-        """Per run entry the tensors that the kernel reads and writes in place."""
-        out = []
-        for layer, cache in self.model.run:
-            block, kv = self.model.layers[layer], self.caches[cache]
-            out.append((block.mixer.qkv.weight, block.mixer.out.weight, block.feed_forward.gate_up.weight, block.feed_forward.down.weight, block.mixer_norm.weight, block.feed_forward_norm.weight,
-                        block.mixer.qkv.bias, kv.k, kv.v))
-        return out
-
-    def _describe(self) -> None:
-        """The kernel's table of layers, made again if the model was loaded again."""
-        now = self._tensors()
-        if self.described is not None and all(a is b for old, new in zip(self.described, now) for a, b in zip(old, new)):
-            return
-        blocks = [self.model.layers[layer] for layer, _ in self.model.run]
-        entries = [ops.decode_stack_layer(*tensors, block.mixer_norm.eps, block.feed_forward_norm.eps, *self.sizes) for tensors, block in zip(now, blocks)]
-        self.table = torch.frombuffer(bytearray(b"".join(entries)), dtype=torch.uint8).to(self.model.rt.device)
-        self.rope = blocks[0].mixer.position.rotary_table()[0]
-        self.described = now
-
-    @staticmethod
-    def fits(model, caches: dict) -> bool:
-        """Whether the model's layers are of the form the kernel has."""
+    def look(self) -> Optional[Form]:
+        """The model as it is loaded now, None where its layers are not of the
+        form the kernel has (or not loaded).  Looked at anew for every step
+        that is not a replay: a model may be loaded again."""
+        model, caches = self.model, self.caches
         if model.rt.dtype != torch.bfloat16 or model.stream_copies or model.keeps_embedding or model.shared_value_width:
-            return False
-        shapes = set()
+            return None
+        shapes, layers, bf16, fp32, cuda = set(), [], torch.bfloat16, torch.float32, model.rt.device.type == "cuda"
         for i, (layer, cache) in enumerate(model.run):
             block = model.layers[layer]
-            if type(block) is not PrenormResidual or type(block.mixer) is not GQAttention or type(block.feed_forward) is not GatedMLP:
-                return False
-            mixer, ff = block.mixer, block.feed_forward
-            if mixer.qkv is None or ff.gate_up is None:
-                return False  # not loaded yet
-            norms = (block.mixer_norm, block.feed_forward_norm)
-            if any(type(n) is not RMSNorm or n.spec.kind != "rmsnorm" or n.shift is not None for n in norms) or type(mixer.position) is not RotaryNeox:
-                return False
-            if cache != i or not isinstance(caches.get(cache), LayerCache) or mixer.window or mixer.out.bias is not None or ff.down.bias is not None or ff.gate_up.bias is not None:
-                return False
+            if type(block) is not PrenormResidual or type(block.mixer) is not GQAttention or type(block.feed_forward) is not GatedMLP or type(block.mixer.position) is not RotaryNeox:
+                return None
+            mixer, ff, norm_a, norm_b, kv = block.mixer, block.feed_forward, block.mixer_norm, block.feed_forward_norm, caches.get(cache)
+            if cache != i or type(kv) is not LayerCache or mixer.window or type(norm_a) is not RMSNorm or type(norm_b) is not RMSNorm or norm_a.shift is not None or norm_b.shift is not None:
+                return None
             table, rot = mixer.position.rotary_table()
-            if rot != mixer.hd or ff.gate_up.gate != ops.SILU_GATE:
-                return False
-            weights = (mixer.qkv.weight, mixer.out.weight, ff.gate_up.weight, ff.down.weight)
-            if any(w.dtype != torch.bfloat16 or w.data_ptr() % 16 for w in weights):
-                return False
-            shapes.add((norms[0].size, norms[1].size, mixer.hidden, ff.hidden, mixer.nh, mixer.nkv, mixer.hd, ff.inter, mixer.scale, table.data_ptr(), caches[cache].group, tuple(caches[cache].k.shape)))
-        return len(shapes) == 1 and model.spec.hidden_size == next(iter(shapes))[0]
+            qkv, out, gate_up, down = mixer.qkv, mixer.out, ff.gate_up, ff.down
+            if qkv is None or out is None or gate_up is None or down is None or table is None or norm_a.weight is None or norm_b.weight is None:
+                return None  # not loaded yet
+            if (qkv.epi, out.epi, gate_up.epi, down.epi) != (STORE, RESIDUAL, GATED, RESIDUAL) or qkv.act or gate_up.gate != ops.SILU_GATE:
+                return None
+            if out.bias is not None or gate_up.bias is not None or down.bias is not None or rot != mixer.hd:
+                return None
+            hidden, rows, q_dim, inter = mixer.hidden, mixer.q_dim + 2 * mixer.kv_dim, mixer.q_dim, ff.inter
+            bias, k, v = qkv.bias, kv.k, kv.v
+            tensors = (qkv.weight, out.weight, gate_up.weight, down.weight, k, v, norm_a.weight, norm_b.weight) + (() if bias is None else (bias,))
+            if v is None or [t.shape for t in tensors] != [(rows, hidden), (hidden, q_dim), (2 * inter, hidden), (hidden, inter), *[(k.shape[0], mixer.nkv, mixer.hd)] * 2, (hidden,), (hidden,), (rows,)][: len(tensors)]:
+                return None
+            at = [t.data_ptr() for t in tensors if t.dtype == (bf16 if t.dim() > 1 else fp32) and t.is_contiguous() and t.is_cuda == cuda]
+            if len(at) != len(tensors) or any(a % 16 for a in at):
+                return None
+            shapes.add((hidden, mixer.nh, mixer.nkv, mixer.hd, inter, mixer.scale, table.data_ptr(), kv.group, k.shape[0]))
+            layers.append((*at, norm_a.eps, norm_b.eps))
+        if len(shapes) != 1:
+            return None
+        *sizes, scale, rope, group, _ = shapes.pop()
+        return Form(tuple(sizes), scale, group, rope, tuple(layers)) if sizes[0] == model.spec.hidden_size else None
+
+    def _open(self, form: Form) -> None:
+        """Asks the kernel what it takes, makes its scratch and its table of
+        layers (a runner that never decodes a few tokens loads no library for it)."""
+        device, before = self.model.rt.device, self.form
+        if before is not None:
+            torch.cuda.synchronize(device)  # a step may still read the table that goes
+        self.form = None
+        if before is None or before.sizes != form.sizes:
+            self.ctas = [0] + [ops.decode_stack_ctas(n, *form.sizes, self.page) for n in range(1, ops.DECODE_STACK_TOKENS + 1)]
+            if any(self.ctas):
+                # the kernel's own scratch: rotated queries, the key splits' outputs, the activation; and its barrier word
+                _, heads, _, hd, inter = form.sizes
+                most, ctas = max(n for n, c in enumerate(self.ctas) if c), max(self.ctas)
+                self.q = torch.empty((most, heads * hd), dtype=torch.bfloat16, device=device)
+                self.act = torch.empty(ops.decode_stack_act_numbers(most, inter, ctas), dtype=torch.bfloat16, device=device)
+                self.part_o = torch.empty((ctas, 8, hd), dtype=torch.float32, device=device)
+                self.part_ml = torch.empty((ctas, 8, 2), dtype=torch.float32, device=device)
+                self.barrier = torch.zeros(32, dtype=torch.int32, device=device)
+        if any(self.ctas):
+            entries = []
+            for layer, cache in self.model.run:
+                block, kv = self.model.layers[layer], self.caches[cache]
+                mixer, ff = block.mixer, block.feed_forward
+                entries.append(ops.decode_stack_layer(mixer.qkv.weight, mixer.out.weight, ff.gate_up.weight, ff.down.weight, block.mixer_norm.weight, block.feed_forward_norm.weight, mixer.qkv.bias,
+                                                      kv.k, kv.v, block.mixer_norm.eps, block.feed_forward_norm.eps, *form.sizes))
+            self.table = torch.frombuffer(bytearray(b"".join(entries)), dtype=torch.uint8).to(device)
+        self.form = form
 
     @classmethod
     def build(cls, model, caches: dict, block_size: int) -> Optional["DecodeStack"]:
-        """The stack of a loaded model over one runner's caches, or None where
-        the model's layers or sizes are not ones the kernel takes."""
-        if model.rt.device.type != "cuda" or not cls.fits(model, caches):
+        """The stack of a model over one runner's caches, or None where the
+        model's blocks are not ones the kernel could take.  (Whether they are is
+        seen at a step: the model may be loaded, or loaded again, after this.)"""
+        if model.rt.device.type != "cuda" or model.rt.dtype != torch.bfloat16 or any(type(block) is not PrenormResidual for block in model.layers):
             return None
         return cls(model, caches, block_size)
 
     def takes(self, ctx, h) -> bool:
         n = ctx.n_tokens
-        if not ctx.decode_only or n > ops.DECODE_STACK_TOKENS or n * self.sizes[0] > self.MOST_NUMBERS or ctx.stream_of(h) is None:
+        if not ctx.decode_only or n > ops.DECODE_STACK_TOKENS or n * h.shape[1] > self.MOST_NUMBERS or ctx.stream_of(h) is None:
             return False
-        if self.ctas is None:
-            self._open()
+        form = self.look()
+        if form is None:
+            return False
+        if form != self.form:
+            self._open(form)
         return self.ctas[n] > 0
 
     def forward(self, ctx, h) -> None:
-        """The step's rows through all layers: what the last product added to
-        ``h`` is left in the stream's accumulator."""
-        self._describe()
+        """The step's rows through all layers (a step that :meth:`takes` has
+        just said yes to): what the last product added to ``h`` is left in the
+        stream's accumulator."""
+        form = self.form
         alt, acc, other = ctx.stream_buffers(h)
-        group = ctx.groups[self.group]
-        ops.decode_stack(self.table, len(self.model.run), self.ctas[ctx.n_tokens], self.sizes, self.page, self.scale, h, alt, acc, other, ctx.positions, group.block_table, group.slot_map, self.rope,
+        group = ctx.groups[form.group]
+        rope = self.model.layers[self.model.run[0][0]].mixer.position.rotary_table()[0]
+        ops.decode_stack(self.table, len(form.layers), self.ctas[ctx.n_tokens], form.sizes, self.page, form.scale, h, alt, acc, other, ctx.positions, group.block_table, group.slot_map, rope,
                          self.q, self.part_o, self.part_ml, self.act, self.barrier, ctx.status)
         ctx.owe_accumulator(h)
+        ctx.keep += [self.table, rope, self.q, self.part_o, self.part_ml, self.act, self.barrier]  # a recording of this launch reads them at its replays
 
     def reset(self) -> None:
         """After a kernel gave up: its barrier may stand half way."""
-        if self.ctas is not None and any(self.ctas):
+        if any(self.ctas):
             self.barrier.zero_()

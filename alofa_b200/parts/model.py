@@ -42,6 +42,7 @@ class Model:
         if len(copies) > 1:
             raise AlofaError("unsupported", "blocks over several residual streams cannot be mixed with others", f"stream_copies={sorted(copies)}")
         self.stream_copies = copies.pop() if copies else 0
+        self.loads = 0  # how often weights were loaded: what was recorded of earlier ones is not run again
 
     def parts(self):
         return [self.embedding, *self.layers, self.final_norm, self.head]
@@ -54,6 +55,7 @@ class Model:
 
     def load(self, state: dict) -> None:
         state = dict(state)
+        self.loads += 1
         for part in self.parts():
             part.load(state)
 

@@ -2,8 +2,10 @@
 matrices and within shared memory, over shapes with odd and even chunk counts, groups of one to eight and one to eight
 tokens."""
 import ctypes
+import weakref
 
 import pytest
+import torch
 
 SHAPES = {
     "0.5b": (896, 14, 2, 64, 4864), "1.5b": (1536, 12, 2, 128, 8960), "7b": (3584, 28, 4, 128, 18944),
@@ -72,3 +74,74 @@ def test_products_are_covered_once(name, tokens, ctas):
                     first, second = (8 * t, inter) if phase == 2 else (16 * t, 8)
                 covered |= set(range(first, first + 8)) | set(range(first + second, first + second + 8))
         assert len(seen) == tiles * slices and covered == set(range(rows))
+
+
+@pytest.fixture
+def small():
+    """A bfloat16 model of the kernel's form on the CPU, not loaded, weights for it, and what looks at it."""
+    from alofa_b200.engine.step import StepRunner
+    from alofa_b200.models.qwen2 import Qwen2Config, build_spec
+    from alofa_b200.parts.base import Runtime
+    from alofa_b200.parts.decode_stack import DecodeStack
+    from alofa_b200.parts.model import Model
+    from alofa_b200.weights.loader import load_state
+    from alofa_b200.weights.random_init import random_state
+
+    rt = Runtime(torch.device("cpu"), torch.bfloat16)
+    model = Model(build_spec(Qwen2Config(2, 192, 3, 3, 64, 576, 300, 1e-6, 1e4, True, 4096)), rt)
+    runner = StepRunner(model, block_size=64, num_pages=4, max_requests=2, max_tokens=128, max_step_tokens=32)
+    state = lambda seed: load_state(model.tensors(), random_state(model.tensors(), seed, torch.bfloat16, "cpu"), rt.dtype, rt.device)  # noqa: E731
+    return model, state, DecodeStack(model, runner.storage.caches, 64)
+
+
+def test_a_model_may_be_loaded_after_its_runner_was_made(small):
+    model, state, stack = small
+    assert stack.look() is None
+    model.load(state(1))
+    form = stack.look()
+    assert form.sizes == (192, 3, 3, 64, 576) and len(form.layers) == 2 and form == stack.look()
+
+
+def test_a_model_loaded_again_is_described_again_and_its_old_weights_go(small):
+    model, state, stack = small
+    model.load(state(1))
+    stack.form = first = stack.look()
+    old = [weakref.ref(block.mixer.out.weight) for block in model.layers] + [weakref.ref(model.layers[0].mixer.position.rotary_table()[0])]
+    again = state(2)  # beside the old ones: other addresses
+    model.load(again)
+    assert stack.look() != first and model.loads == 2
+    assert [ref() for ref in old] == [None] * len(old)
+
+
+def unaligned(t):
+    room = torch.empty(t.numel() + 1, dtype=t.dtype)
+    room[1:] = t.flatten()
+    return room[1:].view(t.shape)
+
+
+@pytest.mark.parametrize("what", ["alignment", "type", "bias", "vector", "eps", "mixer", "window"])
+def test_what_the_kernel_does_not_have_goes_layer_by_layer(small, what):
+    """Looked at anew at every step: what changed behind the runner's back is refused, not run wrongly or raised at."""
+    from alofa_b200.parts.linear import RESIDUAL, Linear
+
+    model, state, stack = small
+    model.load(state(1))
+    form, block = stack.look(), model.layers[1]
+    weight = block.mixer.out.weight
+    if what == "alignment":
+        block.mixer.out = Linear(unaligned(weight), None, RESIDUAL)
+    elif what == "type":
+        block.mixer.out = Linear(weight.float(), None, RESIDUAL)
+    elif what == "bias":
+        block.mixer.out = Linear(weight, torch.ones(192), RESIDUAL)
+    elif what == "vector":
+        block.mixer_norm.weight = unaligned(block.mixer_norm.weight)
+    elif what == "mixer":
+        block.mixer = type("Other", (type(block.mixer),), {})(block.mixer.spec, model.rt)
+    elif what == "window":
+        block.mixer.window = 64
+    else:
+        block.mixer_norm.eps = 1e-3
+        assert stack.look() is not None and stack.look() != form
+        return
+    assert stack.look() is None

@@ -164,3 +164,74 @@ def test_infinities_nan_and_large_numbers_of_an_embedding_reach_the_logits(folde
     assert want[0].isnan().all() and not want[2:].isnan().any()
     for i in (2, 3, 4):
         assert (got[i] - want[i]).norm() <= 2**-7 * want[i].norm()
+
+
+def test_recorded_steps_of_a_model_loaded_again(folders):
+    """A model that is loaded again decodes with the new weights, at sizes that were recorded before and at others; one that the kernel
+    cannot take any more goes layer by layer."""
+    from alofa_b200.csrc import ops
+    from alofa_b200.engine.loading import load_model
+    from alofa_b200.engine.step import StepEntry, StepRunner
+    from alofa_b200.parts.linear import RESIDUAL, Linear
+    from alofa_b200.weights.loader import load_state
+
+    def make(model):
+        return StepRunner(model, block_size=64, num_pages=8, max_requests=2, max_tokens=128, max_step_tokens=64)
+
+    def steps(runner, n):
+        """Logits of the last of three steps (outright, recorded, replayed) of n requests, and its launches."""
+        slots = [runner.admit(i) for i in range(n)]
+        for t in range(3):
+            before = ops.launch_count()
+            out = runner.forward([StepEntry(s, [7 + t + i], [0]) for i, s in enumerate(slots)]).clone()
+        for s in slots:
+            runner.release(s)
+        runner.check_status()
+        return out, ops.launch_count() - before
+
+    model, _, _ = load_model(folders["h64_even"], "bfloat16")
+    runner = make(model)
+    first = {n: steps(runner, n)[0] for n in (1, 2)}
+    state = load_state(model.tensors(), folders["h64_even"], model.rt.dtype, model.rt.device)
+    for name in state:
+        if name.endswith("o_proj.weight"):
+            state[name] = state[name] * 3
+    model.load(state)
+    fresh = make(model)
+    for n in (1, 2):
+        got, launches = steps(runner, n)
+        want, fewest = steps(fresh, n)
+        assert torch.equal(got, want) and launches == fewest
+        assert (got - first[n]).norm() > 0.01 * got.norm()
+    # a bias, which the kernel does not have, behind the runner's back: the next size is layer by layer (recorded ones stay what they are)
+    model.loads += 1
+    for block in model.layers:
+        block.mixer.out = Linear(block.mixer.out.weight, torch.ones(256, device="cuda"), RESIDUAL)
+    got, launches = steps(runner, 2)
+    fresh.decode_stack = None
+    fresh._graphs.clear()
+    want, layers = steps(fresh, 2)
+    assert launches == layers > fewest and torch.equal(got, want)
+
+
+def test_runner_made_before_its_model_is_loaded(folders):
+    from alofa_b200.csrc import ops
+    from alofa_b200.engine.loading import load_model
+    from alofa_b200.engine.step import StepEntry, StepRunner
+    from alofa_b200.parts.model import Model
+    from alofa_b200.weights.loader import load_state
+
+    loaded, _, _ = load_model(folders["h64_even"], "bfloat16")
+    out, launches = [], []
+    for early in (True, False):
+        model = Model(loaded.spec, loaded.rt)
+        load = lambda: model.load(load_state(model.tensors(), folders["h64_even"], model.rt.dtype, model.rt.device))  # noqa: E731
+        if not early:
+            load()
+        runner = StepRunner(model, block_size=64, num_pages=4, max_requests=1, max_tokens=128, max_step_tokens=64, cuda_graphs=False)
+        if early:
+            load()
+        slot, before = runner.admit(1), ops.launch_count()
+        out.append(runner.forward([StepEntry(slot, [9], [0])]).clone())
+        launches.append(ops.launch_count() - before)
+    assert torch.equal(*out) and launches[0] == launches[1]
