@@ -235,3 +235,33 @@ def test_runner_made_before_its_model_is_loaded(folders):
         out.append(runner.forward([StepEntry(slot, [9], [0])]).clone())
         launches.append(ops.launch_count() - before)
     assert torch.equal(*out) and launches[0] == launches[1]
+
+
+@pytest.mark.parametrize("name", ["h64_even", "h128"])
+@pytest.mark.parametrize("context, pages, rows", [(40, 1, 16), (600, 7, 64)])
+def test_keys_that_weigh_nothing(folders, name, context, pages, rows):
+    """Scores of minus infinity, and finite ones as far below the others, over a whole granule, warp and split of keys: the others decide."""
+    from alofa_b200.engine.loading import load_model
+    from alofa_b200.engine.step import StepEntry, StepRunner
+
+    model, _, _ = load_model(folders[name], "bfloat16")
+    for block in model.layers:  # queries that are known: ten everywhere, turned by the position
+        block.mixer.qkv.weight[: block.mixer.q_dim] = 0
+        block.mixer.qkv.bias[: block.mixer.q_dim] = 10
+    ids = [int(t) for t in np.random.default_rng(3).integers(0, 300, context + 1)]
+    out = []
+    for stacked, value in ((False, -3e38), (True, -3e38), (True, -1e32)):
+        runner = StepRunner(model, block_size=64, num_pages=10, max_requests=1, max_tokens=640, max_step_tokens=640, cuda_graphs=False)
+        if not stacked:
+            runner.decode_stack = None
+        slot = runner.admit(1)
+        runner.forward([StepEntry(slot, ids[:context])])
+        for kv in runner.storage.caches.values():
+            k = kv.k.view(-1, 64, *kv.k.shape[1:])
+            k[:pages, :rows, :, kv.k.shape[2] // 2 - 1] = value  # of the slowest pair: hardly turned
+        out.append(runner.forward([StepEntry(slot, ids[context:], [0])]).clone())
+        runner.check_status()
+    want, got, finite = out
+    assert want.isfinite().all() and got.isfinite().all()
+    assert (got - want).norm() <= 2**-7 * want.norm()
+    assert torch.equal(got, finite)
