@@ -960,6 +960,15 @@ bool make_piece_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t 
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+constexpr int SMEM_LIMIT = 232448;  // bytes a CTA may have
+
+// Sizes that the kernel is written for (whether their shares and rings fit is plan_stack's to say).
+bool sizes_fit(int tokens, int hidden, int heads, int kv_heads, int head_dim, int inter) {
+  if (tokens < 1 || tokens > MAX_TOKENS || hidden < 64 || hidden % 64 || inter < 64 || inter % 64 || kv_heads < 1 || heads < 1 || heads % kv_heads || heads / kv_heads > 8) return false;
+  // (far more than fits; below it no product of sizes leaves 32 bits)
+  return (head_dim == 64 || head_dim == 128) && hidden <= 1 << 16 && inter <= 1 << 19 && heads <= 1 << 10;
+}
+
 typedef void (*StackKernel)(const StackArgs);
 StackKernel kernel_of(int head_dim) {
   return head_dim == 64 ? (StackKernel)decode_stack_kernel<64> : head_dim == 128 ? (StackKernel)decode_stack_kernel<128> : nullptr;
@@ -1006,6 +1015,11 @@ size_t plan_stack(StackArgs* a, int head_dim, int ctas) {
     }
   }
   if (most > MAX_TILES) return 0;
+  for (int p = 0; p < 4; ++p) {  // pieces of a CTA are counted in 16 bits
+    const PhasePlan& s = a->plan[p];
+    const int tiles = s.kg ? (s.tiles + s.rg - 1) / s.rg : (s.tiles + ctas - 1) / ctas, slices = s.kg ? (s.slices + s.kg - 1) / s.kg : s.slices;
+    if ((long long)tiles * slices > 32767) return 0;
+  }
   a->act_stride = ((a->plan[P_GATE].tiles + ctas - 1) / ctas * T * 8 + 63) / 64 * 64;
   a->x_stride = 2 * wide + 16;
   a->x_bytes = T * a->x_stride;
@@ -1014,7 +1028,7 @@ size_t plan_stack(StackArgs* a, int head_dim, int ctas) {
   a->work_bytes = a->x_bytes + sums > merge ? a->x_bytes + sums : merge;
   a->work_bytes = (a->work_bytes + 15) / 16 * 16;
   const size_t rest = (size_t)a->work_bytes + (size_t)T * head_dim * 4 + (size_t)H * 4 + 64 * (size_t)a->qkv_tiles + sizeof(Small) + 64;
-  const size_t limit = 232448, piece = (size_t)WARPS * (2048 * a->chunks + 8);
+  const size_t limit = SMEM_LIMIT, piece = (size_t)WARPS * (2048 * a->chunks + 8);
   if (rest + 2 * piece > limit) return 0;
   a->slots = (int)((limit - rest) / piece);
   if (a->slots > 8) a->slots = 8;
@@ -1029,11 +1043,12 @@ size_t plan_stack(StackArgs* a, int head_dim, int ctas) {
 }  // namespace
 
 ALOFA_API int alofa_decode_stack_layer_bytes() { return (int)sizeof(StackLayer); }
-ALOFA_API int alofa_decode_stack_cta_floats(int head_dim) { return 8 * (head_dim + 2); }
 
 // What plan_stack decides, for a look from outside: out[0..15] the phases' tiles, slices, ranges of slices and of tiles, then chunks,
-// pieces in a ring, an operand row's bytes, the operand's and the work area's, all shared memory.  0: sizes the kernel does not take.
+// pieces in a ring, an operand row's bytes, the operand's and the work area's, all shared memory, whether it is paced.  0: sizes the kernel does not take.
 ALOFA_API int alofa_decode_stack_plan(int tokens, int hidden, int heads, int kv_heads, int head_dim, int inter, int ctas, int* out) {
+  memset(out, 0, 23 * sizeof(int));
+  if (ctas < 1 || !sizes_fit(tokens, hidden, heads, kv_heads, head_dim, inter)) return 0;
   StackArgs a = {};
   a.tokens = tokens;
   a.hidden = hidden;
@@ -1043,16 +1058,15 @@ ALOFA_API int alofa_decode_stack_plan(int tokens, int hidden, int heads, int kv_
   a.inter = inter;
   const size_t smem = plan_stack(&a, head_dim, ctas);
   memcpy(out, a.plan, sizeof(a.plan));
-  const int rest[6] = {a.chunks, a.slots, a.x_stride, a.x_bytes, a.work_bytes, (int)smem};
+  const int rest[7] = {a.chunks, a.slots, a.x_stride, a.x_bytes, a.work_bytes, (int)smem, a.paced};
   memcpy(out + 16, rest, sizeof(rest));
   return smem > 0;
 }
 
 // How many CTAs run a step of these sizes: one per SM, all resident together; 0 where the kernel does not take them.
 ALOFA_API int alofa_decode_stack_ctas(int tokens, int hidden, int heads, int kv_heads, int head_dim, int inter, int page) {
-  if (tokens < 1 || tokens > MAX_TOKENS || hidden % 64 || inter % 64 || inter < 64 || kv_heads < 1 || heads % kv_heads || heads / kv_heads > 8 || page % GRANULE || page < GRANULE) return 0;
+  if (!sizes_fit(tokens, hidden, heads, kv_heads, head_dim, inter) || page % GRANULE || page < GRANULE) return 0;
   StackKernel kernel = kernel_of(head_dim);
-  if (!kernel || (heads * head_dim) % 64) return 0;
   int device, sms, coop;
   if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
       cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop)
@@ -1066,7 +1080,7 @@ ALOFA_API int alofa_decode_stack_ctas(int tokens, int hidden, int heads, int kv_
   a.group = heads / kv_heads;
   a.inter = inter;
   const size_t smem = plan_stack(&a, head_dim, sms);
-  if (!smem || cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+  if (!smem || cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT) != cudaSuccess) return 0;
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, THREADS, smem) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
@@ -1079,6 +1093,7 @@ ALOFA_API int alofa_decode_stack_ctas(int tokens, int hidden, int heads, int kv_
 ALOFA_API int alofa_decode_stack_layer(void* entry, const void* qkv, const void* out, const void* gate_up, const void* down, const float* gamma_mixer,
                                        const float* gamma_ff, const float* qkv_bias, void* k, void* v, float eps_mixer, float eps_ff, int hidden, int heads,
                                        int kv_heads, int head_dim, int inter) {
+  if (!entry || !qkv || !out || !gate_up || !down || !gamma_mixer || !gamma_ff || !k || !v || !sizes_fit(1, hidden, heads, kv_heads, head_dim, inter)) return ALOFA_ERR_ARGUMENT;
   StackLayer L;
   memset(&L, 0, sizeof(L));
   const int q_dim = heads * head_dim, chunks = (hidden / 64) % 2 || (q_dim / 64) % 2 || (inter / 64) % 2 ? 1 : 2;
@@ -1102,7 +1117,7 @@ ALOFA_API int alofa_decode_stack(const void* layers, int n_layers, int ctas, int
                                  const int* slot_map, const float* rope, void* q, float* part_o, float* part_ml, void* act, unsigned* barrier, int* status,
                                  cudaStream_t stream) {
   StackKernel kernel = kernel_of(head_dim);
-  if (!kernel || tokens < 1 || tokens > MAX_TOKENS) return ALOFA_ERR_ARGUMENT;
+  if (!sizes_fit(tokens, hidden, heads, kv_heads, head_dim, inter) || page % GRANULE || page < GRANULE || n_layers < 1 || table_stride < 1 || ctas < 1 || tokens * kv_heads > ctas) return ALOFA_ERR_ARGUMENT;
   StackArgs a = {};
   a.layers = (const StackLayer*)layers;
   a.n_layers = n_layers;
@@ -1133,7 +1148,8 @@ ALOFA_API int alofa_decode_stack(const void* layers, int n_layers, int ctas, int
   a.per_cta = 1.0f / (float)ctas;
   const size_t smem = plan_stack(&a, head_dim, ctas);
   if (!smem) return ALOFA_ERR_ARGUMENT;
-  if (cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return ALOFA_ERR_LAUNCH;
+  // always the most there is: a size of its own for each step could come between another thread's setting and its launch
+  if (cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT) != cudaSuccess) return ALOFA_ERR_LAUNCH;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(THREADS);

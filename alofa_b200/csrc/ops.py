@@ -1579,9 +1579,12 @@ def decode_stack(table, n_layers: int, ctas: int, sizes: tuple, page: int, scale
     (hidden, heads, kv_heads, head_dim, inter); ``barrier``: a word that only
     this kernel writes, zero at first."""
     tokens, hidden = base.shape
-    hd, kv = sizes[3], sizes[2]
-    if hidden != sizes[0] or any(tuple(t.shape) != (tokens, hidden) for t in (alt, acc, other)) or block_table.shape[0] != tokens or q.shape[0] < tokens or act.numel() < decode_stack_act_numbers(tokens, sizes[4], ctas) or part_o.shape[0] < ctas or tokens * kv > ctas:
-        raise AlofaError("invalid_argument", "decode_stack sizes disagree", f"base={tuple(base.shape)} acc={tuple(acc.shape)} tables={tuple(block_table.shape)} ctas={ctas}")
+    _, heads, kv, hd, inter = sizes
+    if hidden != sizes[0] or any(tuple(t.shape) != (tokens, hidden) for t in (alt, acc, other)) or block_table.dim() != 2 or block_table.shape[0] != tokens or positions.numel() < tokens or slot_map.numel() < tokens:
+        raise AlofaError("invalid_argument", "decode_stack sizes disagree", f"base={tuple(base.shape)} acc={tuple(acc.shape)} tables={tuple(block_table.shape)}")
+    if (table.numel() * table.element_size() < n_layers * _decode_stack().alofa_decode_stack_layer_bytes() or rope.dim() != 3 or tuple(rope.shape[1:]) != (hd // 2, 2) or q.numel() < tokens * heads * hd
+            or act.numel() < decode_stack_act_numbers(tokens, inter, ctas) or part_o.numel() < ctas * 8 * hd or part_ml.numel() < ctas * 16):
+        raise AlofaError("invalid_argument", "decode_stack scratch or tables are too small", f"table={tuple(table.shape)} rope={tuple(rope.shape)} q={tuple(q.shape)} act={tuple(act.shape)} part_o={tuple(part_o.shape)} ctas={ctas}")
     _done(
         _decode_stack().alofa_decode_stack(
             _dev(table, "table"), n_layers, ctas, tokens, *sizes, page, block_table.shape[1], float(scale), _dev(base, "base", torch.float32), _dev(alt, "alt", torch.float32), _dev(acc, "acc", torch.int64), _dev(other, "other", torch.int64),

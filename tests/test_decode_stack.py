@@ -145,3 +145,32 @@ def test_what_the_kernel_does_not_have_goes_layer_by_layer(small, what):
         assert stack.look() is not None and stack.look() != form
         return
     assert stack.look() is None
+
+
+BAD = [(0, 896, 14, 2, 64, 4864), (9, 896, 14, 2, 64, 4864), (1, 0, 14, 2, 64, 4864), (1, 896, 14, 0, 64, 4864), (1, 896, 0, 2, 64, 4864), (1, 896, 14, 4, 64, 4864), (1, 896, 18, 2, 64, 4864),
+       (1, 896, 14, 2, 96, 4864), (1, 896, 14, 2, 0, 4864), (1, 900, 14, 2, 64, 4864), (1, 896, 14, 2, 64, 0), (1, 896, 14, 2, 64, 4800 + 32), (1, 1 << 30, 14, 2, 64, 4864), (1, 896, 14, 2, 64, 1 << 30)]
+
+
+@pytest.mark.parametrize("sizes", BAD)
+def test_entries_refuse_sizes_without_a_look_at_the_device(sizes):
+    from alofa_b200.csrc import ops
+
+    lib, out = ops._decode_stack(), (ctypes.c_int * 23)()
+    tokens, hidden, heads, kv_heads, hd, inter = sizes
+    assert lib.alofa_decode_stack_plan(*sizes, 148, out) == 0 and not any(out)
+    assert lib.alofa_decode_stack_ctas(*sizes, 64) == 0
+    if tokens == 1:
+        assert lib.alofa_decode_stack_layer(*[16] * 7, None, 16, 16, 1e-6, 1e-6, *sizes[1:]) == 1
+    assert lib.alofa_decode_stack(16, 1, 148, tokens, hidden, heads, kv_heads, hd, inter, 64, 1, 1.0, *[16] * 15, None) == 1
+
+
+def test_entries_refuse_pages_grids_and_tables():
+    from alofa_b200.csrc import ops
+
+    lib, out, good = ops._decode_stack(), (ctypes.c_int * 23)(), (8, 896, 14, 2, 64, 4864)
+    assert lib.alofa_decode_stack_plan(*good, 148, out) == 1 and lib.alofa_decode_stack_plan(*good, 0, out) == 0
+    for page in (0, 8, 24):
+        assert lib.alofa_decode_stack_ctas(*good, page) == 0
+    for layers, ctas, page, stride in ((0, 148, 64, 1), (1, 0, 64, 1), (1, 15, 64, 1), (1, 148, 0, 1), (1, 148, 24, 1), (1, 148, 64, 0)):
+        assert lib.alofa_decode_stack(16, layers, ctas, *good, page, stride, 1.0, *[16] * 15, None) == 1
+    assert lib.alofa_decode_stack_layer(16, None, *[16] * 5, None, 16, 16, 1e-6, 1e-6, *good[1:]) == 1

@@ -265,3 +265,34 @@ def test_keys_that_weigh_nothing(folders, name, context, pages, rows):
     assert want.isfinite().all() and got.isfinite().all()
     assert (got - want).norm() <= 2**-7 * want.norm()
     assert torch.equal(got, finite)
+
+
+def test_two_runners_on_two_streams(folders):
+    """Steps of two runners side by side, of shapes that want different amounts of shared memory: the same bits as one after the other."""
+    from alofa_b200.engine.loading import load_model
+    from alofa_b200.engine.step import StepEntry, StepRunner
+
+    def make(name, n):
+        model, _, _ = load_model(folders[name], "bfloat16")
+        runner = StepRunner(model, block_size=64, num_pages=2 * n, max_requests=n, max_tokens=128, max_step_tokens=64)
+        return runner, [runner.admit(i) for i in range(n)]
+
+    def step(pair, t):
+        runner, slots = pair
+        return runner.forward([StepEntry(s, [(7 * t + i) % 300], [0]) for i, s in enumerate(slots)])
+
+    kinds, steps = [("h64_odd", 1), ("h128_group7", 8)], 12
+    want = []
+    for kind in kinds:
+        pair = make(*kind)
+        want.append([step(pair, t).clone() for t in range(steps)])
+    pairs, streams, got = [make(*kind) for kind in kinds], [torch.cuda.Stream() for _ in kinds], [[], []]
+    torch.cuda.synchronize()
+    for t in range(steps):
+        for i, (pair, stream) in enumerate(zip(pairs, streams)):
+            with torch.cuda.stream(stream):
+                got[i].append(step(pair, t).clone())
+    torch.cuda.synchronize()
+    for i, (runner, _) in enumerate(pairs):
+        runner.check_status()
+        assert all(torch.equal(a, b) for a, b in zip(got[i], want[i]))
