@@ -58,12 +58,19 @@ struct LayerVectors {
   bf16* v;
   float eps_mixer, eps_ff;
 };
-struct alignas(64) StackLayer {
+struct alignas(64) StackLayer {  // of the table of layers
   CUtensorMap maps[4];  // q/k/v, output, gate and up, down: boxes of 8 rows x 2 x `chunks` x 64 columns
   LayerVectors vectors;
   int pad[4];
 };
 static_assert(sizeof(StackLayer) % 64 == 0, "tensor maps need 64-byte alignment");
+// The table is a kernel parameter, as the maps of every other kernel are: in global memory that the host writes, each map would want a
+// fence of the tensor-map proxy in every CTA first, 100 ns a map and SM (10 us a step of 0.5B sizes).  Parameters have 32,764 bytes: a
+// deeper model goes in launches of so many layers.
+constexpr int MAX_LAYERS = 48;
+struct StackTable {
+  StackLayer layers[MAX_LAYERS];
+};
 
 struct PhasePlan {
   int tiles, slices;  // tiles of 16 rows, slices of `chunks` * 64 columns
@@ -71,8 +78,8 @@ struct PhasePlan {
 };
 
 struct StackArgs {
-  const StackLayer* layers;
   int n_layers;
+  int added;                 // whether `acc` holds something already (a launch that goes on where another stopped)
   int tokens, hidden, heads, kv_heads, group, inter;
   int page, table_stride;
   int chunks, slots;         // 64-column chunks of a piece, pieces in a warp's ring
@@ -85,8 +92,8 @@ struct StackArgs {
   PhasePlan plan[4];
   float* base;               // [tokens, hidden]: the stream, before phase 1 (and at the end) without what `acc` holds
   float* base_ff;            // the same before phase 4, without what `acc_ff` holds
-  long long* acc;            // [tokens, hidden]: what the last feed-forward added; zero before, as is acc_ff
-  long long* acc_ff;         // what the attention added; zero afterwards
+  long long* acc;            // [tokens, hidden]: what the last feed-forward added; zero before unless `added`
+  long long* acc_ff;         // what the attention added; zero before and afterwards
   const int* positions;
   const int* block_table;    // [tokens, table_stride]
   const int* slot_map;       // [tokens]
@@ -201,7 +208,7 @@ __device__ __forceinline__ void next_phase(Loader& ld, const Small& sm, int warp
 // load may leave out is set to zero first.  (Loads that go to a clamped place instead all hit one line: 7,500 cycles for an
 // operand of one token.)
 template <int HD>
-__global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_constant__ StackArgs a) {
+__global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_constant__ StackArgs a, const __grid_constant__ StackTable table) {
   constexpr int TP = MAX_TOKENS, C32 = HD / 32;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t piece_bytes = 2048u * a.chunks;
@@ -256,12 +263,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
     s.head_rows = tid == P_QKV ? HD : 16;
     sm.share[tid] = s;
   }
-  if (tid < (int)(sizeof(LayerVectors) / 4)) reinterpret_cast<int*>(&sm.layer[0])[tid] = reinterpret_cast<const int*>(&a.layers[0].vectors)[tid];
-  if (cta == ctas - 1)  // the table into L2
-    for (int i = tid * 128; i < a.n_layers * (int)sizeof(StackLayer); i += THREADS * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(a.layers) + i));
-  // The maps lie in global memory that the host wrote: without this an SM may use what it kept of another table that lay at the same
-  // address.  A map by a thread, dealt over the warps; the __syncthreads() below hands that on to the lanes that ask for copies.
-  for (int i = warp + WARPS * lane; i < a.n_layers * 4; i += THREADS) asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(&a.layers[i >> 2].maps[i & 3]) : "memory");
+  if (tid < (int)(sizeof(LayerVectors) / 4)) reinterpret_cast<int*>(&sm.layer[0])[tid] = reinterpret_cast<const int*>(&table.layers[0].vectors)[tid];
   if (tid == 0) sm.abort_flag = 0;
   if (tid < WARPS * a.slots) mbar_init(bars + tid, 1);
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -325,7 +327,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
 #pragma unroll 1
       for (int k = 0; k < ask && ld.layer < a.n_layers; ++k) {
         mbar_expect_tx(my_bars + into, piece_bytes);
-        tma_load_piece(my_ring + (uint32_t)into * piece_bytes, &a.layers[ld.layer].maps[ld.phase], smem_u32(my_bars + into), ld.row, ld.chunk);
+        tma_load_piece(my_ring + (uint32_t)into * piece_bytes, &table.layers[ld.layer].maps[ld.phase], smem_u32(my_bars + into), ld.row, ld.chunk);
         ++ld.asked;
         if (++ld.piece == ld.end) {
           next_phase(ld, sm, warp, a.n_layers, a.chunks);
@@ -552,7 +554,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
     const LayerVectors& L = sm.layer[layer & 1];
     const LayerVectors& N = sm.layer[(layer + 1) & 1];
     if (layer + 1 < a.n_layers) {
-      const LayerVectors& next = a.layers[layer + 1].vectors;
+      const LayerVectors& next = table.layers[layer + 1].vectors;
       if (tid < (int)(sizeof(LayerVectors) / 4)) reinterpret_cast<int*>(&sm.layer[(layer + 1) & 1])[tid] = reinterpret_cast<const int*>(&next)[tid];
       if (cta == ctas - 1) {  // the next layer's vectors into L2
         for (int i = tid * 32; i < H; i += THREADS * 32) {
@@ -572,7 +574,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
         // the operand
         if (phase == P_QKV || phase == P_GATE) {
           const bool mixer = phase == P_QKV;
-          normed_rows(mixer ? L.eps_mixer : L.eps_ff, mixer ? a.base : a.base_ff, mixer ? a.acc : a.acc_ff, !mixer || layer > 0);
+          normed_rows(mixer ? L.eps_mixer : L.eps_ff, mixer ? a.base : a.base_ff, mixer ? a.acc : a.acc_ff, !mixer || layer > 0 || a.added);
         } else {
           const int per_row = WARPS >> t_bits, t = warp >> (4 - t_bits), first = (warp & (per_row - 1)) * 32 + lane, step = 32 * per_row;
           const int cols = s.slices * a.chunks * 64, col0 = s.slice0 * a.chunks * 64;
@@ -759,9 +761,9 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
           }
         }
         if (!a.paced) refill(a.slots);
-        settle(a.base_ff, a.base, a.acc, layer > 0);
+        settle(a.base_ff, a.base, a.acc, layer > 0 || a.added);
         if (!wait()) goto leave;
-        if (layer > 0) clear(a.acc);
+        if (layer > 0 || a.added) clear(a.acc);
         if (it_token >= 0) {
           float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;  // of heads 2j and 2j + 1 of the group
           float o[HD / 16][4];
@@ -969,7 +971,7 @@ bool sizes_fit(int tokens, int hidden, int heads, int kv_heads, int head_dim, in
   return (head_dim == 64 || head_dim == 128) && hidden <= 1 << 16 && inter <= 1 << 19 && heads <= 1 << 10;
 }
 
-typedef void (*StackKernel)(const StackArgs);
+typedef void (*StackKernel)(const StackArgs, const StackTable);
 StackKernel kernel_of(int head_dim) {
   return head_dim == 64 ? (StackKernel)decode_stack_kernel<64> : head_dim == 128 ? (StackKernel)decode_stack_kernel<128> : nullptr;
 }
@@ -1089,7 +1091,7 @@ ALOFA_API int alofa_decode_stack_ctas(int tokens, int hidden, int heads, int kv_
   return sms;
 }
 
-// Fills one layer's entry of the table that the kernel reads (host memory; the caller copies the table to the device).
+// Fills one layer's entry of the table that a launch takes (host memory).
 ALOFA_API int alofa_decode_stack_layer(void* entry, const void* qkv, const void* out, const void* gate_up, const void* down, const float* gamma_mixer,
                                        const float* gamma_ff, const float* qkv_bias, void* k, void* v, float eps_mixer, float eps_ff, int hidden, int heads,
                                        int kv_heads, int head_dim, int inter) {
@@ -1112,6 +1114,7 @@ ALOFA_API int alofa_decode_stack_layer(void* entry, const void* qkv, const void*
   return ALOFA_OK;
 }
 
+// `layers`: the entries of alofa_decode_stack_layer one after the other, in host memory.
 ALOFA_API int alofa_decode_stack(const void* layers, int n_layers, int ctas, int tokens, int hidden, int heads, int kv_heads, int head_dim, int inter, int page,
                                  int table_stride, float scale, float* base, float* base_ff, long long* acc, long long* acc_ff, const int* positions, const int* block_table,
                                  const int* slot_map, const float* rope, void* q, float* part_o, float* part_ml, void* act, unsigned* barrier, int* status,
@@ -1119,8 +1122,6 @@ ALOFA_API int alofa_decode_stack(const void* layers, int n_layers, int ctas, int
   StackKernel kernel = kernel_of(head_dim);
   if (!sizes_fit(tokens, hidden, heads, kv_heads, head_dim, inter) || page % GRANULE || page < GRANULE || n_layers < 1 || table_stride < 1 || ctas < 1 || tokens * kv_heads > ctas) return ALOFA_ERR_ARGUMENT;
   StackArgs a = {};
-  a.layers = (const StackLayer*)layers;
-  a.n_layers = n_layers;
   a.tokens = tokens;
   a.hidden = hidden;
   a.heads = heads;
@@ -1160,9 +1161,16 @@ ALOFA_API int alofa_decode_stack(const void* layers, int n_layers, int ctas, int
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, kernel, a) != cudaSuccess) {
-    cudaGetLastError();
-    return ALOFA_ERR_LAUNCH;
+  for (int first = 0; first < n_layers; first += MAX_LAYERS) {
+    StackTable table;
+    a.n_layers = n_layers - first < MAX_LAYERS ? n_layers - first : MAX_LAYERS;
+    a.added = first > 0;
+    memcpy(&table, (const char*)layers + first * sizeof(StackLayer), a.n_layers * sizeof(StackLayer));
+    memset((char*)&table + a.n_layers * sizeof(StackLayer), 0, sizeof(table) - a.n_layers * sizeof(StackLayer));
+    if (cudaLaunchKernelEx(&cfg, kernel, a, table) != cudaSuccess) {
+      cudaGetLastError();
+      return ALOFA_ERR_LAUNCH;
+    }
   }
   return ALOFA_OK;
 }

@@ -1535,6 +1535,7 @@ def lru_scan(out, a, b, y, y_off: int, act: str, state, q_start, state_slots, n_
 
 
 DECODE_STACK_TOKENS = 8  # the most tokens that the one-kernel decode step takes
+DECODE_STACK_LAYERS = 48  # the layers that one launch of it takes
 
 
 def decode_stack_ctas(tokens: int, hidden: int, heads: int, kv_heads: int, head_dim: int, inter: int, page: int) -> int:
@@ -1575,22 +1576,24 @@ def decode_stack(table, n_layers: int, ctas: int, sizes: tuple, page: int, scale
     """All layers of a decode step, one token per request: what they add to the
     stream ``base`` is in ``base`` and the accumulator ``acc`` afterwards.  ``alt``:
     like ``base``, overwritten; ``acc`` and ``other``, like it, are zero before,
-    ``other`` afterwards too.  ``table``: the entries of :func:`decode_stack_layer` one after the other; ``sizes``:
-    (hidden, heads, kv_heads, head_dim, inter); ``barrier``: a word that only
-    this kernel writes, zero at first."""
+    ``other`` afterwards too.  ``table`` (bytes): the entries of
+    :func:`decode_stack_layer` one after the other; ``sizes``: (hidden, heads,
+    kv_heads, head_dim, inter); ``barrier``: a word that only this kernel
+    writes, zero at first."""
     tokens, hidden = base.shape
     _, heads, kv, hd, inter = sizes
     if hidden != sizes[0] or any(tuple(t.shape) != (tokens, hidden) for t in (alt, acc, other)) or block_table.dim() != 2 or block_table.shape[0] != tokens or positions.numel() < tokens or slot_map.numel() < tokens:
         raise AlofaError("invalid_argument", "decode_stack sizes disagree", f"base={tuple(base.shape)} acc={tuple(acc.shape)} tables={tuple(block_table.shape)}")
-    if (table.numel() * table.element_size() < n_layers * _decode_stack().alofa_decode_stack_layer_bytes() or rope.dim() != 3 or tuple(rope.shape[1:]) != (hd // 2, 2) or q.numel() < tokens * heads * hd
+    if (len(table) < n_layers * _decode_stack().alofa_decode_stack_layer_bytes() or rope.dim() != 3 or tuple(rope.shape[1:]) != (hd // 2, 2) or q.numel() < tokens * heads * hd
             or act.numel() < decode_stack_act_numbers(tokens, inter, ctas) or part_o.numel() < ctas * 8 * hd or part_ml.numel() < ctas * 16):
-        raise AlofaError("invalid_argument", "decode_stack scratch or tables are too small", f"table={tuple(table.shape)} rope={tuple(rope.shape)} q={tuple(q.shape)} act={tuple(act.shape)} part_o={tuple(part_o.shape)} ctas={ctas}")
+        raise AlofaError("invalid_argument", "decode_stack scratch or tables are too small", f"table={len(table)} rope={tuple(rope.shape)} q={tuple(q.shape)} act={tuple(act.shape)} part_o={tuple(part_o.shape)} ctas={ctas}")
     _done(
         _decode_stack().alofa_decode_stack(
-            _dev(table, "table"), n_layers, ctas, tokens, *sizes, page, block_table.shape[1], float(scale), _dev(base, "base", torch.float32), _dev(alt, "alt", torch.float32), _dev(acc, "acc", torch.int64), _dev(other, "other", torch.int64),
+            table, n_layers, ctas, tokens, *sizes, page, block_table.shape[1], float(scale), _dev(base, "base", torch.float32), _dev(alt, "alt", torch.float32), _dev(acc, "acc", torch.int64), _dev(other, "other", torch.int64),
             _dev(positions, "positions", torch.int32), _dev(block_table, "block_table", torch.int32), _dev(slot_map, "slot_map", torch.int32), _dev(rope, "rope", torch.float32),
             _dev(q, "q", torch.bfloat16), _dev(part_o, "part_o", torch.float32), _dev(part_ml, "part_ml", torch.float32), _dev(act, "act", torch.bfloat16), _dev(barrier, "barrier", torch.int32),
             _dev(status, "status", torch.int32), _stream(),
         ),
         "decode_stack", f"tokens={tokens} hidden={hidden} head_dim={hd}",
     )
+    count_launches(-(-n_layers // DECODE_STACK_LAYERS) - 1)

@@ -92,8 +92,6 @@ class DecodeStack:
         """Asks the kernel what it takes, makes its scratch and its table of
         layers (a runner that never decodes a few tokens loads no library for it)."""
         device, before = self.model.rt.device, self.form
-        if before is not None:
-            torch.cuda.synchronize(device)  # a step may still read the table that goes
         self.form = None
         if before is None or before.sizes != form.sizes:
             self.ctas = [0] + [ops.decode_stack_ctas(n, *form.sizes, self.page) for n in range(1, ops.DECODE_STACK_TOKENS + 1)]
@@ -113,7 +111,7 @@ class DecodeStack:
                 mixer, ff = block.mixer, block.feed_forward
                 entries.append(ops.decode_stack_layer(mixer.qkv.weight, mixer.out.weight, ff.gate_up.weight, ff.down.weight, block.mixer_norm.weight, block.feed_forward_norm.weight, mixer.qkv.bias,
                                                       kv.k, kv.v, block.mixer_norm.eps, block.feed_forward_norm.eps, *form.sizes))
-            self.table = torch.frombuffer(bytearray(b"".join(entries)), dtype=torch.uint8).to(device)
+            self.table = b"".join(entries)
         self.form = form
 
     @classmethod
@@ -147,7 +145,7 @@ class DecodeStack:
         ops.decode_stack(self.table, len(form.layers), self.ctas[ctx.n_tokens], form.sizes, self.page, form.scale, h, alt, acc, other, ctx.positions, group.block_table, group.slot_map, rope,
                          self.q, self.part_o, self.part_ml, self.act, self.barrier, ctx.status)
         ctx.owe_accumulator(h)
-        ctx.keep += [self.table, rope, self.q, self.part_o, self.part_ml, self.act, self.barrier]  # a recording of this launch reads them at its replays
+        ctx.keep += [rope, self.q, self.part_o, self.part_ml, self.act, self.barrier]  # a recording of this launch reads them at its replays
 
     def reset(self) -> None:
         """After a kernel gave up: its barrier may stand half way."""

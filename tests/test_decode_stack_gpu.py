@@ -112,30 +112,6 @@ def test_model_loaded_again(folders):
     assert (changed - want).norm() <= 2**-8 * want.norm()
 
 
-def test_table_at_an_address_used_before(folders):
-    """A table of layers that takes the place of a dropped one in memory describes other weights: none of the old one's maps is used."""
-    from alofa_b200.engine.loading import load_model
-    from alofa_b200.engine.step import StepEntry, StepRunner
-
-    models, places, reused = [], [], False
-    for i in range(6):
-        model, _, _ = load_model(folders["h64_even"], "bfloat16")  # earlier models stay: these weights lie elsewhere
-        for block in model.layers:
-            block.mixer.out.weight.mul_(1 + i)
-        models.append(model)
-        runner = StepRunner(model, block_size=64, num_pages=4, max_requests=1, max_tokens=128, max_step_tokens=64, cuda_graphs=False)
-        got = runner.forward([StepEntry(runner.admit(1), [7], [0])]).clone()
-        runner.check_status()
-        runner.release(0)
-        reused = reused or runner.decode_stack.table.data_ptr() in places
-        places.append(runner.decode_stack.table.data_ptr())
-        runner.decode_stack = None
-        want = runner.forward([StepEntry(runner.admit(2), [7], [0])]).clone()
-        assert (got - want).norm() <= 2**-8 * want.norm()
-        del runner
-    assert reused, "no table lay where another had been"
-
-
 def test_infinities_nan_and_large_numbers_of_an_embedding_reach_the_logits(folders):
     """The stream of a step as one kernel loses nothing that the same step layer by layer keeps."""
     from alofa_b200.engine.loading import load_model
@@ -296,3 +272,17 @@ def test_two_runners_on_two_streams(folders):
     for i, (runner, _) in enumerate(pairs):
         runner.check_status()
         assert all(torch.equal(a, b) for a, b in zip(got[i], want[i]))
+
+
+def test_more_layers_than_a_launch_takes(tmp_path):
+    """A model of more layers than the kernel's parameters hold goes in several launches; also one whose last launch is a single layer."""
+    from alofa_b200.models.qwen2 import NAME, Qwen2Config
+    from alofa_b200.weights.random_init import write_random_model
+
+    for layers in (48, 49, 100):
+        folder = write_random_model(tmp_path / str(layers), NAME, Qwen2Config(layers, 64, 1, 1, 64, 128, 300, 1e-6, 1e4, True, 4096), 7, torch.bfloat16)
+        got, launched, _ = decode(folder, [70, 3], 3, True)
+        want, more, _ = decode(folder, [70, 3], 3, False)
+        assert launched < more
+        # as in test_matches_layer_by_layer, the roundings of all layers: sqrt(2 sides * layers * 8) * 2^-9 / sqrt(3)
+        assert (got - want).norm() <= (2 * layers * 8 / 3) ** 0.5 * 2**-9 * want.norm()
