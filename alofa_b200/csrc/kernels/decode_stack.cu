@@ -135,9 +135,9 @@ __device__ __forceinline__ float exp2_fast(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// What a maximum of scores is taken off them as: scores of minus infinity (keys or queries out of bfloat16's range) weigh nothing, also
-// where a granule, a warp or a split has no others.
-__device__ __forceinline__ float finite(float top) { return top == -INFINITY ? 0.f : top; }
+// Where a maximum of scores starts.  Scores of minus infinity (keys or queries out of bfloat16's range) then weigh nothing also where a
+// granule, a warp or a split has no others: 2^(-inf - LOWEST) is 0, the difference of two such maxima 0.
+constexpr float LOWEST = -3.402823466e38f;
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&p);
@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
             for (int i = first; i < cols / 2; i += step) {
               const int c = (i >> 1) * 4, head = (col0 + c) / HD, d = (col0 + c) % HD, g = (int)((head + 0.5f) * a.per_group);
               const size_t at = (size_t)(sm.item0[t] + g * n) * 8 + (head - g * group);
-              float top = -INFINITY, sum = 0.f;
+              float top = LOWEST, sum = 0.f;
               float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
               for (int p0 = half; p0 < n; p0 += 10) {
@@ -605,9 +605,8 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
                 float up = top;
 #pragma unroll
                 for (int u = 0; u < 5; ++u) up = fmaxf(up, ml[u].x);
-                const float f = exp2_fast(top - finite(up));
+                const float f = exp2_fast(top - up);
                 top = up;
-                up = finite(up);
                 sum *= f;
                 v.x *= f;
                 v.y *= f;
@@ -625,7 +624,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
                 }
               }
               // the neighbour's half (cols / 2 is a multiple of 32: whole warps get here)
-              const float top2 = __shfl_xor_sync(0xffffffffu, top, 1), up = finite(fmaxf(top, top2)), f = exp2_fast(top - up);
+              const float top2 = __shfl_xor_sync(0xffffffffu, top, 1), up = fmaxf(top, top2), f = exp2_fast(top - up);
               sum *= f;
               v.x *= f;
               v.y *= f;
@@ -765,7 +764,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
         if (!wait()) goto leave;
         if (layer > 0 || a.added) clear(a.acc);
         if (it_token >= 0) {
-          float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;  // of heads 2j and 2j + 1 of the group
+          float m0 = LOWEST, m1 = LOWEST, l0 = 0.f, l1 = 0.f;  // of heads 2j and 2j + 1 of the group
           float o[HD / 16][4];
 #pragma unroll
           for (int i = 0; i < HD / 16; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
@@ -819,11 +818,9 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
               }
               n0 = fmaxf(n0, m0);
               n1 = fmaxf(n1, m1);
-              const float f0 = exp2_fast(m0 - finite(n0)), f1 = exp2_fast(m1 - finite(n1));
+              const float f0 = exp2_fast(m0 - n0), f1 = exp2_fast(m1 - n1);
               m0 = n0;
               m1 = n1;
-              n0 = finite(n0);
-              n1 = finite(n1);
               s[0] = exp2_fast(s[0] - n0);
               s[1] = exp2_fast(s[1] - n1);
               s[2] = exp2_fast(s[2] - n0);
@@ -873,10 +870,10 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
           if (warp < SETS && warp < used) {  // a warp's own set is read and written by that warp alone
             if (warp + SETS < used) {
               const float2 m = *reinterpret_cast<const float2*>(&sm.wm[warp + SETS][2 * j]), l = *reinterpret_cast<const float2*>(&sm.wl[warp + SETS][2 * j]);
-              const float t0 = fmaxf(m0, m.x), t1 = fmaxf(m1, m.y), n0 = finite(t0), n1 = finite(t1);
+              const float n0 = fmaxf(m0, m.x), n1 = fmaxf(m1, m.y);
               const float f0 = exp2_fast(m0 - n0), f1 = exp2_fast(m1 - n1), g0 = exp2_fast(m.x - n0), g1 = exp2_fast(m.y - n1);
-              m0 = t0;
-              m1 = t1;
+              m0 = n0;
+              m1 = n1;
               l0 = l0 * f0 + l.x * g0;
               l1 = l1 * f1 + l.y * g1;
 #pragma unroll
@@ -914,7 +911,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
 #pragma unroll
             for (int w = 0; w < SETS; ++w)
               if (w < sets) {
-                const float f = exp2_fast(m[w] - finite(top));
+                const float f = exp2_fast(m[w] - top);
                 v += osm[(w * 8 + h) * ROW + d] * f;
                 sum += sm.wl[w][h] * f;
               }
