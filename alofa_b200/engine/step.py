@@ -242,7 +242,8 @@ class StepRunner:
             self._graphs_of = self.model.loads
         if self.cuda_graphs and ctx.decode_only and ctx.n_out == ctx.n_seqs:
             ctx.max_context = self._context_bucket(ctx.max_kv_len)
-            key = (ctx.n_seqs, ctx.max_context, "decode")
+            # steps that the one kernel is not the faster way for, because of their keys, are recorded apart from those it is
+            key = (ctx.n_seqs, ctx.max_context, "decode", self.decode_stack is not None and self.decode_stack.reaches(ctx))
             g = self._graphs.get(key)
             if g is None:
                 return self._capture(ctx, key, sample)

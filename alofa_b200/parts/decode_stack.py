@@ -17,6 +17,7 @@ import torch
 
 from ..cache.storage import LayerCache
 from ..csrc import ops
+from . import fast_linear
 from .attention import GQAttention
 from .block import PrenormResidual
 from .feed_forward import GatedMLP
@@ -37,11 +38,37 @@ class Form:
     layers: tuple  # per run entry the addresses of its weights, vectors and caches, and the norms' eps
 
 
+GRANULE, WARPS = 16, 16  # keys a warp takes at a time, warps of a CTA
+
+
+def keys_per_cta_fit(lengths: list, kv_heads: int, ctas: int, most: int) -> bool:
+    """Whether requests of these lengths leave no CTA a split of more than
+    ``most`` granules, and, where a warp takes more than one, none of more than
+    five fourths of what even shares would be.  The kernel's own division: the
+    smallest splits of which all are resident together, a granule a warp at least."""
+    granules = [-(-n // GRANULE) for n in lengths]
+    total = sum(granules) * kv_heads
+    per = max(WARPS, -(-total // ctas))
+    while per <= most and sum(-(-g // per) for g in granules) * kv_heads > ctas:
+        per += 1
+    return per <= most and (per == WARPS or 4 * per * ctas <= 5 * total)
+
+
 class DecodeStack:
-    # Steps this kernel is the faster way for: as many numbers of the stream as every SM can read before each product.  us a pass of four
-    # steps, layer by layer and here: hidden 896, 3 tokens 2,748 and 2,535; hidden 1,536, 1 token 4,955 and 4,602, 4 tokens 5,207 and
-    # 4,855, 8 tokens 5,414 and 5,387; hidden 3,584, 1 token 12,682 and 11,118, 4 tokens 12,890 and 11,836, 6 tokens 12,974 and 13,015.
+    # Steps this kernel is the faster way for: as many numbers of the stream as every SM can read before each product (us a decode step at
+    # 128 tokens of context, layer by layer and here: hidden 896, 1 token 590 and 542, 8 tokens 664 and 616; hidden 1,536, 1 token 1,112 and
+    # 1,054, 8 tokens 1,201 and 1,186; hidden 3,584, 4 tokens 2,959 and 2,744, 5 tokens 2,975 and 2,933, 6 tokens more than layer by layer; hidden
+    # 2,560, 6 tokens 695 and 684, 8 tokens 695 and 735) ...
     MOST_NUMBERS = 16384
+    # ... and as many keys as the SMs get through in a few trips.  A CTA has one split of one (request, KV head) pair's keys, a warp of it 16
+    # keys at a time with none on their way behind them: up to 16 granules of 16 keys a split one trip, with twice that two.  Beyond, the
+    # kernels of a layer read faster (6 TB/s; 3.6 here with heads of 64, 4.4 with 128): hidden 896 (2 KV heads), 8 requests of 4,096 tokens
+    # (29 granules) 742 and 711, of 8,192 (57) 805 and 822, of 32,768 1,198 and 1,515; hidden 1,536, 4 of 8,192 (29) 1,379 and 1,354, 8 of
+    # 8,192 (57) 1,522 and 1,661.  A model whose layers are many rings of weights gains more by the rest: hidden 3,584, 1 of 32,768 (56) 3,465
+    # and 3,159, 4 of 8,192 (57) 3,367 and 3,299, 4 of 32,768 (228) 4,207 and 4,506.
+    MOST_GRANULES, MOST_GRANULES_WIDE, WIDE_BYTES = 32, 64, 1 << 28
+    # More than one trip only where the splits keep the SMs busy, a quarter more than with keys dealt evenly at most: 16 KV heads of 64,
+    # 8 requests of 512 tokens (128 CTAs of 32 granules where 28 would be even) 381 and 370, 5 of 512 (80 CTAs, 17) 366 and 383.
 
     def __init__(self, model, caches: dict, block_size: int):
         self.model = model
@@ -49,6 +76,7 @@ class DecodeStack:
         self.page = block_size
         self.form = None  # what the table and the scratch below were made for
         self.ctas = [0] * (ops.DECODE_STACK_TOKENS + 1)  # by tokens, 0 where the kernel does not take a step
+        self.sms = torch.cuda.get_device_properties(model.rt.device).multi_processor_count if model.rt.device.type == "cuda" else fast_linear.SMS
 
     def look(self) -> Optional[Form]:
         """The model as it is loaded now, None where its layers are not of the
@@ -123,9 +151,23 @@ class DecodeStack:
             return None
         return cls(model, caches, block_size)
 
+    def reaches(self, ctx) -> bool:
+        """Whether a step's tokens and keys are as few as this kernel is the
+        faster way for: from its lengths alone, for recorded steps too (which
+        are recorded apart by it)."""
+        n = ctx.n_tokens
+        if not ctx.decode_only or n > ops.DECODE_STACK_TOKENS or n * self.model.spec.hidden_size > self.MOST_NUMBERS:
+            return False
+        block = self.model.layers[self.model.run[0][0]]
+        pairs, inter = getattr(block.mixer, "nkv", 0), getattr(block.feed_forward, "inter", 0)
+        if not pairs or not inter:
+            return False
+        wide = 6 * self.model.spec.hidden_size * inter >= self.WIDE_BYTES  # the gate, up and down weights' bytes
+        return keys_per_cta_fit(ctx.host_field("kv_len").tolist(), pairs, self.sms, self.MOST_GRANULES_WIDE if wide else self.MOST_GRANULES)
+
     def takes(self, ctx, h) -> bool:
         n = ctx.n_tokens
-        if not ctx.decode_only or n > ops.DECODE_STACK_TOKENS or n * h.shape[1] > self.MOST_NUMBERS or ctx.stream_of(h) is None:
+        if ctx.stream_of(h) is None or not self.reaches(ctx):
             return False
         form = self.look()
         if form is None:

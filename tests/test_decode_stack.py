@@ -174,3 +174,40 @@ def test_entries_refuse_pages_grids_and_tables():
     for layers, ctas, page, stride in ((0, 148, 64, 1), (1, 0, 64, 1), (1, 15, 64, 1), (1, 148, 0, 1), (1, 148, 24, 1), (1, 148, 64, 0)):
         assert lib.alofa_decode_stack(16, layers, ctas, *good, page, stride, 1.0, *[16] * 15, None) == 1
     assert lib.alofa_decode_stack_layer(16, None, *[16] * 5, None, 16, 16, 1e-6, 1e-6, *good[1:]) == 1
+
+
+def kernel_split(lengths, kv_heads, ctas):
+    """Granules a split has at most, as the kernel looks for it: all candidates from the smallest on."""
+    granules = [n // 16 if n % 16 == 0 else n // 16 + 1 for n in lengths]
+    per = max(16, (sum(granules) * kv_heads + ctas - 1) // ctas)
+    while sum((g + per - 1) // per for g in granules) * kv_heads > ctas:
+        per += 1
+    return per, sum(granules) * kv_heads / ctas
+
+
+@pytest.mark.parametrize("kv_heads", [1, 2, 4, 8, 16])
+@pytest.mark.parametrize("most", [32, 64])
+def test_long_or_uneven_keys_go_layer_by_layer(kv_heads, most):
+    import random
+
+    from alofa_b200.parts.decode_stack import keys_per_cta_fit
+
+    rng = random.Random(kv_heads)
+    seen = set()
+    for _ in range(400):
+        lengths = [rng.choice([1, 16, 17, 256, 257, int(2 ** rng.uniform(0, 17))]) for _ in range(rng.randint(1, 8))]
+        per, even = kernel_split(lengths, kv_heads, 148)
+        want = per == 16 or (per <= most and per <= 1.25 * even)
+        assert keys_per_cta_fit(lengths, kv_heads, 148, most) == want, lengths
+        seen.add(want)
+    assert len(seen) == 2
+
+
+def test_lengths_on_either_side_of_the_rule():
+    from alofa_b200.parts.decode_stack import keys_per_cta_fit
+
+    assert keys_per_cta_fit([2049] * 8, 2, 148, 32) and keys_per_cta_fit([4096] * 8, 2, 148, 32) and not keys_per_cta_fit([8192] * 8, 2, 148, 32)
+    assert keys_per_cta_fit([32768], 2, 148, 32) and keys_per_cta_fit([32768] + [64] * 7, 2, 148, 32) and not keys_per_cta_fit([32768] * 4, 2, 148, 32)
+    assert keys_per_cta_fit([8192] * 4, 4, 148, 64) and not keys_per_cta_fit([32768] * 4, 4, 148, 64)
+    assert keys_per_cta_fit([512] * 8, 16, 148, 32) and not keys_per_cta_fit([512] * 5, 16, 148, 32) and not keys_per_cta_fit([32768] + [64] * 7, 16, 148, 32)
+    assert keys_per_cta_fit([256] * 8, 16, 148, 32) and not keys_per_cta_fit([4096] * 8, 16, 148, 32)

@@ -286,3 +286,29 @@ def test_more_layers_than_a_launch_takes(tmp_path):
         assert launched < more
         # as in test_matches_layer_by_layer, the roundings of all layers: sqrt(2 sides * layers * 8) * 2^-9 / sqrt(3)
         assert (got - want).norm() <= (2 * layers * 8 / 3) ** 0.5 * 2**-9 * want.norm()
+
+
+def test_a_step_whose_keys_outgrow_the_kernel_goes_layer_by_layer(folders):
+    """Recorded steps of one size and context bucket on either side of the line: each replay is the route of its own lengths."""
+    from alofa_b200.csrc import ops
+    from alofa_b200.engine.loading import load_model
+    from alofa_b200.engine.step import StepEntry, StepRunner
+
+    model, _, _ = load_model(folders["h64_odd"], "bfloat16")
+    ids = [int(t) for t in np.random.default_rng(9).integers(0, 300, 4000)]
+    lengths = [3000, 40, 40]  # with 3 KV heads: splits of one length for 148 CTAs at first, then too long a one beside many short
+    runner = StepRunner(model, block_size=64, num_pages=80, max_requests=8, max_tokens=4096, max_step_tokens=2048)
+    stack, launches, out = runner.decode_stack, [], []
+    slots = [runner.admit(i) for i in range(3)]
+    for s, n in zip(slots, lengths):
+        for lo in range(0, n, 2000):
+            runner.forward([StepEntry(s, ids[lo : min(n, lo + 2000)])])
+    bucket = runner._context_bucket(3001)
+    for most in (32, 0, 32, 0, 32, 0):  # the line moved, not the lengths: whether this step is on its near side
+        stack.MOST_GRANULES = most
+        before = ops.launch_count()
+        out.append(runner.forward([StepEntry(s, [5 + i], [0]) for i, s in enumerate(slots)]).clone())
+        launches.append(ops.launch_count() - before)
+    runner.check_status()
+    assert launches[4] == launches[2] < launches[3] == launches[5]
+    assert {key for key in runner._graphs if key[2] == "decode"} == {(3, bucket, "decode", True), (3, bucket, "decode", False)}
