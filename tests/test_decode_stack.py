@@ -11,6 +11,7 @@ SHAPES = {
     "0.5b": (896, 14, 2, 64, 4864), "1.5b": (1536, 12, 2, 128, 8960), "7b": (3584, 28, 4, 128, 18944),
     "one_chunk": (64, 2, 1, 64, 64), "odd": (192, 3, 3, 64, 576), "wide_ff": (256, 8, 1, 64, 16384), "group7": (896, 7, 1, 128, 2432),
 }
+UNPACED = ("1.5b", "7b")  # layers of many rings of weights: their copies are asked for behind the barriers and inside the products
 WARPS, LIMIT, MAX_TILES = 16, 232448, 64
 
 
@@ -43,6 +44,8 @@ def test_products_are_covered_once(name, tokens, ctas):
         assert name == "7b" and tokens > 4, "only wide operands of many tokens leave no room"
         return
     chunks, slots, x_stride, x_bytes, work_bytes, smem = p[16:22]
+    paced = p[22]
+    assert paced == (name not in UNPACED)
     assert slots >= 2 and smem <= LIMIT and x_bytes >= tokens * x_stride
     sizes = [((heads + 2 * kv_heads) * hd, hidden), (hidden, heads * hd), (2 * inter, hidden), (hidden, inter)]
     for phase, (rows, cols) in enumerate(sizes):

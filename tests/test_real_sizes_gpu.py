@@ -3,6 +3,8 @@ intermediate 4864, vocabulary 151936, tied head), two layers deep, against the
 plain implementation: whole prompt, decoded tail, and a mixed step.  These are
 the sizes the tensor-core kernels are tuned for (tiles of 128/256 with tails:
 1152 = 9 x 128, 4864 = 38 x 128, 151936 = 1187 x 128)."""
+import gc
+
 import numpy as np
 import pytest
 import torch
@@ -134,6 +136,7 @@ def test_steps_allocate_nothing(shaped):
         runner.release(sb)
 
     steps()  # kernels loaded, the arena grown to what these shapes need
+    gc.collect()  # what other tests left in reference cycles does not go in between
     torch.cuda.synchronize()
     grown = runner.arena.grown
     before = torch.cuda.memory_allocated()
@@ -146,13 +149,15 @@ def test_steps_allocate_nothing(shaped):
     runner.check_status()
 
 
-@pytest.mark.parametrize("n", [8, 40])
-def test_decode_steps_on_the_accumulator_stream_give_the_same_bits_every_run(shaped, n):
-    """Requests decoded together (eight: the five-kernel layer; forty: the
+@pytest.mark.parametrize("n, whole", [(8, True), (8, False), (12, False), (40, False)])
+def test_decode_steps_on_the_accumulator_stream_give_the_same_bits_every_run(shaped, n, whole):
+    """Requests decoded together (eight: all layers in one kernel, and the
+    five-kernel layer in its place; twelve: the five-kernel layer; forty: the
     layer of larger steps), whose residual products add their split sums with
     atomic integer adds in whatever order their CTAs finish: two runs from the
     same state must give the same logits bit for bit, and the accumulators are
     zero between steps."""
+    from alofa_b200.csrc import ops
     from alofa_b200.engine.loading import compute_dtype
     from alofa_b200.engine.step import StepEntry, StepRunner
     from alofa_b200.models.qwen2 import build_spec
@@ -170,13 +175,17 @@ def test_decode_steps_on_the_accumulator_stream_give_the_same_bits_every_run(sha
     for graphs in (True, True, False):
         runner = StepRunner(model, block_size=64, num_pages=5 * n, max_requests=n, max_tokens=512, max_step_tokens=256, cuda_graphs=graphs)
         assert runner._stream_acc is not None and n <= runner.STREAM_TOKENS
+        if not whole and n <= ops.DECODE_STACK_TOKENS:
+            runner.decode_stack = None
         slots = [runner.admit(i) for i in range(n)]
         for s, p in zip(slots, prompts):
             runner.forward([StepEntry(s, p, [])])
         rows = []
         for step in feed:
+            before = ops.launch_count()
             rows.append(runner.forward([StepEntry(s, [int(t)], [0]) for s, t in zip(slots, step)]).clone())
             assert int(runner._stream_acc.abs().sum()) == 0, "an accumulator was left with a value after the step"
+        assert graphs or (ops.launch_count() - before < 5 * cfg.num_hidden_layers) == whole, "the step went another way than this test says"
         runner.check_status()
         runs.append(torch.stack(rows))
     assert torch.equal(runs[0], runs[1]), "two runs of the same steps differ"
