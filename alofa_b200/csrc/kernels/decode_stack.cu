@@ -13,10 +13,10 @@
 //   3  merge of the key splits, output projection, added into the stream
 //   4  norm, gate and up product, silu(gate) * up
 //   5  down projection, added into the stream
-// A layer of 0.5B sizes takes 39,000 to 46,000 cycles at one to eight tokens (20 to 24 us; 23 to 28 as kernels, 4.5 for the
-// weights alone): per phase 1,100 for the barrier's fence, 800 for the wait of the last CTA, 1,500 to 3,700 for the operand
-// (a trip to L2 and the work on it), 800 to 1,500 for the product, 600 to 1,600 for what becomes of its sums.  us a pass of
-// perf/cases.py, layer by layer and here: decode_05b_1 4,834 and 4,551, decode_05b_8 5,903 and 5,300, decode_7b_4 12,920 and 11,680.
+// A layer of 0.5B sizes takes 22 to 25 us at one to eight tokens (23 to 28 as kernels, 4.5 for the weights alone): per phase
+// some 1,100 cycles for the barrier's fence, 800 for the wait of the last CTA, 1,500 to 4,500 for the operand (a trip to L2 and
+// the work on it), 800 to 1,500 for the product, 600 to 1,600 for what becomes of its sums.  us a pass of perf/cases.py,
+// layer by layer and here: decode_05b_1 4,857 and 4,618, decode_05b_8 5,902 and 5,471, decode_7b_4 12,859 and 11,785.
 // Products run on mma.sync m16n8k16 with the weights as the 16-row operand and 8 tokens as the other:
 // a warp multiplies straight from its ring, without the tensor-memory round trip of tcgen05 (which for a
 // handful of tokens took 70 to 110 ns per 128 x 16 x 16 instruction); the math is a
@@ -45,7 +45,7 @@ constexpr int WARPS = 16;
 constexpr int THREADS = 32 * WARPS;
 constexpr int PACE = 3;                  // pieces a paced warp asks for ahead of a product
 constexpr int GRANULE = 16;              // keys a warp takes at a time
-constexpr int MAX_TOKENS = 8;             // the columns of a product (with two groups of them, 9 to 16 tokens, 0.5B sizes lost 3 % against layer by layer, 1.5B sizes 17 %)
+constexpr int MAX_TOKENS = 8;             // the columns of a product: two groups of them were slower than layer by layer (9 to 16 tokens of 0.5B sizes 3 %, of 1.5B sizes 17 %)
 constexpr int MAX_TILES = 64;             // of 16 rows a CTA and phase
 constexpr uint32_t BARRIER_LIMIT = 1u << 21;  // polls of the grid barrier, about a second
 enum { P_QKV = 0, P_OUT = 1, P_GATE = 2, P_DOWN = 3 };
@@ -65,8 +65,8 @@ struct alignas(64) StackLayer {  // of the table of layers
 };
 static_assert(sizeof(StackLayer) % 64 == 0, "tensor maps need 64-byte alignment");
 // The table is a kernel parameter, as the maps of every other kernel are: in global memory that the host writes, each map would want a
-// fence of the tensor-map proxy in every CTA first, 100 ns a map and SM (10 us a step of 0.5B sizes).  Parameters have 32,764 bytes: a
-// deeper model goes in launches of so many layers.
+// fence of the tensor-map proxy in every CTA first, 100 ns a map (decode_05b_1 of perf/cases.py 4,661 us a pass that way, 4,620 this).
+// Parameters have 32,764 bytes: a deeper model goes in launches of so many layers.
 constexpr int MAX_LAYERS = 48;
 struct StackTable {
   StackLayer layers[MAX_LAYERS];
@@ -108,8 +108,8 @@ struct StackArgs {
 };
 
 // ---- wrappers ---------------------------------------------------------------------------------------------
-// A piece: both groups of rows at once, marked to leave L2 first (a weight is read once a step; without the mark what the phases
-// hand over was driven out: four requests of the 7B shape 12.6 and 12.1 ms a pass of four steps).
+// A piece: both groups of rows at once, marked to leave L2 first: a weight is read once a step, what the phases hand over stays
+// (four requests of the 7B shape, us a pass of four steps without and with the mark: 12,590 and 12,120).
 __device__ __forceinline__ void tma_load_piece(uint32_t dst, const CUtensorMap* map, uint32_t bar, int row, int chunk) {
   asm volatile(
       "{\n\t.reg .b64 p;\n\tcreatepolicy.fractional.L2::evict_first.b64 p, 1.0;\n\t"
@@ -205,8 +205,7 @@ __device__ __forceinline__ void next_phase(Loader& ld, const Small& sm, int warp
 }
 
 // A register that only some paths write counts as held from the start of the loop over layers to its end; that is why what a
-// load may leave out is set to zero first.  (Loads that go to a clamped place instead all hit one line: 7,500 cycles for an
-// operand of one token.)
+// load may leave out is set to zero first.
 template <int HD>
 __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_constant__ StackArgs a, const __grid_constant__ StackTable table) {
   constexpr int TP = MAX_TOKENS, C32 = HD / 32;
@@ -432,11 +431,9 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
     }
   };
 
-  // A paced warp asks for its next pieces while the operand's loads are on their way.  (All that a ring has room for, behind the
-  // barrier: that flood of copies held up the fences of the CTAs behind, 4,100 cycles after gate and up and 2,900 after the
-  // down projection, 1,100 to 1,500 this way.  Before the product, after the operand: 700 to 1,000 cycles a phase more.  0.5B sizes, us
-  // a pass of eight steps with one and eight requests: behind the barrier 5,031 and 5,658, one piece a phase 4,860 and 5,520, two
-  // 4,774 and 5,494, three 4,747 and 5,430.)
+  // A paced warp asks for its next pieces while the operand's loads are on their way: asked for behind the barrier, as many as
+  // the ring has room for, they hold up the fences of the CTAs behind (4,100 cycles after gate and up, 1,100 to 1,500 this way; 0.5B
+  // sizes, one and eight requests, 5,031 and 5,658 us a pass of eight steps that way, 4,747 and 5,430 with three a phase).
   bool asked = false;
   auto ahead = [&]() {
     if (!asked && a.paced) refill(PACE);
@@ -705,7 +702,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
               else if (sm.slot[t] >= 0) dst = (kv < a.kv_heads ? L.k + ((size_t)sm.slot[t] * a.kv_heads + kv) * HD : L.v + ((size_t)sm.slot[t] * a.kv_heads + kv - a.kv_heads) * HD) + d;
             }
           }
-          // 16 bytes a store (a fence behind stores of two bytes took 2,000 to 4,000 cycles, behind these 1,000)
+          // 16 bytes a store: the fence behind them is the shorter
           uint4 v;
           v.x = pack2(x, __shfl_down_sync(0xffffffffu, x, 1));
           v.y = __shfl_down_sync(0xffffffffu, v.x, 2);

@@ -147,7 +147,7 @@ class DecodeStack:
         """The stack of a model over one runner's caches, or None where the
         model's blocks are not ones the kernel could take.  (Whether they are is
         seen at a step: the model may be loaded, or loaded again, after this.)"""
-        if model.rt.device.type != "cuda" or model.rt.dtype != torch.bfloat16 or any(type(block) is not PrenormResidual for block in model.layers):
+        if model.rt.device.type != "cuda" or model.rt.dtype != torch.bfloat16 or not model.run or any(type(block) is not PrenormResidual for block in model.layers):
             return None
         return cls(model, caches, block_size)
 
