@@ -433,7 +433,8 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
 
   // A paced warp asks for its next pieces while the operand's loads are on their way: asked for behind the barrier, as many as
   // the ring has room for, they hold up the fences of the CTAs behind (4,100 cycles after gate and up, 1,100 to 1,500 this way; 0.5B
-  // sizes, one and eight requests, 5,031 and 5,658 us a pass of eight steps that way, 4,747 and 5,430 with three a phase).
+  // sizes, one and eight requests, us a pass of eight steps when both were measured: 5,031 and 5,658 that way, 4,747 and 5,430 with three
+  // a phase).
   bool asked = false;
   auto ahead = [&]() {
     if (!asked && a.paced) refill(PACE);

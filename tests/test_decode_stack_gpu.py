@@ -304,7 +304,8 @@ def test_keys_that_weigh_nothing(folders, name, context, pages, rows):
 
 
 def test_two_runners_on_two_streams(folders):
-    """Steps of two runners side by side, of shapes that want different amounts of shared memory: the same bits as one after the other."""
+    """Steps of two runners side by side, of shapes that want different amounts of shared memory, and beside other work that fills the
+    device: the same bits as one after the other."""
     from alofa_b200.engine.loading import load_model
     from alofa_b200.engine.step import StepEntry, StepRunner
 
@@ -323,8 +324,12 @@ def test_two_runners_on_two_streams(folders):
         pair = make(*kind)
         want.append([step(pair, t).clone() for t in range(steps)])
     pairs, streams, got = [make(*kind) for kind in kinds], [torch.cuda.Stream() for _ in kinds], [[], []]
+    other, a = torch.cuda.Stream(), torch.ones((4096, 4096), dtype=torch.bfloat16, device="cuda")
     torch.cuda.synchronize()
     for t in range(steps):
+        with torch.cuda.stream(other):
+            for _ in range(4):
+                a @ a
         for i, (pair, stream) in enumerate(zip(pairs, streams)):
             with torch.cuda.stream(stream):
                 got[i].append(step(pair, t).clone())
@@ -356,7 +361,7 @@ def test_a_step_whose_keys_outgrow_the_kernel_goes_layer_by_layer(folders):
 
     model, _, _ = load_model(folders["h64_odd"], "bfloat16")
     ids = [int(t) for t in np.random.default_rng(9).integers(0, 300, 4000)]
-    lengths = [3000, 40, 40]  # with 3 KV heads: splits of one length for 148 CTAs at first, then too long a one beside many short
+    lengths = [3000, 40, 40]
     runner = StepRunner(model, block_size=64, num_pages=80, max_requests=8, max_tokens=4096, max_step_tokens=2048)
     stack, launches, out = runner.decode_stack, [], []
     slots = [runner.admit(i) for i in range(3)]
